@@ -172,9 +172,6 @@ pcrp_status f64_solve(const double* a, const double* b, const double* c, const d
         return set_error(PCRP_EINVAL, "%s: m*n = %lld * %lld is too large for the split-path scratch", who,
                          (long long)m, (long long)n);
 
-    // null a and e: a tridiagonal batch, both bands +0.0; the first pass
-    // reads neither, and every pass runs the zero-state strides
-    const bool tri = !a && !e;
     F64Plan pl = f64_plan(o, n);
     if (force_small && pl.smem_rows < n) pl.smem_rows = (int)n;         // the n <= 1024 path is one tile
     if (force_split && pl.smem_rows >= n) pl.smem_rows = 1024;         // the n > 1024 path splits
@@ -209,7 +206,7 @@ pcrp_status f64_solve(const double* a, const double* b, const double* c, const d
     // fill their tiles better with the wider halo); a pass of fewer strides
     // turns the halo rows it does not need into tile rows.
     const int npass = s1 > 0 ? (s1 + pl.fuse - 1) / pl.fuse : 0;
-    int cur = 0;
+    int cur = 0, rem = ns;
     for (int ip = 0; ip < npass; ip++) {
         const int K = s1 / npass + (ip >= npass - s1 % npass ? 1 : 0);
         const int H = 2 * ((1 << K) - 1);
@@ -222,12 +219,13 @@ pcrp_status f64_solve(const double* a, const double* b, const double* c, const d
         // subsystem (results do not depend on where windows start)
         p.nwin = ceil_div(nrmax, L);
         L = (int)ceil_div(nrmax, p.nwin);
-        p.K = K; p.H = H; p.L = L; p.final_step = 0;
+        p.K = K; p.H = H; p.L = L; p.final_step = 0; p.rem = rem;
+        rem -= K;
         p.TRmax = (int)std::min<int64_t>(L + 2 * H, nrmax);
         for (int k = 0; k < NSTATE; k++) p.dst[k] = bufs[cur][k];
         p.dst_ss = n; p.dst_rs = 1;
         p.dst_sub = 1;                      // the next pass reads each subsystem in one run
-        cudaError_t ce = launch_pcr_pass(p, pl.threads, st, tri);
+        cudaError_t ce = launch_pcr_pass(p, pl.threads, st);
         if (ce != cudaSuccess) return cuda_error(ce, "pcr global pass launch");
         for (int k = 0; k < NSTATE; k++) p.src[k] = bufs[cur][k];
         p.src_ss = n; p.src_rs = 1; p.src_sub = 1;
@@ -237,7 +235,7 @@ pcrp_status f64_solve(const double* a, const double* b, const double* c, const d
 
     // shared-memory finish on whole subsystems of at most smem_rows rows
     const int64_t nrmax = ceil_div(n, p.G);
-    p.K = ns - s1; p.H = 0; p.L = (int)nrmax; p.final_step = 1; p.nwin = 1;
+    p.K = p.rem = ns - s1; p.H = 0; p.L = (int)nrmax; p.final_step = 1; p.nwin = 1;
     p.TRmax = (int)nrmax;
     // whole systems read straight from the caller's arrays: bulk-staged
     // tiles where every array row run is 16-byte aligned (contiguous layout,
@@ -250,7 +248,7 @@ pcrp_status f64_solve(const double* a, const double* b, const double* c, const d
     }
     p.x = y; p.dst_ss = ss; p.dst_rs = rs; p.dst_sub = 0;
     for (int k = 0; k < NSTATE; k++) p.dst[k] = nullptr;
-    cudaError_t ce = launch_pcr_pass(p, pl.threads, st, tri);
+    cudaError_t ce = launch_pcr_pass(p, pl.threads, st);
     if (ce != cudaSuccess) return cuda_error(ce, "pcr shared-memory pass launch");
     return PCRP_OK;
 }

@@ -142,8 +142,8 @@ __device__ __forceinline__ double operand(uint64_t r, int mode)
     return __longlong_as_double((long long)(((r >> 63) << 63) | ((uint64_t)e << 52) | mant));
 }
 
-// The phase-B quotient of the FP64 kernels (mdiv: Markstein's correction
-// from the correctly rounded reciprocal) against __ddiv_rn on random pairs.
+// The quotient of the FP64 kernels (quot: on the integer pipe inside its
+// guard) against __ddiv_rn on random pairs.
 __global__ void __launch_bounds__(kProbeThreads)
 quotient_check(int mode, uint64_t seed, int64_t per_thread, unsigned long long* bad, unsigned long long* fast)
 {
@@ -154,11 +154,10 @@ quotient_check(int mode, uint64_t seed, int64_t per_thread, unsigned long long* 
         const uint64_t r2 = mix64(seed + t * 0x9E37ull + (uint64_t)i * 2 + 1);
         const double a = operand(r1, mode), b = operand(r2, (r2 & 1) ? 4 : mode);
         if (!nz(b)) continue;                     // the kernels never divide by zero
-        const double q = mdiv(a, b, __drcp_rn(b)), ref = __ddiv_rn(a, b);
+        const double q = quot(a, b, ieee::recip(b)), ref = __ddiv_rn(a, b);
         const bool same = __double_as_longlong(q) == __double_as_longlong(ref) || (q != q && ref != ref);
         nb += !same;
-        const int ea = (int)((hiw(a) >> 20) & 0x7FFu), eb = (int)((hiw(b) >> 20) & 0x7FFu);
-        nf += (unsigned)(ea - 100) <= 1846u && (unsigned)(eb - 100) <= 1846u && (unsigned)(ea - eb + 900) <= 1800u;
+        nf += ieee::div_guard(a, b);
     }
     atomicAdd(bad, nb);
     atomicAdd(fast, nf);

@@ -61,66 +61,54 @@
 namespace pcrp {
 namespace {
 
-// Three CTAs per SM where shared memory allows (tiles up to ~620 rows): the
-// tile state fits 80 registers without spills up to 4 rows per thread, and
-// the extra warps hide more of the FP64 latency; two for 8 rows per thread.
-template <int RPT, bool kZero>
-__global__ void __launch_bounds__(kMaxThreads, RPT >= 8 ? 2 : 3)
+// CTAs per SM the register budget is set for: as many as shared memory holds
+// (100 bytes per row), at most 1024 threads.
+template <int CAP>
+__global__ void __launch_bounds__(kMaxThreads, CAP > 1024 ? 1 : CAP > 544 ? 2 : 4)
 pcr_pass_kernel(const PcrPassArgs p)
 {
-    extern __shared__ double smem[];
+    extern __shared__ __align__(16) unsigned char pcr_smem[];
     const int64_t blk  = blockIdx.x;
     const int64_t item = blk / p.nwin;
     const int64_t w    = blk - item * p.nwin;
     const int64_t j    = item / p.G;
     const int64_t r    = item - j * p.G;
-    pcr_tile<RPT, false, kZero>(p, j, r, w, smem);
+    pcr_tile<CAP>(p, j, r, w, *reinterpret_cast<TileRows<CAP>*>(pcr_smem));
 }
 
-
-template <int RPT, bool kZero>
-cudaError_t launch_rz(const PcrPassArgs& p, int threads, size_t smem, int64_t blocks, cudaStream_t s)
+template <int CAP>
+cudaError_t launch_cap(const PcrPassArgs& p, int threads, int64_t blocks, cudaStream_t s)
 {
     // per-device attribute; cheap, and legal while a stream is being captured
-    cudaError_t e = cudaFuncSetAttribute(pcr_pass_kernel<RPT, kZero>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         pcr_max_smem_rows() * kSmemArrays * (int)sizeof(double));
+    cudaError_t e = cudaFuncSetAttribute(pcr_pass_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(TileRows<CAP>));
     if (e != cudaSuccess) return e;
-    pcr_pass_kernel<RPT, kZero><<<(unsigned)blocks, threads, smem, s>>>(p);
+    pcr_pass_kernel<CAP><<<(unsigned)blocks, threads, sizeof(TileRows<CAP>), s>>>(p);
     count_launch();
     return cudaGetLastError();
 }
 
-template <int RPT>
-cudaError_t launch_rpt(const PcrPassArgs& p, bool tridiagonal, int threads, size_t smem, int64_t blocks,
-                       cudaStream_t s)
-{
-    if (pass_votes(p, tridiagonal))
-        return launch_rz<RPT, true>(p, threads, smem, blocks, s);
-    return launch_rz<RPT, false>(p, threads, smem, blocks, s);
-}
-
 }  // namespace
 
-int pcr_max_smem_rows() { return 1920; }   // 15 arrays * 1920 * 8 B = 225 KiB
+int pcr_max_smem_rows() { return 1920; }
 
-size_t pcr_pass_smem_bytes(int TRmax) { return (size_t)TRmax * kSmemArrays * sizeof(double); }
-
-cudaError_t launch_pcr_pass(const PcrPassArgs& p, int threads, cudaStream_t s, bool tridiagonal)
+cudaError_t launch_pcr_pass(const PcrPassArgs& p, int threads, cudaStream_t s)
 {
     if (threads <= 0 || threads > kMaxThreads) threads = kMaxThreads;
     threads = (threads + 31) / 32 * 32;
     if (p.TRmax < threads) threads = (p.TRmax + 31) / 32 * 32;   // small (sub)systems: no idle warps
-    int rpt = (p.TRmax + threads - 1) / threads;
-    while (rpt > 8 && threads < kMaxThreads) { threads += 32; rpt = (p.TRmax + threads - 1) / threads; }
-    if (rpt > 8 || p.TRmax > pcr_max_smem_rows()) return cudaErrorInvalidValue;
+    while ((p.TRmax + threads - 1) / threads > kMaxRowsPerThread && threads < kMaxThreads) threads += 32;
+    if (p.TRmax > pcr_max_smem_rows()) return cudaErrorInvalidValue;
     const int64_t blocks = p.m * p.G * p.nwin;
     if (blocks <= 0) return cudaSuccess;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    const size_t smem = pcr_pass_smem_bytes(p.TRmax);
-    if (rpt <= 1) return launch_rpt<1>(p, tridiagonal, threads, smem, blocks, s);
-    if (rpt <= 2) return launch_rpt<2>(p, tridiagonal, threads, smem, blocks, s);
-    if (rpt <= 4) return launch_rpt<4>(p, tridiagonal, threads, smem, blocks, s);
-    return launch_rpt<8>(p, tridiagonal, threads, smem, blocks, s);
+    if (p.TRmax <= 32) return launch_cap<32>(p, threads, blocks, s);
+    if (p.TRmax <= 64) return launch_cap<64>(p, threads, blocks, s);
+    if (p.TRmax <= 128) return launch_cap<128>(p, threads, blocks, s);
+    if (p.TRmax <= 256) return launch_cap<256>(p, threads, blocks, s);
+    if (p.TRmax <= 544) return launch_cap<544>(p, threads, blocks, s);
+    if (p.TRmax <= 1024) return launch_cap<1024>(p, threads, blocks, s);
+    return launch_cap<1920>(p, threads, blocks, s);
 }
 
 }  // namespace pcrp

@@ -3,6 +3,7 @@
 // The arithmetic and its correspondence with the reference are described at
 // the top of pcr_f64.cu.
 #pragma once
+#include "ieee_int.cuh"
 #include "pcrp_internal.h"
 #include "tma.cuh"
 
@@ -23,18 +24,6 @@ __device__ __forceinline__ unsigned magbits(double x) {
 }
 // x != 0.0 (false for +-0, true for everything else including NaN)
 __device__ __forceinline__ bool nz(double x) { return magbits(x) != 0u; }
-// x / y, IEEE round-to-nearest.  A zero x over a nonzero finite y is the
-// signed zero IEEE 754 prescribes (sign of x xor sign of y), formed on the
-// integer pipe: the FP64 division takes ~2.6x its normal time for a zero
-// numerator, and from stride ~2^9 on the outer coefficients of a diagonally
-// dominant system are zero, so half of the divisions of the late strides
-// have one.  Every other operand pair goes to the division.
-__device__ __forceinline__ double dvd(double x, double y) {
-    const unsigned yh = (unsigned)__double2hiint(y);
-    if (magbits(x) == 0u && magbits(y) != 0u && (yh & 0x7FF00000u) != 0x7FF00000u)
-        return __hiloint2double((int)((((unsigned)__double2hiint(x)) ^ yh) & 0x80000000u), 0);
-    return __ddiv_rn(x, y);
-}
 // -x by flipping the sign bit on the integer pipe (bit-identical to unary
 // minus), in PTX for the same reason as magbits
 __device__ __forceinline__ double neg(double x) {
@@ -53,33 +42,359 @@ __device__ __forceinline__ double szero(unsigned s) { return __hiloint2double((i
 // x + z for a zero z with sign bit zs, x not NaN: x itself, unless x is a
 // zero too (then -0 only if both are -0: round-to-nearest)
 __device__ __forceinline__ double add_z(double x, unsigned zs) { return nz(x) ? x : szero(hiw(x) & zs); }
-// x / y from y's correctly rounded reciprocal r = RN(1/y) (__drcp_rn):
-// Markstein's correction (IBM J. Res. Dev. 1990): q0 = RN(x r) is within an
-// ulp of x/y, the remainder x - y q0 is exact in one FMA, and RN(q0 + rem r)
-// = RN(x / y) while no intermediate leaves the normal range, which the
-// exponent guard ensures; other operands take the division.
-__device__ __forceinline__ double mdiv(double x, double y, double r) {
-    const int ex = (int)((hiw(x) >> 20) & 0x7FFu), ey = (int)((hiw(y) >> 20) & 0x7FFu);
-    if ((unsigned)(ex - 100) <= 1846u && (unsigned)(ey - 100) <= 1846u && (unsigned)(ex - ey + 900) <= 1800u) {
-        const double q0 = __dmul_rn(x, r);
-        const double rem = __fma_rn(-y, q0, x);
-        return __fma_rn(rem, r, q0);
-    }
+// x / y, IEEE round-to-nearest, off the main path: a zero x over a nonzero
+// finite y is the signed zero IEEE 754 prescribes; then the integer quotient
+// of any size; the FP64 division for the rest (infinities, nans, zero and
+// subnormal divisors, overflow).
+static __device__ __noinline__ double dvd(double x, double y) {
+    if (!nz(x) && nz(y) && (hiw(y) & 0x7FF00000u) != 0x7FF00000u) return szero(hiw(x) ^ hiw(y));
+    double q;
+    if (ieee::div_any(x, y, q)) return q;
+    return __ddiv_rn(x, y);
+}
+// x / y from G = ieee::recip(y) on the integer pipe where both operands are
+// inside its guard; other operands take dvd.
+__device__ __forceinline__ double quot(double x, double y, uint32_t G) {
+    if (ieee::div_guard(x, y)) return ieee::div(x, y, G);
     return dvd(x, y);
 }
-__device__ __forceinline__ bool finite4(double p, double q, double r, double s) {
-    return max(max(hiw(p) & 0x7FF00000u, hiw(q) & 0x7FF00000u), max(hiw(r) & 0x7FF00000u, hiw(s) & 0x7FF00000u))
-           < 0x7FF00000u;
+__device__ __forceinline__ double quot(double x, double y) { return quot(x, y, ieee::recip(y)); }
+
+// z - x for a zero z with sign bit zs, x not NaN
+__device__ __forceinline__ double sub_z(unsigned zs, double x) { return nz(x) ? neg(x) : szero(zs & ~hiw(x)); }
+// every one of the values +-0 / finite
+__device__ __forceinline__ bool zeros(double x, double y, double z) {
+    return (magbits(x) | magbits(y) | magbits(z)) == 0u;
 }
-// "zero state" of a row: outer coefficients a, e zero, the others finite.
-// While every row a stride reads is in it, both multipliers of phase A are
-// zeros, every product with them is a zero and phase A forms no FP64 value.
-__device__ __forceinline__ bool zero_state(double a, double b, double c, double d, double e, double y) {
-    return !nz(a) && !nz(e) && finite4(b, c, d, y);
+__device__ __forceinline__ unsigned expw(double x) { return hiw(x) & 0x7FF00000u; }
+__device__ __forceinline__ bool finite6(double p, double q, double r, double s, double t, double u) {
+    return max(max(max(expw(p), expw(q)), max(expw(r), expw(s))), max(expw(t), expw(u))) < 0x7FF00000u;
 }
 
 constexpr int kMaxThreads = 256;
-constexpr int kSmemArrays = 15;   // 6 state + 6 T coefficients + 2 T multipliers + 1/cT
+constexpr int kMaxRowsPerThread = 8;
+
+// ---------------------------------------------------------------------------
+// One row of a stride, straight-line per case
+// ---------------------------------------------------------------------------
+// The row updates below give the bits of the reference's operations
+// (Reductions I-III, kernel.cu:63-140) for one case of operands each; they
+// return false, with nothing written, for rows outside their case, and those
+// rows take the general form in pcr_tile.  In every case the quotients and
+// most products run on the integer pipe (ieee_int.cuh), the sums and the rhs
+// products (a rhs is often zero, which is outside the integer product's
+// guard) on the FP64 pipe: per row and stride 36 products and sums and 4
+// quotients, of which 16 sums and 4 products stay FP64.  No branch inside a
+// case: with a branch per operation the chains of a row serialise (measured:
+// 14.0 against 13.2 ms for m=16 n=2^20).
+//
+// A multiplier of a side (left: row - dl, right: row + dl) is "active" when
+// it is a nonzero quotient inside the guard.  Otherwise it is a zero (its
+// numerator is zero, or the row two steps out does not exist) or the side
+// itself is missing; then every product with it is a zero whose sign is the
+// factors' sign xor, adding it leaves a nonzero term alone, and no FP64
+// operation is issued for that side.  This covers the ends of a (sub)system
+// (in a whole-system tile the last two strides consist of them), one-sided
+// and tridiagonal batches (a or e zero), and the late strides of diagonally
+// dominant systems, whose outer coefficients underflow to zero.
+template <int CAP>
+struct TileRows {
+    double a[CAP], b[CAP], c[CAP], d[CAP], e[CAP], y[CAP];            // state
+    double Ta[CAP], Tb[CAP], Tc[CAP], Td[CAP], Te[CAP], Ty[CAP];      // T(m)
+    uint32_t Tr[CAP];                                                 // ieee::recip of Tc
+};
+
+// signs (bit 31) of the products of a zero multiplier of sign s with a row
+struct Signs { unsigned a, b, c, d, e, y; };
+
+// Phase A, both multipliers active.
+template <int CAP>
+__device__ __forceinline__ bool row_a_both(TileRows<CAP>& t, int k, int dl, double& cT)
+{
+    const int l = k - dl, r = k + dl;
+    const double am = t.a[k], em = t.e[k];
+    const double aL = t.a[l], bL = t.b[l], cL = t.c[l], dL = t.d[l], eL = t.e[l];
+    const double aR = t.a[r], bR = t.b[r], cR = t.c[r], dR = t.d[r], eR = t.e[r];
+    const unsigned w = ieee::off(am) | ieee::off(em) | ieee::off(aL) | ieee::off(bL) | ieee::off(cL) | ieee::off(dL) |
+                       ieee::off(eL) | ieee::off(aR) | ieee::off(bR) | ieee::off(cR) | ieee::off(dR) | ieee::off(eR);
+    if (!ieee::fits(w)) return false;
+    const double al1 = ieee::div(neg(am), bL, ieee::recip(bL)), al2 = ieee::div(neg(em), dR, ieee::recip(dR));
+    const ieee::Factor f1 = ieee::factor(al1), f2 = ieee::factor(al2);
+    cT = add(add(ieee::mul(f1, dL), t.c[k]), ieee::mul(f2, bR));
+    t.Tc[k] = cT;
+    t.Tr[k] = ieee::recip(cT);
+    t.Tb[k] = add(add(ieee::mul(f1, cL), t.b[k]), ieee::mul(f2, aR));
+    t.Td[k] = add(add(ieee::mul(f1, eL), t.d[k]), ieee::mul(f2, cR));
+    t.Ty[k] = add(add(mul(al1, t.y[l]), t.y[k]), mul(al2, t.y[r]));
+    t.Ta[k] = ieee::mul(f1, aL);
+    t.Te[k] = ieee::mul(f2, eR);
+    return true;
+}
+
+// A multiplier num/piv of any size; false for a zero pivot.
+__device__ __forceinline__ bool tiny_quotient(double num, double piv, uint32_t G, double& f)
+{
+    if (!nz(piv)) return false;
+    f = quot(num, piv, G);
+    return true;
+}
+// f*x cannot change a sum with c (|f*x| < 2^-54 |c|, or f*x a zero and c
+// not): from the exponent fields, x finite, c inside `mid`
+__device__ __forceinline__ bool absorbed(double f, double x, double c)
+{
+    return expw(x) < 0x7FF00000u && expw(f) < (1100u << 20) && ieee::mid(c) && expw(f) + expw(x) + (55u << 20) <= expw(c) + (1022u << 20);
+}
+
+// Phase A once the couplings are tiny (al1*dL, al2*bR and the rhs products
+// too small to change the row's c and y): the quotients as above, cT and the
+// rhs are the row's own, the other products and sums on the FP64 pipe, whose
+// subnormal and zero results need no case of their own.  A missing side adds
+// -0, which changes nothing.
+template <int CAP>
+__device__ __forceinline__ bool row_a_tiny(TileRows<CAP>& t, int k, int dl, bool hasL, bool has2L, bool hasR, bool has2R, double& cT)
+{
+    const int l = hasL ? k - dl : k, r = hasR ? k + dl : k;
+    const double cm = t.c[k], ym = t.y[k];
+    double al1 = 0.0, al2 = 0.0;
+    if (has2L && !tiny_quotient(neg(t.a[k]), t.b[l], ieee::recip(t.b[l]), al1)) return false;
+    if (has2R && !tiny_quotient(neg(t.e[k]), t.d[r], ieee::recip(t.d[r]), al2)) return false;
+    if (!(absorbed(al1, t.d[l], cm) && absorbed(al1, t.y[l], ym) && absorbed(al2, t.b[r], cm) &&
+          absorbed(al2, t.y[r], ym))) return false;
+    const double m0 = szero(~0u);
+    t.Tb[k] = hasL ? add(add(mul(al1, t.c[l]), t.b[k]), hasR ? mul(al2, t.a[r]) : m0) : 0.0;
+    t.Td[k] = hasR ? add(add(hasL ? mul(al1, t.e[l]) : m0, t.d[k]), mul(al2, t.c[r])) : 0.0;
+    t.Ta[k] = hasL ? mul(al1, t.a[l]) : 0.0;
+    t.Te[k] = hasR ? mul(al2, t.e[r]) : 0.0;
+    cT = cm;
+    t.Tc[k] = cm; t.Ty[k] = ym;
+    t.Tr[k] = ieee::recip(cm);
+    return true;
+}
+
+// Zero multiplier of phase A towards row q (l or r): its sign, and the signs
+// of its products with that row; false if it is not a zero or a factor is not
+// finite.  num: the row's numerator, piv: row q's pivot, has2: the row two
+// steps out exists (else the multiplier is +0).
+template <int CAP>
+__device__ __forceinline__ bool zero_side(TileRows<CAP>& t, int q, bool has2, double num, double piv, unsigned& s,
+                                          Signs& g)
+{
+    if (has2 && nz(num)) return false;
+    const double qa = t.a[q], qb = t.b[q], qc = t.c[q], qd = t.d[q], qe = t.e[q], qy = t.y[q];
+    if (!finite6(qa, qb, qc, qd, qe, qy)) return false;
+    s = has2 && nz(piv) ? hiw(num) ^ hiw(piv) ^ 0x80000000u : 0u;
+    g = {s ^ hiw(qa), s ^ hiw(qb), s ^ hiw(qc), s ^ hiw(qd), s ^ hiw(qe), s ^ hiw(qy)};
+    return true;
+}
+
+// A missing side adds nothing, which is what adding -0 does.
+__device__ __forceinline__ Signs absent() { return {~0u, ~0u, ~0u, ~0u, ~0u, ~0u}; }
+
+// Phase A of a row with both sides, one multiplier active and the other one a
+// zero: the right one active, or the mirror image in the same code (a and e,
+// b and d exchanged; the zero terms may be added in any order).  One-sided
+// batches (a = 0 from upwind differences, for instance).
+template <int CAP>
+__device__ __forceinline__ bool row_a_one(TileRows<CAP>& t, int k, int dl, bool right, double& cT)
+{
+    const int q = right ? k + dl : k - dl, o = right ? k - dl : k + dl;
+    // inner and outer coefficients of the active side (in, out) and the other (io, oo)
+    const double* in = right ? t.d : t.b;
+    const double* io = right ? t.b : t.d;
+    const double* out = right ? t.e : t.a;
+    const double* oo = right ? t.a : t.e;
+    const double num = out[k], piv = in[q], p1 = io[q], p2 = t.c[q], p4 = out[q];
+    if (!ieee::fits(ieee::off(num) | ieee::off(piv) | ieee::off(p1) | ieee::off(p2) | ieee::off(p4))) return false;
+    unsigned s;
+    Signs g;
+    if (!zero_side(t, o, true, oo[k], io[o], s, g)) return false;
+    const double al = ieee::div(neg(num), piv, ieee::recip(piv));
+    const ieee::Factor f = ieee::factor(al);
+    cT = add(add_z(t.c[k], right ? g.d : g.b), ieee::mul(f, p1));
+    const double inner = add(add_z(in[k], right ? g.e : g.a), ieee::mul(f, p2));   // dT (bT)
+    const double across = add(add_z(io[k], g.c), mul(al, oo[q]));                  // bT (dT)
+    const double far = ieee::mul(f, p4), near = szero(right ? g.a : g.e);          // eT, aT (aT, eT)
+    t.Tc[k] = cT;
+    t.Tr[k] = ieee::recip(cT);
+    t.Ty[k] = add(add_z(t.y[k], g.y), mul(al, t.y[q]));
+    t.Tb[k] = right ? across : inner; t.Td[k] = right ? inner : across;
+    t.Ta[k] = right ? near : far;     t.Te[k] = right ? far : near;
+    return true;
+}
+
+// Phase A, neither multiplier active (at least one side present): no FP64
+// operation at all.
+template <int CAP>
+__device__ __forceinline__ bool row_a_none(TileRows<CAP>& t, int k, int dl, bool hasL, bool has2L, bool hasR, bool has2R, double& cT)
+{
+    unsigned s1 = 0u, s2 = 0u;
+    Signs g1 = absent(), g2 = absent();
+    if (hasL && !zero_side(t, k - dl, has2L, t.a[k], t.b[k - dl], s1, g1)) return false;
+    if (hasR && !zero_side(t, k + dl, has2R, t.e[k], t.d[k + dl], s2, g2)) return false;
+    cT = add_z(add_z(t.c[k], g1.d), g2.b);
+    t.Tc[k] = cT;
+    t.Tr[k] = ieee::recip(cT);
+    t.Tb[k] = hasL ? add_z(add_z(t.b[k], g1.c), g2.a) : 0.0;
+    t.Td[k] = hasR ? add_z(add_z(t.d[k], g1.e), g2.c) : 0.0;
+    t.Ty[k] = add_z(add_z(t.y[k], g1.y), g2.y);
+    t.Ta[k] = hasL ? szero(g1.a) : 0.0;
+    t.Te[k] = hasR ? szero(g2.e) : 0.0;
+    return true;
+}
+
+// Phase B, both multipliers active (f1 = b/cT(l), f2 = d/cT(r)); kA, kE: the
+// coefficients a and e of the row and of T are zeros (only their signs
+// matter).
+template <bool kA, bool kE, int CAP>
+__device__ __forceinline__ bool row_b_both(TileRows<CAP>& t, int k, int dl, double& f1, double& f2)
+{
+    const int l = k - dl, r = k + dl;
+    const double bi = t.b[k], di = t.d[k], cL = t.Tc[l], cR = t.Tc[r];
+    const double aL = t.Ta[l], bL = t.Tb[l], dL = t.Td[l], eL = t.Te[l];
+    const double aR = t.Ta[r], bR = t.Tb[r], dR = t.Td[r], eR = t.Te[r];
+    unsigned w = ieee::off(bi) | ieee::off(di) | ieee::off(cL) | ieee::off(cR) | ieee::off(bL) | ieee::off(dL) |
+                 ieee::off(bR) | ieee::off(dR);
+    if (!kA) w |= ieee::off(aL) | ieee::off(aR);
+    if (!kE) w |= ieee::off(eL) | ieee::off(eR);
+    if (!ieee::fits(w)) return false;
+    if (kA && !zeros(t.a[k], aL, aR)) return false;
+    if (kE && !zeros(t.e[k], eL, eR)) return false;
+    f1 = ieee::div(bi, cL, t.Tr[l]); f2 = ieee::div(di, cR, t.Tr[r]);
+    const ieee::Factor g1 = ieee::factor(f1), g2 = ieee::factor(f2);
+    const double ny = add(sub(mul(f1, t.Ty[l]), t.y[k]), mul(f2, t.Ty[r]));
+    const double nc = add(sub(ieee::mul(g1, dL), t.c[k]), ieee::mul(g2, bR));
+    const double b1 = ieee::mul(g1, bL), d2 = ieee::mul(g2, dR);        // nonzero
+    const double nb = kA ? b1 : add(sub(b1, t.a[k]), ieee::mul(g2, aR));
+    const double nd = kE ? d2 : add(sub(ieee::mul(g1, eL), t.e[k]), d2);
+    t.y[k] = ny; t.c[k] = nc; t.b[k] = nb; t.d[k] = nd;
+    t.a[k] = kA ? szero(hiw(f1) ^ hiw(aL)) : ieee::mul(g1, aL);
+    t.e[k] = kE ? szero(hiw(f2) ^ hiw(eR)) : ieee::mul(g2, eR);
+    return true;
+}
+
+// Phase B once the couplings are tiny: c and y change sign, the rest on the
+// FP64 pipe (a missing side's products are +0).
+template <int CAP>
+__device__ __forceinline__ bool row_b_tiny(TileRows<CAP>& t, int k, int dl, bool hasL, bool hasR, double& f1,
+                                           double& f2)
+{
+    const int l = hasL ? k - dl : k, r = hasR ? k + dl : k;
+    const double ci = t.c[k], yi = t.y[k];
+    double g1 = 0.0, g2 = 0.0;
+    if (hasL && !(tiny_quotient(t.b[k], t.Tc[l], t.Tr[l], g1) && absorbed(g1, t.Td[l], ci) &&
+                  absorbed(g1, t.Ty[l], yi))) return false;
+    if (hasR && !(tiny_quotient(t.d[k], t.Tc[r], t.Tr[r], g2) && absorbed(g2, t.Tb[r], ci) &&
+                  absorbed(g2, t.Ty[r], yi))) return false;
+    t.b[k] = add(sub(hasL ? mul(g1, t.Tb[l]) : 0.0, t.a[k]), hasR ? mul(g2, t.Ta[r]) : 0.0);
+    t.d[k] = add(sub(hasL ? mul(g1, t.Te[l]) : 0.0, t.e[k]), hasR ? mul(g2, t.Td[r]) : 0.0);
+    t.a[k] = hasL ? mul(g1, t.Ta[l]) : 0.0;
+    t.e[k] = hasR ? mul(g2, t.Te[r]) : 0.0;
+    t.c[k] = neg(ci); t.y[k] = neg(yi);
+    if (hasL) f1 = g1;
+    if (hasR) f2 = g2;
+    return true;
+}
+
+// Zero multiplier num/cT(q) of phase B; false if it is not a zero or a factor
+// is not finite.
+template <int CAP>
+__device__ __forceinline__ bool zero_quotient(TileRows<CAP>& t, int q, double num, double& f, Signs& g)
+{
+    const double qc = t.Tc[q];
+    if (nz(num) || !nz(qc)) return false;
+    const double qa = t.Ta[q], qb = t.Tb[q], qd = t.Td[q], qe = t.Te[q], qy = t.Ty[q];
+    if (!finite6(qa, qb, qc, qd, qe, qy)) return false;
+    const unsigned s = hiw(num) ^ hiw(qc);
+    f = szero(s);
+    g = {s ^ hiw(qa), s ^ hiw(qb), s ^ hiw(qc), s ^ hiw(qd), s ^ hiw(qe), s ^ hiw(qy)};
+    return true;
+}
+
+// Phase B, neither multiplier active: the row changes sign.
+template <int CAP>
+__device__ __forceinline__ bool row_b_none(TileRows<CAP>& t, int k, int dl, bool hasL, bool hasR, double& f1, double& f2)
+{
+    Signs g1{0u, 0u, 0u, 0u, 0u, 0u}, g2{0u, 0u, 0u, 0u, 0u, 0u};
+    const double ai = t.a[k], ci = t.c[k], ei = t.e[k], yi = t.y[k];
+    if (!finite6(ai, ci, ei, yi, ci, yi)) return false;
+    if (hasL && !zero_quotient(t, k - dl, t.b[k], f1, g1)) return false;
+    if (hasR && !zero_quotient(t, k + dl, t.d[k], f2, g2)) return false;
+    t.b[k] = add_z(sub_z(g1.b, ai), g2.a);
+    t.c[k] = add_z(sub_z(g1.d, ci), g2.b);
+    t.d[k] = add_z(sub_z(g1.e, ei), g2.d);
+    t.y[k] = add_z(sub_z(g1.y, yi), g2.y);
+    t.a[k] = szero(g1.a);
+    t.e[k] = szero(g2.e);
+    return true;
+}
+
+// The general forms: every operation on the FP64 pipe but the quotients whose
+// operands are inside the integer quotient's guard.
+template <int CAP>
+__device__ __forceinline__ double row_a_general(TileRows<CAP>& t, int k, int dl, bool hasL, bool has2L, bool hasR, bool has2R)
+{
+    const int l = k - dl, r = k + dl;
+    double al1 = 0.0, al2 = 0.0;
+    if (has2L && nz(t.b[l])) al1 = quot(neg(t.a[k]), t.b[l]);
+    if (has2R && nz(t.d[r])) al2 = quot(neg(t.e[k]), t.d[r]);
+    // (a missing side adds -0, which changes nothing: kernel.cu:82-91,108-117)
+    const double m0 = szero(~0u);
+    const int lc = hasL ? l : k, rc = hasR ? r : k;
+    const double cT = add(add(hasL ? mul(al1, t.d[lc]) : m0, t.c[k]), hasR ? mul(al2, t.b[rc]) : m0);
+    const double kT = add(add(hasL ? mul(al1, t.y[lc]) : m0, t.y[k]), hasR ? mul(al2, t.y[rc]) : m0);
+    const double bT = hasL ? add(add(mul(al1, t.c[lc]), t.b[k]), hasR ? mul(al2, t.a[rc]) : m0) : 0.0;
+    const double dT = hasR ? add(add(hasL ? mul(al1, t.e[lc]) : m0, t.d[k]), mul(al2, t.c[rc])) : 0.0;
+    const double aT = hasL ? mul(al1, t.a[lc]) : 0.0, eT = hasR ? mul(al2, t.e[rc]) : 0.0;
+    t.Ta[k] = aT; t.Tb[k] = bT; t.Tc[k] = cT; t.Td[k] = dT; t.Te[k] = eT; t.Ty[k] = kT;
+    t.Tr[k] = ieee::recip(cT);
+    return cT;
+}
+
+// f1, f2 enter as the multipliers a zero pivot leaves in place (kernel.cu:122,129)
+template <int CAP>
+__device__ __forceinline__ double2 row_b_general(TileRows<CAP>& t, int k, int dl, bool hasL, bool hasR, double f1, double f2)
+{
+    const int l = k - dl, r = k + dl;
+    double a1 = 0.0, b1 = 0.0, c1 = 0.0, d1 = 0.0, k1 = 0.0;
+    double b2 = 0.0, c2 = 0.0, d2 = 0.0, e2 = 0.0, k2 = 0.0;
+    if (hasL) {                            // kernel.cu:120-125
+        if (nz(t.Tc[l])) f1 = quot(t.b[k], t.Tc[l], t.Tr[l]);
+        a1 = mul(f1, t.Ta[l]); b1 = mul(f1, t.Tb[l]); c1 = mul(f1, t.Td[l]);
+        d1 = mul(f1, t.Te[l]); k1 = mul(f1, t.Ty[l]);
+    }
+    if (hasR) {                            // kernel.cu:127-132
+        if (nz(t.Tc[r])) f2 = quot(t.d[k], t.Tc[r], t.Tr[r]);
+        c2 = mul(f2, t.Tb[r]); b2 = mul(f2, t.Ta[r]); d2 = mul(f2, t.Td[r]);
+        e2 = mul(f2, t.Te[r]); k2 = mul(f2, t.Ty[r]);
+    }
+    t.b[k] = add(sub(b1, t.a[k]), b2);     // kernel.cu:138-140
+    t.c[k] = add(sub(c1, t.c[k]), c2);
+    t.d[k] = add(sub(d1, t.e[k]), d2);
+    t.y[k] = add(sub(k1, t.y[k]), k2);
+    t.a[k] = a1; t.e[k] = e2;
+    return make_double2(f1, f2);
+}
+
+// Phase A's multipliers of row m (T(m) = left*row(m-d) + row(m) +
+// right*row(m+d)), formed again
+template <int CAP>
+__device__ __noinline__ double multiplier_left(TileRows<CAP>& t, int m, int dl, int kfirst)
+{
+    return m - 2 * dl >= kfirst && nz(t.b[m - dl]) ? quot(neg(t.a[m]), t.b[m - dl]) : 0.0;
+}
+template <int CAP>
+__device__ __noinline__ double multiplier_right(TileRows<CAP>& t, int m, int dl, int klast)
+{
+    return m + 2 * dl <= klast && nz(t.d[m + dl]) ? quot(neg(t.e[m]), t.d[m + dl]) : 0.0;
+}
+
+// Row k couples to no other row, and no product of its c and y with another
+// such row's can leave the normal range.
+template <int CAP>
+__device__ __forceinline__ bool decoupled(TileRows<CAP>& t, int k)
+{
+    return zeros(t.a[k], t.b[k], t.d[k]) && !nz(t.e[k]) && ieee::mid(t.c[k]) && ieee::mid(t.y[k]);
+}
 
 // Global loads of the state; kL2Only reads through L2 only (ld.global.cg), for
 // persistent kernels that read data other CTAs wrote earlier in the same launch.
@@ -91,19 +406,9 @@ __device__ __forceinline__ double gload(const double* p) {
 
 // One CTA's work: window w of subsystem r of system j (whole subsystem when
 // p.final_step).  Every thread of the CTA must call it with the same (j, r, w).
-// kZero compiles the zero-state vote and its integer-pipe strides in; without
-// it every stride takes the FP64 operations (passes of short strides, where
-// the outer coefficients have not underflowed yet, skip the vote's cost).
-template <int RPT, bool kL2Only = false, bool kZero = true>
-__device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_t r, int64_t w, double* smem)
+template <int CAP, bool kL2Only = false>
+__device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_t r, int64_t w, TileRows<CAP>& T)
 {
-    const int TRm = p.TRmax;
-    double* sa = smem;            double* sb = sa + TRm;  double* sc = sb + TRm;
-    double* sd = sc + TRm;        double* se = sd + TRm;  double* sy = se + TRm;
-    double* Ta = sy + TRm;        double* Tb = Ta + TRm;  double* Tc = Tb + TRm;
-    double* Td = Tc + TRm;        double* Te = Td + TRm;  double* Tk = Te + TRm;
-    double* T1 = Tk + TRm;        double* T2 = T1 + TRm;  double* Tr = T2 + TRm;
-
     const int64_t sbase = p.offsets ? p.offsets[j] : j * p.src_ss;
     const int64_t dbase = p.offsets ? p.offsets[j] : j * p.dst_ss;
     const int64_t nsys = p.offsets ? (p.offsets[j + 1] - p.offsets[j]) : p.n;
@@ -130,9 +435,14 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_
     const double* __restrict__ ge = has_e ? p.src[E_] + soff : nullptr;
     const double* __restrict__ gy = p.src[Y_] + soff;
 
-    double al1p[RPT], al2p[RPT];
-    bool zrow = true;           // every row this thread holds in the zero state
-    bool zdrow = true;          // ... with d = 0 as well
+    // The multipliers of phase B that the reference keeps from one stride to
+    // the next (kernel.cu:60) are read in one case only: in the last stride of
+    // a whole subsystem, by a row whose pivot cT is exactly zero and that has
+    // no other multiplier of that stride (kernel.cu:122,129): fewer than 3*dl
+    // rows are left then, and a subsystem with p.rem strides to go has at least
+    // 2^p.rem rows.  So they are kept (in local memory) by the last stride but
+    // one, and pass through global memory only if a global pass ends with it.
+    double kept1[kMaxRowsPerThread], kept2[kMaxRowsPerThread];
     if (p.bulk) {
         // The whole system is the tile (t0 = 0, TR = n, even): thread 0
         // stages each array with one bulk asynchronous copy straight into its
@@ -150,12 +460,12 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_
             const uint32_t bytes = (uint32_t)TR * (uint32_t)sizeof(double);
             const uint64_t pol = tma::policy_evict_first();
             tma::mbar_expect_tx(&bulk_bar, (4u + (has_a ? 1u : 0u) + (has_e ? 1u : 0u)) * bytes);
-            if (has_a) tma::bulk_g2s(sa, ga, bytes, &bulk_bar, pol);
-            tma::bulk_g2s(sb, gb, bytes, &bulk_bar, pol);
-            tma::bulk_g2s(sc, gc, bytes, &bulk_bar, pol);
-            tma::bulk_g2s(sd, gd, bytes, &bulk_bar, pol);
-            if (has_e) tma::bulk_g2s(se, ge, bytes, &bulk_bar, pol);
-            tma::bulk_g2s(sy, gy, bytes, &bulk_bar, pol);
+            if (has_a) tma::bulk_g2s(T.a, ga, bytes, &bulk_bar, pol);
+            tma::bulk_g2s(T.b, gb, bytes, &bulk_bar, pol);
+            tma::bulk_g2s(T.c, gc, bytes, &bulk_bar, pol);
+            tma::bulk_g2s(T.d, gd, bytes, &bulk_bar, pol);
+            if (has_e) tma::bulk_g2s(T.e, ge, bytes, &bulk_bar, pol);
+            tma::bulk_g2s(T.y, gy, bytes, &bulk_bar, pol);
         }
         const bool got = tma::mbar_wait_bounded(&bulk_bar, 0, 2000000000ull);
         if (__syncthreads_or(!got)) {
@@ -165,334 +475,145 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_
             for (int k = tid; k < TR; k += bd) gx[k * dstep] = __longlong_as_double(0x7FF8000000000000LL);
             return;
         }
-#pragma unroll
-        for (int q = 0; q < RPT; q++) {
-            const int k = tid + q * bd;
-            al1p[q] = 0.0; al2p[q] = 0.0;
-            if (k < TR) {
-                if (!has_a) sa[k] = 0.0;
-                if (!has_e) se[k] = 0.0;
-                if constexpr (kZero) {
-                    const bool z = zero_state(sa[k], sb[k], sc[k], sd[k], se[k], sy[k]);
-                    zrow = zrow && z; zdrow = zdrow && z && !nz(sd[k]);
-                }
-            }
+        for (int k = tid; k < TR; k += bd) {
+            if (!has_a) T.a[k] = 0.0;
+            if (!has_e) T.e[k] = 0.0;
         }
     } else {
-    #pragma unroll
-        for (int q = 0; q < RPT; q++) {
-            const int k = tid + q * bd;
-            al1p[q] = 0.0; al2p[q] = 0.0;
-            if (k < TR) {
-                const int64_t gi = (t0 + k) * sstep;
-                const double a = has_a ? gload<kL2Only>(ga + gi) : 0.0;
-                const double e = has_e ? gload<kL2Only>(ge + gi) : 0.0;
-                const double b = gload<kL2Only>(gb + gi), c = gload<kL2Only>(gc + gi);
-                const double d = gload<kL2Only>(gd + gi), y = gload<kL2Only>(gy + gi);
-                sa[k] = a; sb[k] = b; sc[k] = c; sd[k] = d; se[k] = e; sy[k] = y;
-                if constexpr (kZero) {
-                    const bool z = zero_state(a, b, c, d, e, y);
-                    zrow = zrow && z; zdrow = zdrow && z && !nz(d);
-                }
-                if (p.src[AL1_]) {
-                    al1p[q] = gload<kL2Only>(p.src[AL1_] + soff + gi);
-                    al2p[q] = gload<kL2Only>(p.src[AL2_] + soff + gi);
-                }
-            }
+#pragma unroll 2
+        for (int k = tid; k < TR; k += bd) {
+            const int64_t gi = (t0 + k) * sstep;
+            const double a = has_a ? gload<kL2Only>(ga + gi) : 0.0;
+            const double e = has_e ? gload<kL2Only>(ge + gi) : 0.0;
+            const double b = gload<kL2Only>(gb + gi), c = gload<kL2Only>(gc + gi);
+            const double d = gload<kL2Only>(gd + gi), y = gload<kL2Only>(gy + gi);
+            T.a[k] = a; T.b[k] = b; T.c[k] = c; T.d[k] = d; T.e[k] = e; T.y[k] = y;
         }
     }
-    // rows read by a stride are the rows the previous stride wrote (all
-    // loaded rows for the first): votes per stride tell whether the whole
-    // tile is in the zero state, and in it with d = 0 too
-    int ztile = 0, zdtile = 0;
-    if constexpr (kZero) { ztile = __syncthreads_and(zrow); zdtile = __syncthreads_and(zdrow); }
-    else __syncthreads();
+    if (p.rem == 1)
+        for (int k = tid, q = 0; k < TR; k += bd, q++) {
+            const int64_t gi = soff + (t0 + k) * sstep;
+            kept1[q] = p.src[AL1_] ? gload<kL2Only>(p.src[AL1_] + gi) : 0.0;
+            kept2[q] = p.src[AL1_] ? gload<kL2Only>(p.src[AL2_] + gi) : 0.0;
+        }
+    // local rows of the subsystem's ends: row k of the tile has a neighbour at
+    // distance x iff k - x >= kfirst / k + x <= klast (32-bit: ends further
+    // away than any distance of the tile are moved in to 2^14 rows)
+    const int kfirst = -(int)min(t0, (int64_t)16384), klast = (int)min(nr - 1 - t0, (int64_t)16384);
 
-    for (int s = 0; s < p.K; s++) {
+    // A whole subsystem whose rows are all decoupled (a = b = d = e = 0, c and
+    // y away from the ends of the exponent range): every further stride only
+    // changes the signs of c and y of every row, which the final step's
+    // products and quotients cancel, so the remaining strides are skipped.
+    bool apart = p.final_step != 0;
+    if (apart)
+        for (int k = tid; k < TR; k += bd) apart = apart && decoupled(T, k);
+    const int strides = __syncthreads_and(apart) ? 0 : p.K;
+
+    for (int s = 0; s < strides; s++) {
         const int dl = 1 << s;
         // rows this stride must produce: the window widened by the halo the
         // remaining strides of the pass still consume (everything if final).
-        int64_t rlo, rhi;
-        if (p.final_step) { rlo = 0; rhi = nr; }
+        int klo, khi;
+        if (p.final_step) { klo = 0; khi = TR; }
         else {
             const int64_t rem = 2 * ((int64_t(1) << p.K) - (int64_t(2) << s));
-            rlo = max(wlo - rem, (int64_t)0); rhi = min(whi + rem, nr);
+            klo = (int)(max(wlo - rem, (int64_t)0) - t0); khi = (int)(min(whi + rem, nr) - t0);
         }
-        const int64_t Tlo = max(rlo - dl, (int64_t)0), Thi = min(rhi + dl, nr);
+        // the rows whose T(m) those need, all in the tile
+        const int Alo = max(klo - dl, 0), Ahi = min(khi + dl, TR);
 
         // ---- phase A: T(m) = a1*row(m-d) + row(m) + a2*row(m+d) ----------
-        if (kZero && ztile) {
-            // a1 = -a(m)/b(m-d) and a2 = -e(m)/d(m+d) are zeros (b, d finite):
-            // only their signs are formed; every product with them is the
-            // zero of sign xor, every sum row m's value (kernel.cu:63-117)
-#pragma unroll
-            for (int q = 0; q < RPT; q++) {
-                const int k = tid + q * bd;
-                const int64_t t = t0 + k;
-                if (k < TR && t >= Tlo && t < Thi) {
-                    const bool hasL = t - dl >= 0, hasR = t + dl <= nr - 1;
-                    if (hasL || hasR) {
-                        const double bm = sb[k], cm = sc[k], dm = sd[k], ym = sy[k];
-                        unsigned s1 = 0u, s2 = 0u;
-                        if (hasL && t - 2 * dl >= 0) {
-                            const double bL = sb[k - dl];
-                            if (nz(bL)) s1 = (hiw(sa[k]) ^ hiw(bL)) ^ 0x80000000u;
-                        }
-                        if (hasR && t + 2 * dl <= nr - 1) {
-                            const double dR = sd[k + dl];
-                            if (nz(dR)) s2 = (hiw(se[k]) ^ hiw(dR)) ^ 0x80000000u;
-                        }
-                        // sign bits of the products a1*row(m-d) and a2*row(m+d)
-                        // (+0 for a missing neighbour: adding +0 keeps -0 out)
-                        unsigned La = 0u, Lc = 0u, Ld = 0u, Le = 0u, Ly = 0u;
-                        unsigned Ra = 0u, Rb = 0u, Rc = 0u, Re = 0u, Ry = 0u;
-                        if (hasL) {
-                            La = s1 ^ hiw(sa[k - dl]); Lc = s1 ^ hiw(sc[k - dl]); Ld = s1 ^ hiw(sd[k - dl]);
-                            Le = s1 ^ hiw(se[k - dl]); Ly = s1 ^ hiw(sy[k - dl]);
-                        }
-                        if (hasR) {
-                            Ra = s2 ^ hiw(sa[k + dl]); Rb = s2 ^ hiw(sb[k + dl]); Rc = s2 ^ hiw(sc[k + dl]);
-                            Re = s2 ^ hiw(se[k + dl]); Ry = s2 ^ hiw(sy[k + dl]);
-                        }
-                        if (hasL && hasR) {
-                            Ta[k] = szero(La);
-                            Tb[k] = add_z(bm, Lc & Ra); Tc[k] = add_z(cm, Ld & Rb);
-                            Td[k] = add_z(dm, Le & Rc); Te[k] = szero(Re);
-                            Tk[k] = add_z(ym, Ly & Ry);
-                        } else if (hasR) {     // kernel.cu:82-91: aT = bT = 0
-                            Ta[k] = 0.0; Tb[k] = 0.0;
-                            Tc[k] = add_z(cm, Rb); Td[k] = add_z(dm, Rc); Te[k] = szero(Re);
-                            Tk[k] = add_z(ym, Ry);
-                        } else {               // kernel.cu:108-117: dT = eT = 0
-                            Ta[k] = szero(La); Tb[k] = add_z(bm, Lc); Tc[k] = add_z(cm, Ld);
-                            Td[k] = 0.0; Te[k] = 0.0;
-                            Tk[k] = add_z(ym, Ly);
-                        }
-                        T1[k] = szero(s1); T2[k] = szero(s2);
-                    }
-                }
+        bool zero_pivot = false;
+#pragma unroll 1
+        for (int k = tid; k < TR; k += bd) {
+            if (k < Alo || k >= Ahi) continue;
+            const bool hasL = k - dl >= kfirst, hasR = k + dl <= klast;
+            const bool has2L = k - 2 * dl >= kfirst, has2R = k + 2 * dl <= klast;
+            if (!(hasL || hasR)) continue;
+            const bool left = has2L && nz(T.a[k]), right = has2R && nz(T.e[k]);   // nonzero multipliers
+            // rows near the subsystem's ends, where neighbouring rows hold
+            // structural zeros, take the general form at once
+            double cT;
+            bool done = false;
+            if (!left && !right) done = row_a_none(T, k, dl, hasL, has2L, hasR, has2R, cT);
+            else if (has2L && has2R) {
+                if (left && right) done = row_a_both(T, k, dl, cT);
+                else done = row_a_one(T, k, dl, right, cT);
+                if (!done) done = row_a_tiny(T, k, dl, hasL, has2L, hasR, has2R, cT);
             }
-        } else {
-#pragma unroll
-        for (int q = 0; q < RPT; q++) {
-            const int k = tid + q * bd;
-            const int64_t t = t0 + k;
-            if (k < TR && t >= Tlo && t < Thi) {
-                const bool hasL = t - dl >= 0, hasR = t + dl <= nr - 1;
-                if (hasL || hasR) {
-                    const double am = sa[k], bm = sb[k], cm = sc[k], dm = sd[k], em = se[k], ym = sy[k];
-                    double al1 = 0.0, al2 = 0.0;
-                    double aT, bT, cT, dT, eT, kT;
-                    if (hasL && hasR) {
-                        const double aL = sa[k - dl], bL = sb[k - dl], cL = sc[k - dl], dL = sd[k - dl],
-                                     eL = se[k - dl], yL = sy[k - dl];
-                        const double aR = sa[k + dl], bR = sb[k + dl], cR = sc[k + dl], dR = sd[k + dl],
-                                     eR = se[k + dl], yR = sy[k + dl];
-                        if (t - 2 * dl >= 0 && nz(bL)) al1 = dvd(neg(am), bL);
-                        if (t + 2 * dl <= nr - 1 && nz(dR)) al2 = dvd(neg(em), dR);
-                        aT = mul(al1, aL);
-                        bT = add(add(mul(al1, cL), bm), mul(al2, aR));
-                        cT = add(add(mul(al1, dL), cm), mul(al2, bR));
-                        dT = add(add(mul(al1, eL), dm), mul(al2, cR));
-                        eT = mul(al2, eR);
-                        kT = add(add(mul(al1, yL), ym), mul(al2, yR));
-                    } else if (hasR) {     // row m-d outside: kernel.cu:82-91
-                        const double aR = sa[k + dl], bR = sb[k + dl], cR = sc[k + dl], dR = sd[k + dl],
-                                     eR = se[k + dl], yR = sy[k + dl];
-                        (void)aR;
-                        if (t + 2 * dl <= nr - 1 && nz(dR)) al2 = dvd(neg(em), dR);
-                        aT = 0.0; bT = 0.0;
-                        cT = add(cm, mul(al2, bR));
-                        dT = add(dm, mul(al2, cR));
-                        eT = mul(al2, eR);
-                        kT = add(ym, mul(al2, yR));
-                    } else {               // row m+d outside: kernel.cu:108-117
-                        const double aL = sa[k - dl], bL = sb[k - dl], cL = sc[k - dl], dL = sd[k - dl],
-                                     yL = sy[k - dl];
-                        if (t - 2 * dl >= 0 && nz(bL)) al1 = dvd(neg(am), bL);
-                        aT = mul(al1, aL);
-                        bT = add(mul(al1, cL), bm);
-                        cT = add(mul(al1, dL), cm);
-                        dT = 0.0; eT = 0.0;
-                        kT = add(mul(al1, yL), ym);
-                        (void)em;
-                    }
-                    Ta[k] = aT; Tb[k] = bT; Tc[k] = cT; Td[k] = dT; Te[k] = eT; Tk[k] = kT;
-                    T1[k] = al1; T2[k] = al2;
-                    Tr[k] = __drcp_rn(cT);
-                }
+            if (!done) cT = row_a_general(T, k, dl, hasL, has2L, hasR, has2R);
+            zero_pivot = zero_pivot || !nz(cT);
+        }
+        double pre1[kMaxRowsPerThread], pre2[kMaxRowsPerThread];
+        if (__syncthreads_or(zero_pivot)) {
+            // some pivot cT of the tile is exactly zero: the multipliers the
+            // reference then uses (kernel.cu:96-112), from the state before
+            // phase B changes it
+            for (int k = tid, q = 0; k < TR; k += bd, q++) {
+                const bool hasL = k - dl >= kfirst, hasR = k + dl <= klast;
+                const bool has2L = k - 2 * dl >= kfirst, has2R = k + 2 * dl <= klast;
+                if (k < klo || k >= khi) continue;
+                pre1[q] = hasR ? multiplier_left(T, k + dl, dl, kfirst)
+                               : has2L ? multiplier_left(T, k - dl, dl, kfirst) : kept1[q];
+                pre2[q] = has2R ? multiplier_right(T, k + dl, dl, klast)
+                                : hasL ? multiplier_right(T, k - dl, dl, klast) : kept2[q];
             }
+            __syncthreads();
         }
-        }
-        __syncthreads();
 
         // ---- phase B: new row = b/cT(i-d)*T(i-d) - row(i) + d/cT(i+d)*T(i+d)
-        zrow = true; zdrow = true;
-        // the reference's update of row i (kernel.cu:120-140, in place: phase
-        // B reads no other row's state); folds the row's zero state into zrow
-        auto row_b = [&](int q, int k, bool hasL, bool hasR, double a1pre, double a2pre, bool rcp) {
-            const double ai = sa[k], bi = sb[k], ci = sc[k], di = sd[k], ei = se[k], yi = sy[k];
-            double a1 = 0.0, b1 = 0.0, c1 = 0.0, d1 = 0.0, k1 = 0.0, f1 = a1pre;
-            double b2 = 0.0, c2 = 0.0, d2 = 0.0, e2 = 0.0, k2 = 0.0, f2 = a2pre;
-            if (hasL) {                    // kernel.cu:120-125
-                const double cTL = Tc[k - dl];
-                if (nz(cTL)) f1 = rcp ? mdiv(bi, cTL, Tr[k - dl]) : dvd(bi, cTL);
-                a1 = mul(f1, Ta[k - dl]); b1 = mul(f1, Tb[k - dl]); c1 = mul(f1, Td[k - dl]);
-                d1 = mul(f1, Te[k - dl]); k1 = mul(f1, Tk[k - dl]);
-            }
-            if (hasR) {                    // kernel.cu:127-132
-                const double cTR = Tc[k + dl];
-                if (nz(cTR)) f2 = rcp ? mdiv(di, cTR, Tr[k + dl]) : dvd(di, cTR);
-                c2 = mul(f2, Tb[k + dl]); b2 = mul(f2, Ta[k + dl]); d2 = mul(f2, Td[k + dl]);
-                e2 = mul(f2, Te[k + dl]); k2 = mul(f2, Tk[k + dl]);
-            }
-            const double nb = add(sub(b1, ai), b2), nc = add(sub(c1, ci), c2);   // kernel.cu:138-140
-            const double nd = add(sub(d1, ei), d2), ny = add(sub(k1, yi), k2);
-            sb[k] = nb; sc[k] = nc; sd[k] = nd; sy[k] = ny;
-            sa[k] = a1; se[k] = e2;
-            al1p[q] = f1; al2p[q] = f2;
-            if constexpr (kZero) {
-                const bool z = zero_state(a1, nb, nc, nd, e2, ny);
-                zrow = zrow && z; zdrow = zdrow && z && !nz(nd);
-            }
-        };
-        if (kZero && zdtile) {
-            // zero state with d = 0: f2 = d(i)/cT(i+d) is a zero, and so is
-            // every product with it; dT of the neighbours is zero, so c1 is
-            // too: besides the quotient f1 only b1, k1 and k1 - y(i) are FP64
-#pragma unroll
-            for (int q = 0; q < RPT; q++) {
-                const int k = tid + q * bd;
-                const int64_t t = t0 + k;
-                if (k < TR && t >= rlo && t < rhi) {
-                    const bool hasL = t - dl >= 0, hasR = t + dl <= nr - 1;
-                    // multipliers last assigned before Reduction-III (kernel.cu:96-112)
-                    const double a1pre = hasR ? T1[k + dl] : ((t - 2 * dl >= 0) ? T1[k - dl] : al1p[q]);
-                    const double a2pre = (t + 2 * dl <= nr - 1) ? T2[k + dl] : (hasL ? T2[k - dl] : al2p[q]);
-                    double f1 = a1pre, f2 = a2pre;
-                    if (hasL) { const double cTL = Tc[k - dl]; if (nz(cTL)) f1 = dvd(sb[k], cTL); }
-                    if (hasR) { const double cTR = Tc[k + dl]; if (nz(cTR)) f2 = dvd(sd[k], cTR); }
-                    // f2 is the stored multiplier where cT(i+d) = 0: then the row
-                    // takes the reference's operations
-                    if (finite4(hasL ? f1 : 0.0, 0.0, 0.0, 0.0) && (!hasR || !nz(f2))) {
-                        const double ai = sa[k], ci = sc[k], ei = se[k], yi = sy[k];
-                        const unsigned s1 = hiw(f1), s2 = hiw(f2);
-                        unsigned a1s = 0u, c1s = 0u, d1s = 0u, b2s = 0u, c2s = 0u, d2s = 0u, e2s = 0u, k2s = 0u;
-                        double b1 = 0.0, k1 = 0.0;
-                        if (hasL) {
-                            a1s = s1 ^ hiw(Ta[k - dl]); c1s = s1 ^ hiw(Td[k - dl]); d1s = s1 ^ hiw(Te[k - dl]);
-                            b1 = mul(f1, Tb[k - dl]); k1 = mul(f1, Tk[k - dl]);
-                        }
-                        if (hasR) {
-                            b2s = s2 ^ hiw(Ta[k + dl]); c2s = s2 ^ hiw(Tb[k + dl]); d2s = s2 ^ hiw(Td[k + dl]);
-                            e2s = s2 ^ hiw(Te[k + dl]); k2s = s2 ^ hiw(Tk[k + dl]);
-                        }
-                        // (b1 - ai) + b2, (c1 - ci) + c2, (d1 - ei) + d2, (k1 - yi) + k2
-                        // with zeros ai, b2, c1, c2, d1, ei, d2, k2
-                        const double nb = add_z(add_z(b1, hiw(ai) ^ 0x80000000u), b2s);
-                        const double nc = add_z(add_z(neg(ci), c1s), c2s);
-                        const double nd = szero(d1s & (hiw(ei) ^ 0x80000000u) & d2s);
-                        const double ny = add_z(sub(k1, yi), k2s);
-                        sb[k] = nb; sc[k] = nc; sd[k] = nd; sy[k] = ny;
-                        sa[k] = szero(a1s); se[k] = szero(e2s);
-                        al1p[q] = f1; al2p[q] = f2;
-                        const bool z = finite4(nb, nc, nd, ny);
-                        zrow = zrow && z; zdrow = zdrow && z;
-                    } else {
-                        row_b(q, k, hasL, hasR, a1pre, a2pre, false);
-                    }
+        // (in place: phase B reads no other row's state)
+        apart = p.final_step != 0;
+        const bool keep = s == p.rem - 2;
+#pragma unroll 1
+        for (int k = tid, q = 0; k < TR; k += bd, q++) {
+            if (k < klo || k >= khi) continue;
+            const bool hasL = k - dl >= kfirst, hasR = k + dl <= klast;
+            const bool left = hasL && nz(T.b[k]), right = hasR && nz(T.d[k]);
+            double f1 = 0.0, f2 = 0.0;
+            bool done = false;
+            if (!left && !right) done = row_b_none(T, k, dl, hasL, hasR, f1, f2);
+            else if (k - 3 * dl >= kfirst && k + 3 * dl <= klast) {
+                if (left && right) {
+                    const bool za = !nz(T.a[k]), ze = !nz(T.e[k]);
+                    if (za && ze) done = row_b_both<true, true>(T, k, dl, f1, f2);
+                    else if (za) done = row_b_both<true, false>(T, k, dl, f1, f2);
+                    else done = row_b_both<false, false>(T, k, dl, f1, f2);
                 }
+                if (!done) done = row_b_tiny(T, k, dl, hasL, hasR, f1, f2);
             }
-        } else if (kZero && ztile) {
-            // zero state: aT, eT of both neighbours and a, e of row i are
-            // zeros, so are a1, d1, b2, e2 (for finite f1, f2), and the b and
-            // d sums reduce to one term
-#pragma unroll
-            for (int q = 0; q < RPT; q++) {
-                const int k = tid + q * bd;
-                const int64_t t = t0 + k;
-                if (k < TR && t >= rlo && t < rhi) {
-                    const bool hasL = t - dl >= 0, hasR = t + dl <= nr - 1;
-                    // multipliers last assigned before Reduction-III (kernel.cu:96-112)
-                    const double a1pre = hasR ? T1[k + dl] : ((t - 2 * dl >= 0) ? T1[k - dl] : al1p[q]);
-                    const double a2pre = (t + 2 * dl <= nr - 1) ? T2[k + dl] : (hasL ? T2[k - dl] : al2p[q]);
-                    double f1 = a1pre, f2 = a2pre;
-                    if (hasL) { const double cTL = Tc[k - dl]; if (nz(cTL)) f1 = dvd(sb[k], cTL); }
-                    if (hasR) { const double cTR = Tc[k + dl]; if (nz(cTR)) f2 = dvd(sd[k], cTR); }
-                    if (finite4(hasL ? f1 : 0.0, hasR ? f2 : 0.0, 0.0, 0.0)) {
-                        const double ai = sa[k], ci = sc[k], ei = se[k], yi = sy[k];
-                        const unsigned s1 = hiw(f1), s2 = hiw(f2);
-                        unsigned a1s = 0u, d1s = 0u, b2s = 0u, e2s = 0u;
-                        double b1 = 0.0, c1 = 0.0, k1 = 0.0, c2 = 0.0, d2 = 0.0, k2 = 0.0;
-                        if (hasL) {
-                            a1s = s1 ^ hiw(Ta[k - dl]); d1s = s1 ^ hiw(Te[k - dl]);
-                            b1 = mul(f1, Tb[k - dl]); c1 = mul(f1, Td[k - dl]); k1 = mul(f1, Tk[k - dl]);
-                        }
-                        if (hasR) {
-                            b2s = s2 ^ hiw(Ta[k + dl]); e2s = s2 ^ hiw(Te[k + dl]);
-                            c2 = mul(f2, Tb[k + dl]); d2 = mul(f2, Td[k + dl]); k2 = mul(f2, Tk[k + dl]);
-                        }
-                        // b1 - ai + b2 with ai, b2 zeros; d1 - ei + d2 with d1, ei zeros
-                        const double nb = add_z(add_z(b1, hiw(ai) ^ 0x80000000u), b2s);
-                        const double nc = add(sub(c1, ci), c2);
-                        const double nd = add_z(d2, d1s & (hiw(ei) ^ 0x80000000u));
-                        const double ny = add(sub(k1, yi), k2);
-                        sb[k] = nb; sc[k] = nc; sd[k] = nd; sy[k] = ny;
-                        sa[k] = szero(a1s); se[k] = szero(e2s);
-                        al1p[q] = f1; al2p[q] = f2;
-                        const bool z = finite4(nb, nc, nd, ny);
-                        zrow = zrow && z; zdrow = zdrow && z && !nz(nd);
-                    } else {
-                        row_b(q, k, hasL, hasR, a1pre, a2pre, false);
-                    }
-                }
+            if (!done) {
+                const double2 f = row_b_general(T, k, dl, hasL, hasR, pre1[q], pre2[q]);
+                f1 = f.x; f2 = f.y;
             }
-        } else {
-#pragma unroll
-            for (int q = 0; q < RPT; q++) {
-                const int k = tid + q * bd;
-                const int64_t t = t0 + k;
-                if (k < TR && t >= rlo && t < rhi) {
-                    const bool hasL = t - dl >= 0, hasR = t + dl <= nr - 1;
-                    // multipliers last assigned before Reduction-III (kernel.cu:96-112)
-                    const double a1pre = hasR ? T1[k + dl] : ((t - 2 * dl >= 0) ? T1[k - dl] : al1p[q]);
-                    const double a2pre = (t + 2 * dl <= nr - 1) ? T2[k + dl] : (hasL ? T2[k - dl] : al2p[q]);
-                    row_b(q, k, hasL, hasR, a1pre, a2pre, true);
-                }
-            }
+            apart = apart && !left && !right && decoupled(T, k);
+            if (keep) { kept1[q] = f1; kept2[q] = f2; }
         }
-        if constexpr (kZero) { ztile = __syncthreads_and(zrow); zdtile = __syncthreads_and(zdrow); }
-        else __syncthreads();
+        if (__syncthreads_and(apart)) break;
     }
 
     if (p.final_step) {
         // kernel.cu:145-153: pairs (i, i+delta) by Cramer's rule, singles x = y/c
-        const int64_t df = int64_t(1) << p.K;
+        const int df = 1 << p.K;
         double* __restrict__ gx = p.x + doff;
-#pragma unroll
-        for (int q = 0; q < RPT; q++) {
-            const int k = tid + q * bd;
-            if (k < TR) {
-                const int64_t t = k;       // whole subsystem: t0 == 0
-                if (t < nr - df) {
-                    const int kk = k + (int)df;
-                    const double deno = sub(mul(sc[k], sc[kk]), mul(sb[kk], sd[k]));
-                    gx[t * dstep] = dvd(sub(mul(sc[kk], sy[k]), mul(sd[k], sy[kk])), deno);
-                    gx[(t + df) * dstep] = dvd(sub(mul(sc[k], sy[kk]), mul(sb[kk], sy[k])), deno);
-                }
-                if (t >= nr - df && t < df) gx[t * dstep] = dvd(sy[k], sc[k]);
+        for (int k = tid; k < TR; k += bd) {       // whole subsystem: t0 == 0, TR == nr
+            if (k < TR - df) {
+                const int kk = k + df;
+                const double deno = sub(mul(T.c[k], T.c[kk]), mul(T.b[kk], T.d[k]));
+                gx[k * dstep] = quot(sub(mul(T.c[kk], T.y[k]), mul(T.d[k], T.y[kk])), deno);
+                gx[kk * dstep] = quot(sub(mul(T.c[k], T.y[kk]), mul(T.b[kk], T.y[k])), deno);
             }
+            if (k >= TR - df && k < df) gx[k * dstep] = quot(T.y[k], T.c[k]);
         }
     } else {
         // subsystem-major output: row t of subsystem r is row t >> K of
         // subsystem r + (t mod 2^K) G at the next level's stride G 2^K
         const int64_t G2 = p.G << p.K, q2 = nsys / G2, rem2 = nsys % G2;
         const int64_t kmask = (int64_t(1) << p.K) - 1;
-#pragma unroll
-        for (int q = 0; q < RPT; q++) {
-            const int k = tid + q * bd;
+        for (int k = tid, q = 0; k < TR; k += bd, q++) {
             const int64_t t = t0 + k;
-            if (k < TR && t >= wlo && t < whi) {
+            if (t >= wlo && t < whi) {
                 int64_t gi;
                 if (p.dst_sub) {
                     const int64_t r2 = r + (t & kmask) * p.G;
@@ -500,9 +621,9 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_
                 } else {
                     gi = doff + t * dstep;
                 }
-                p.dst[A_][gi] = sa[k]; p.dst[B_][gi] = sb[k]; p.dst[C_][gi] = sc[k];
-                p.dst[D_][gi] = sd[k]; p.dst[E_][gi] = se[k]; p.dst[Y_][gi] = sy[k];
-                p.dst[AL1_][gi] = al1p[q]; p.dst[AL2_][gi] = al2p[q];
+                p.dst[A_][gi] = T.a[k]; p.dst[B_][gi] = T.b[k]; p.dst[C_][gi] = T.c[k];
+                p.dst[D_][gi] = T.d[k]; p.dst[E_][gi] = T.e[k]; p.dst[Y_][gi] = T.y[k];
+                if (p.rem == p.K + 1) { p.dst[AL1_][gi] = kept1[q]; p.dst[AL2_][gi] = kept2[q]; }
             }
         }
     }

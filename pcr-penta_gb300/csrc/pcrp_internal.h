@@ -46,7 +46,7 @@ __host__ __device__ inline int ref_strides(int64_t n) {
 // subsystem contiguous, so a pass reads its subsystem's rows in one run
 // instead of G*8 bytes apart.
 struct PcrPassArgs {
-    const double* src[NSTATE];   // state in (A_/E_/AL1_/AL2_ may be null: zeros)
+    const double* src[NSTATE];   // state in (A_/E_/AL1_ may be null: zeros)
     double* dst[NSTATE];         // state out (non-final passes)
     double* x;                   // solution out (final pass)
     const int64_t* offsets;      // ragged first rows (nullable); ragged data is contiguous
@@ -57,6 +57,8 @@ struct PcrPassArgs {
     int64_t G;                   // gather stride = 2^(strides already done)
     int64_t nwin;                // windows per subsystem
     int K;                       // strides run by this pass (local deltas 1..2^(K-1))
+    int rem;                     // strides the subsystems have left, this pass's included; the AL1_/AL2_ arrays
+                                 // are written by a pass that leaves one stride and read by the next
     int final_step;              // 1: whole subsystem per CTA, finish and write x
     int L;                       // rows written per window (local)
     int H;                       // halo rows on each side (local), 2*(2^K-1)
@@ -67,28 +69,13 @@ struct PcrPassArgs {
                                  // arrays: the tile is staged by bulk asynchronous copies (one per array)
 };
 
-// Passes whose longest stride reaches kZeroStride rows vote on the zero
-// state: the outer coefficients of diagonally dominant systems underflow at
-// strides ~2^8-2^10, and the vote (~10% of a dense stride) pays once two or
-// more strides of the pass run in that state.  Others run without it, unless
-// the batch is tridiagonal (a = e = 0 on entry): then every stride of every
-// pass is in that state and every pass votes.  (Same bits either way.)
-constexpr int64_t kZeroStride = 1024;
-__host__ __device__ inline bool pass_votes(const PcrPassArgs& p, bool tridiagonal)
-{
-    return tridiagonal || (p.K > 0 && (p.G << (p.K - 1)) >= kZeroStride);
-}
-
-
-// Host-side launchers (pcr_f64.cu).  `tridiagonal`: the batch entered with
-// a = e = 0, so every pass compiles in the zero-state vote.
-cudaError_t launch_pcr_pass(const PcrPassArgs& p, int threads, cudaStream_t s, bool tridiagonal = false);
+// Host-side launchers (pcr_f64.cu).
+cudaError_t launch_pcr_pass(const PcrPassArgs& p, int threads, cudaStream_t s);
 // dst[k] (cols x rows) = transpose of src[k] (rows x cols), both row-major,
 // for up to 6 arrays in one launch; pairs with a null pointer are skipped
 // (layout.cu): interleaved n x m <-> contiguous m x n batches
 cudaError_t launch_transpose(const double* const* src, double* const* dst, int narr, int64_t rows, int64_t cols,
                              cudaStream_t s);
-size_t pcr_pass_smem_bytes(int TRmax);
 int pcr_max_smem_rows();
 
 

@@ -60,7 +60,11 @@ def _batch(m, n, seed=1):
 
 
 def f64_candidates():
-    for smem, fuse, threads in itertools.product((480, 512, 640, 960, 1920), (1, 2, 3, 4, 5), (128, 256)):
+    # Tiles of at most 512 rows (four CTAs per SM): the size up to which a
+    # system needs no scratch, which callers of the allocation-free entry rely
+    # on, stays where it is.  (1024-row tiles, two CTAs per SM: 5 % faster at
+    # n = 1024, 2 % at 8192, 6 % slower above.)
+    for smem, fuse, threads in itertools.product((384, 448, 480, 512), (1, 2, 3, 4, 5), (128, 256)):
         H = 2 * ((1 << fuse) - 1)
         if smem - 2 * H < 64:
             continue
@@ -69,7 +73,7 @@ def f64_candidates():
 
 def rg_candidates():
     # the persistent kernel runs 256 threads and up to 512 rows per tile
-    for smem, fuse in itertools.product((384, 448, 480, 512), (1, 2, 3)):
+    for smem, fuse in itertools.product((384, 448, 480, 512), (1, 2, 3, 4, 5)):
         H = 2 * ((1 << fuse) - 1)
         yield dict(smem_rows=smem, fuse_strides=fuse, tile_rows=smem - 2 * H, threads=256)
 
