@@ -105,7 +105,7 @@ typedef struct pcrp_mixed_info {
  * pcrp_solve_f64_small and pcrp_solve_f64_split keep the reference's own
  * n = 1024 split.
  * `a` and `e` may be NULL: that band is +0.0 and is not read; with both NULL
- * (a tridiagonal batch) every stride runs the kernels' zero-operand form, with
+ * (a tridiagonal batch) the rows run the kernels' zero-operand form, with
  * the bits of explicit +0.0 bands.  The same holds for the two paths below,
  * pcrp_solve_f64_noalloc and pcrp_solve_host.
  * Replaces: main.cu:46-87 (time_* dispatch around pcr_penta and the splitting
@@ -278,8 +278,8 @@ pcrp_status pcrp_measure_fp64(double* dfma_per_s, double* ddiv_per_s, pcrp_strea
  * design of the mixed-precision kernels; no counterpart in the reference. */
 pcrp_status pcrp_measure_pipes(float* ms, pcrp_stream stream);
 
-/* Checks the FP64 kernels' phase-B quotient (Markstein's correction from the
- * correctly rounded reciprocal, inside its exponent guard) against IEEE
+/* Checks the FP64 kernels' quotient (formed on the integer pipe where its
+ * exponent guard admits the operands) against IEEE
  * division (__ddiv_rn) on `samples` seeded random operand pairs of class
  * `mode` (0: exponents within 2^+-32, 1: the guard's whole range, 2: mantissas
  * near all ones, 3: near powers of two, 4: any exponent, zeros, subnormals,

@@ -186,6 +186,7 @@ pcrp_status f64_solve(const double* a, const double* b, const double* c, const d
     p.src[A_] = a; p.src[B_] = b; p.src[C_] = c; p.src[D_] = d; p.src[E_] = e; p.src[Y_] = y;
     p.src_ss = ss; p.src_rs = rs;
     p.n = n; p.m = m; p.G = 1;
+    p.tri = !a && !e;
 
     double* bufs[2][NSTATE] = {};
     if (s1 > 0) {

@@ -1,14 +1,13 @@
 // ieee_int.cuh -- IEEE double products and quotients on the integer pipe.
 //
-// GB300 issues FP64 at 1/64 of the FP32 rate (one warp instruction per 64
-// cycles and SM sub-partition) while its 32-bit integer pipe, wide multiplies
-// included, runs beside FP64 work.  A correctly rounded product is 4 wide
-// multiplies and ~24 integer instructions, a quotient ~45 (25 more for its
-// divisor's reciprocal).  Measured (24 warps per SM, independent chains, in
-// units of one FP64 product, which is the FP64 pipe's slot): integer product
-// 0.80 alone, a pair of one FP64 and one integer product 1.08; __ddiv_rn
-// 11.8; integer quotient with its reciprocal 1.49 alone, 1.47 together with
-// an FP64 product.
+// GB300 issues one FP64 warp instruction per ~62 cycles and SM sub-partition,
+// while its integer pipe and wide multipliers run beside FP64 work.  A
+// correctly rounded product is 25 instructions (4 wide multiplies), a quotient
+// 40 from its divisor's reciprocal, which takes another 20.  Measured (24
+// warps per SM, 8 independent chains per thread, in units of one FP64
+// product): integer product 0.55 alone; one FP64 and one integer product
+// together 1.00; __ddiv_rn 7.3; integer quotient with its reciprocal 1.08
+// alone, 1.13 together with an FP64 product.
 //
 // Every function returns the round-to-nearest-even result IEEE 754 prescribes
 // for operands inside its guard (normal operands whose result is normal or

@@ -18,44 +18,30 @@
 //
 // Arithmetic.  Each stride forms the reference's Reductions I, II, III
 // (kernel.cu:68-140) with every product, sum and IEEE quotient rounded on its
-// own (__dmul_rn/__dadd_rn/__ddiv_rn: no FMA contraction), in the
-// reference's order of evaluation.  The two neighbour combinations a row
-// needs, R1(i) (rows i-2d, i-d, i) and R2(i) (rows i, i+d, i+2d), are the
-// same combination T(m) centred on m = i-d and m = i+d, built from identical
-// expressions (compare kernel.cu:77-79 with kernel.cu:103-105), so T(m) is
-// formed once per row in phase A and shared through shared memory in
-// phase B: 4 IEEE quotients per row and stride instead of the reference's 6,
-// with bit-identical results.  The two of phase B divide by cT of the
-// neighbours; phase A also stores cT's correctly rounded reciprocal
-// (__drcp_rn), and phase B finishes each quotient with Markstein's
-// correction (IBM J. Res. Dev. 34(1), 1990): q0 = RN(b r), the remainder
-// b - cT q0 exact in one FMA, RN(q0 + rem r) = RN(b / cT) when no
-// intermediate leaves the normal range, which an exponent guard ensures (other
-// operands take the division).  A reciprocal and two corrections cost ~10.5
-// DFMA slots against ~14.4 for two divisions; pcrp_check_quotients compares
-// them with IEEE division on random operand classes.  The reference's multiplier registers, which
-// outlive a stride and are reused when a Reduction-III pivot is exactly zero
-// (kernel.cu:122,129), are kept per row in registers inside a pass and in
-// two extra state arrays between passes.
+// own (no FMA contraction), in the reference's order of evaluation.  The two
+// neighbour combinations a row needs, R1(i) (rows i-2d, i-d, i) and R2(i)
+// (rows i, i+d, i+2d), are the same combination T(m) centred on m = i-d and
+// m = i+d, built from identical expressions (compare kernel.cu:77-79 with
+// kernel.cu:103-105), so T(m) is formed once per row in phase A and shared
+// through shared memory in phase B: 4 quotients per row and stride instead of
+// the reference's 6, with bit-identical results.
 //
-// GB300 note: FP64 issues at ~0.5 lanes/clk per SM sub-partition on this
-// part, so this kernel is bounded by the FP64 pipe, not HBM; the design goal
-// is to keep that pipe busy (several CTAs per SM, 4 rows per thread for ILP)
-// and to spend no FP64 operation beyond the reference's own arithmetic.
+// What bounds it.  One FP64 warp instruction takes 62 cycles of an SM
+// sub-partition on this part, and the stride's 36 products and sums and 4
+// quotients (an FP64 division: 8.6 such slots) used to keep that pipe 87 %
+// busy.  The integer pipe runs beside it, so the quotients and 16 of the 20
+// products are formed there (ieee_int.cuh: correctly rounded, the same bits;
+// one product 25 instructions, one quotient 40) and 16 sums and 4 products stay
+// FP64.  A dense stride now issues ~1,150 warp instructions per 32 rows with
+// the FP64 and the integer pipe both ~60 % busy (4 CTAs of 256 threads per SM;
+// what is left is the latency of the row's dependent chains between two
+// barriers).  Measured, before and after: m=64 n=2^20 weakly dominant 91.7 ->
+// 36.7 ms, m=256 n=65536 19.8 -> 8.5 ms, m=1024 n=512 0.535 -> 0.30 ms; a dense
+// two-stride pass at m=4 n=2^20 1.00 -> 0.42 ms.
 //
-// Zero operands.  Operations whose result IEEE 754 fixes without rounding
-// (a product with a zero factor: the zero of the factors' sign xor; a sum
-// with a zero term: the other term, or -0 only if both are -0; a zero
-// numerator over a finite nonzero divisor) are formed on the integer pipe,
-// an FP64 operation costing ~40 integer operations of pipe time here and a
-// division with a zero numerator ~2.6 normal ones.  They matter once the
-// outer coefficients a, e of a diagonally dominant system have underflowed
-// to zero (from stride ~2^8-2^10 on): in passes whose longest stride is at
-// least 1024 rows a vote per stride tells whether every row of the tile is in
-// that state (a = e = 0, the rest finite; passes of shorter strides are
-// compiled without the vote and its cost); then phase
-// A forms no FP64 value and phase B only its quotients and the products and
-// sums whose operands are nonzero.  Same bits as the FP64 operations.
+// The reference's multiplier registers, which outlive a stride and are reused
+// when a pivot is exactly zero (kernel.cu:122,129), are formed again when that
+// happens (pcr_tile), not kept.
 #include "pcr_tile.cuh"
 
 namespace pcrp {
@@ -63,7 +49,7 @@ namespace {
 
 // CTAs per SM the register budget is set for: as many as shared memory holds
 // (100 bytes per row), at most 1024 threads.
-template <int CAP>
+template <int CAP, bool kFew>
 __global__ void __launch_bounds__(kMaxThreads, CAP > 1024 ? 1 : CAP > 544 ? 2 : 4)
 pcr_pass_kernel(const PcrPassArgs p)
 {
@@ -73,19 +59,43 @@ pcr_pass_kernel(const PcrPassArgs p)
     const int64_t w    = blk - item * p.nwin;
     const int64_t j    = item / p.G;
     const int64_t r    = item - j * p.G;
-    pcr_tile<CAP>(p, j, r, w, *reinterpret_cast<TileRows<CAP>*>(pcr_smem));
+    pcr_tile<CAP, false, kFew>(p, j, r, w, *reinterpret_cast<TileRows<CAP>*>(pcr_smem));
+}
+
+constexpr int kShortRows = 320;
+
+template <int CAP, bool kFew>
+cudaError_t launch_tiles(const PcrPassArgs& p, int threads, int64_t blocks, cudaStream_t s)
+{
+    // per-device attribute; cheap, and legal while a stream is being captured
+    cudaError_t e = cudaFuncSetAttribute(pcr_pass_kernel<CAP, kFew>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(TileRows<CAP>));
+    if (e != cudaSuccess) return e;
+    pcr_pass_kernel<CAP, kFew><<<(unsigned)blocks, threads, sizeof(TileRows<CAP>), s>>>(p);
+    count_launch();
+    return cudaGetLastError();
 }
 
 template <int CAP>
 cudaError_t launch_cap(const PcrPassArgs& p, int threads, int64_t blocks, cudaStream_t s)
 {
-    // per-device attribute; cheap, and legal while a stream is being captured
-    cudaError_t e = cudaFuncSetAttribute(pcr_pass_kernel<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sizeof(TileRows<CAP>));
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    pcr_pass_kernel<CAP><<<(unsigned)blocks, threads, sizeof(TileRows<CAP>), s>>>(p);
-    count_launch();
-    return cudaGetLastError();
+    // The general rows for launches of at most two warps per SM sub-partition,
+    // where a row's latency counts and the FP64 pipe is not full (us, general /
+    // per-case rows: 8 systems of 100 rows 29 / 43, of 512 rows 71 / 81; 32
+    // systems of 4096 rows, six warps, 152 / 136), and for whole short
+    // pentadiagonal systems, most of whose rows are near an end in the late
+    // strides and would each load another case's code (4000 systems of 100
+    // rows 229 / 316, 2000 of 320 rows 388 / 397, of 384 rows 458 / 438).
+    // Tridiagonal batches never (their rows issue little FP64 work: 8 systems
+    // of 512 rows 71 / 50).
+    const bool few = blocks * (threads / 32) <= 8 * (int64_t)sms;
+    const bool shorts = p.G == 1 && p.final_step && p.TRmax <= kShortRows;
+    if ((few || shorts) && !p.tri) return launch_tiles<CAP, true>(p, threads, blocks, s);
+    return launch_tiles<CAP, false>(p, threads, blocks, s);
 }
 
 }  // namespace

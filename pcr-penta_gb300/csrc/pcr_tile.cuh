@@ -333,13 +333,17 @@ __device__ __forceinline__ bool row_b_none(TileRows<CAP>& t, int k, int dl, bool
 template <int CAP>
 __device__ __forceinline__ double row_a_general(TileRows<CAP>& t, int k, int dl, bool hasL, bool has2L, bool hasR, bool has2R)
 {
-    const int l = k - dl, r = k + dl;
-    double al1 = 0.0, al2 = 0.0;
-    if (has2L && nz(t.b[l])) al1 = quot(neg(t.a[k]), t.b[l]);
-    if (has2R && nz(t.d[r])) al2 = quot(neg(t.e[k]), t.d[r]);
+    const int lc = hasL ? k - dl : k, rc = hasR ? k + dl : k;
+    // both integer quotients first, whatever the operands: one dependent
+    // chain beside the other
+    const double am = neg(t.a[k]), em = neg(t.e[k]), bL = t.b[lc], dR = t.d[rc];
+    double al1 = ieee::div(am, bL, ieee::recip(bL)), al2 = ieee::div(em, dR, ieee::recip(dR));
+    if (!has2L) al1 = 0.0;
+    else if (!ieee::div_guard(am, bL)) al1 = nz(bL) ? dvd(am, bL) : 0.0;
+    if (!has2R) al2 = 0.0;
+    else if (!ieee::div_guard(em, dR)) al2 = nz(dR) ? dvd(em, dR) : 0.0;
     // (a missing side adds -0, which changes nothing: kernel.cu:82-91,108-117)
     const double m0 = szero(~0u);
-    const int lc = hasL ? l : k, rc = hasR ? r : k;
     const double cT = add(add(hasL ? mul(al1, t.d[lc]) : m0, t.c[k]), hasR ? mul(al2, t.b[rc]) : m0);
     const double kT = add(add(hasL ? mul(al1, t.y[lc]) : m0, t.y[k]), hasR ? mul(al2, t.y[rc]) : m0);
     const double bT = hasL ? add(add(mul(al1, t.c[lc]), t.b[k]), hasR ? mul(al2, t.a[rc]) : m0) : 0.0;
@@ -354,19 +358,17 @@ __device__ __forceinline__ double row_a_general(TileRows<CAP>& t, int k, int dl,
 template <int CAP>
 __device__ __forceinline__ double2 row_b_general(TileRows<CAP>& t, int k, int dl, bool hasL, bool hasR, double f1, double f2)
 {
-    const int l = k - dl, r = k + dl;
-    double a1 = 0.0, b1 = 0.0, c1 = 0.0, d1 = 0.0, k1 = 0.0;
-    double b2 = 0.0, c2 = 0.0, d2 = 0.0, e2 = 0.0, k2 = 0.0;
-    if (hasL) {                            // kernel.cu:120-125
-        if (nz(t.Tc[l])) f1 = quot(t.b[k], t.Tc[l], t.Tr[l]);
-        a1 = mul(f1, t.Ta[l]); b1 = mul(f1, t.Tb[l]); c1 = mul(f1, t.Td[l]);
-        d1 = mul(f1, t.Te[l]); k1 = mul(f1, t.Ty[l]);
-    }
-    if (hasR) {                            // kernel.cu:127-132
-        if (nz(t.Tc[r])) f2 = quot(t.d[k], t.Tc[r], t.Tr[r]);
-        c2 = mul(f2, t.Tb[r]); b2 = mul(f2, t.Ta[r]); d2 = mul(f2, t.Td[r]);
-        e2 = mul(f2, t.Te[r]); k2 = mul(f2, t.Ty[r]);
-    }
+    const int lc = hasL ? k - dl : k, rc = hasR ? k + dl : k;
+    const double bi = t.b[k], di = t.d[k], cL = t.Tc[lc], cR = t.Tc[rc];
+    const double q1 = ieee::div(bi, cL, t.Tr[lc]), q2 = ieee::div(di, cR, t.Tr[rc]);
+    if (hasL && nz(cL)) f1 = ieee::div_guard(bi, cL) ? q1 : dvd(bi, cL);
+    if (hasR && nz(cR)) f2 = ieee::div_guard(di, cR) ? q2 : dvd(di, cR);
+    const double a1 = hasL ? mul(f1, t.Ta[lc]) : 0.0, b1 = hasL ? mul(f1, t.Tb[lc]) : 0.0;   // kernel.cu:120-125
+    const double c1 = hasL ? mul(f1, t.Td[lc]) : 0.0, d1 = hasL ? mul(f1, t.Te[lc]) : 0.0;
+    const double k1 = hasL ? mul(f1, t.Ty[lc]) : 0.0;
+    const double c2 = hasR ? mul(f2, t.Tb[rc]) : 0.0, b2 = hasR ? mul(f2, t.Ta[rc]) : 0.0;   // kernel.cu:127-132
+    const double d2 = hasR ? mul(f2, t.Td[rc]) : 0.0, e2 = hasR ? mul(f2, t.Te[rc]) : 0.0;
+    const double k2 = hasR ? mul(f2, t.Ty[rc]) : 0.0;
     t.b[k] = add(sub(b1, t.a[k]), b2);     // kernel.cu:138-140
     t.c[k] = add(sub(c1, t.c[k]), c2);
     t.d[k] = add(sub(d1, t.e[k]), d2);
@@ -406,7 +408,9 @@ __device__ __forceinline__ double gload(const double* p) {
 
 // One CTA's work: window w of subsystem r of system j (whole subsystem when
 // p.final_step).  Every thread of the CTA must call it with the same (j, r, w).
-template <int CAP, bool kL2Only = false>
+// kFew: the launch leaves most of the SM's warp slots empty; every row takes
+// the general form.
+template <int CAP, bool kL2Only = false, bool kFew = false>
 __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_t r, int64_t w, TileRows<CAP>& T)
 {
     const int64_t sbase = p.offsets ? p.offsets[j] : j * p.src_ss;
@@ -536,7 +540,8 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_
             // structural zeros, take the general form at once
             double cT;
             bool done = false;
-            if (!left && !right) done = row_a_none(T, k, dl, hasL, has2L, hasR, has2R, cT);
+            if (kFew) done = false;
+            else if (!left && !right) done = row_a_none(T, k, dl, hasL, has2L, hasR, has2R, cT);
             else if (has2L && has2R) {
                 if (left && right) done = row_a_both(T, k, dl, cT);
                 else done = row_a_one(T, k, dl, right, cT);
@@ -573,7 +578,8 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_
             const bool left = hasL && nz(T.b[k]), right = hasR && nz(T.d[k]);
             double f1 = 0.0, f2 = 0.0;
             bool done = false;
-            if (!left && !right) done = row_b_none(T, k, dl, hasL, hasR, f1, f2);
+            if (kFew) done = false;
+            else if (!left && !right) done = row_b_none(T, k, dl, hasL, hasR, f1, f2);
             else if (k - 3 * dl >= kfirst && k + 3 * dl <= klast) {
                 if (left && right) {
                     const bool za = !nz(T.a[k]), ze = !nz(T.e[k]);
