@@ -658,12 +658,12 @@ __device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, 
         if (k >= klo && k < khi) {
             const int64_t i0 = 2 * (t0 + k), q = j * n + i0;
             dmax = fmaxf(dmax, fabsf(v.x));
-            xbits = max(xbits, (unsigned long long)__double_as_longlong(x.x) & 0x7FFFFFFFFFFFFFFFull);
+            xbits = max(xbits, absbits(x.x));
             if (i0 + 1 < n) {
                 if ((q & 1) == 0) *reinterpret_cast<double2*>(p.X0 + q) = x;   // (X0 is 256-byte aligned)
                 else { p.X0[q] = x.x; p.X0[q + 1] = x.y; }
                 dmax = fmaxf(dmax, fabsf(v.y));
-                xbits = max(xbits, (unsigned long long)__double_as_longlong(x.y) & 0x7FFFFFFFFFFFFFFFull);
+                xbits = max(xbits, absbits(x.y));
             } else {
                 p.X0[q] = x.x;
             }
@@ -881,6 +881,7 @@ __device__ __forceinline__ void block_max(unsigned& dmb, unsigned long long& xb,
     __syncthreads();                              // the scratch is reused by the next call
 }
 
+constexpr int kMpNarrow = 256;                   // block rows of a system solved by 128 threads
 constexpr int kMpSmallThreadsMax = 512;          // systems of >= 1024 block rows: 512 threads
 
 template <bool RG>
@@ -1113,45 +1114,130 @@ residual_kernel(const double* __restrict__ a, const double* __restrict__ b, cons
     }
 }
 
-// x (workspace, contiguous) -> y (caller layout)
-__global__ void copy_out_kernel(const double* __restrict__ X, double* __restrict__ y, int64_t m, int64_t n,
-                                int64_t ss, int64_t rs)
+// Report of a solve: one pass over a tile of rows of system j forms
+// r = y - A x (the FMA order of residual_kernel), the per-system maxima of
+// |r_i|, sum_k |A_ik| and |x_i| (float bit patterns), and moves x to y.  Only
+// the tile's own rows of y are written, after they were read.  Rounding to
+// float is monotone, so the maxima are taken on the doubles' bits (no FP64
+// compare or conversion per row; nans do not count, as with fmaxf) and
+// converted once per warp.  Bound by its FP64 work, 5 FMA per row: the row
+// sums, 4 more, are formed in FP64 only for the rows whose single-precision
+// estimate can be the warp's largest.  Replaces a residual, a norm and a copy
+// kernel that read the bands twice and passed r through memory (m=100
+// n=30001: 48 us, 80 % of the FP64 pipe; 91 us with every row sum in FP64 and
+// its loads behind branches; the three kernels ~130 us).
+__device__ __forceinline__ void fold_max(unsigned long long& m, double v)
 {
-    const int64_t total = m * n;
-    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
-         q += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t j = q / n, i = q - j * n;
-        y[j * ss + i * rs] = X[q];
+    const unsigned long long b = absbits(v);
+    if (b <= 0x7FF0000000000000ull) m = max(m, b);
+}
+
+// |v| truncated to float (0 below 2^-126, inf from 2^128 on and for nans)
+__device__ __forceinline__ float abs_estimate(double v)
+{
+    const unsigned h = (unsigned)__double2hiint(v) & 0x7FFFFFFFu;
+    const unsigned f = ((h - (896u << 20)) << 3) | ((unsigned)__double2loint(v) >> 29);
+    return h < (897u << 20) ? 0.0f : __uint_as_float(h >= (1151u << 20) ? 0x7F800000u : f);
+}
+
+constexpr int kReportRows = 4;                    // rows per thread
+
+__global__ void __launch_bounds__(kMpThreads)
+report_kernel(const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
+              const double* __restrict__ d, const double* __restrict__ e, const double* __restrict__ X, double* y,
+              int64_t m, int64_t n, int64_t ss, int64_t rs, unsigned* __restrict__ rn, unsigned* __restrict__ an,
+              unsigned* __restrict__ xn)
+{
+    constexpr int kTile = kReportRows * kMpThreads;
+    const int64_t tiles = (n + kTile - 1) / kTile;
+    for (int64_t blk = blockIdx.x; blk < m * tiles; blk += gridDim.x) {
+        const int64_t j = blk / tiles, i0 = (blk - j * tiles) * kTile + threadIdx.x;
+        const double* __restrict__ x = X + j * n;
+        unsigned long long rm = 0ull, am = 0ull, xm = 0ull;
+        float est[kReportRows];
+        // every load of a row first (slots outside the system are zeros)
+#pragma unroll 2
+        for (int u = 0; u < kReportRows; u++) {
+            const int64_t i = i0 + u * kMpThreads, g = j * ss + i * rs;
+            est[u] = 0.0f;
+            if (i < n) {
+                const bool l2 = i >= 2, l1 = i >= 1, r1 = i + 1 < n, r2 = i + 2 < n;
+                const double wc = c[g], yv = y[g], xv = x[i];
+                const double wa = a && l2 ? a[g] : 0.0, wb = l1 ? b[g] : 0.0;
+                const double wd = r1 ? d[g] : 0.0, we = e && r2 ? e[g] : 0.0;
+                const double xa = a && l2 ? x[i - 2] : 0.0, xb = l1 ? x[i - 1] : 0.0;
+                const double xd = r1 ? x[i + 1] : 0.0, xe = e && r2 ? x[i + 2] : 0.0;
+                double v = fma(-wc, xv, yv);
+                v = fma(-wa, xa, v);
+                v = fma(-wb, xb, v);
+                v = fma(-wd, xd, v);
+                v = fma(-we, xe, v);
+                est[u] = (abs_estimate(wc) + abs_estimate(wa)) + (abs_estimate(wb) + abs_estimate(wd)) +
+                         abs_estimate(we);
+                fold_max(rm, v); fold_max(xm, xv);
+                y[g] = xv;
+            }
+        }
+        // (an estimate is within 2^-20 of its sum unless terms were below
+        // 2^-126 or above 2^128: then every row counts)
+        float top = est[0];
+#pragma unroll
+        for (int u = 1; u < kReportRows; u++) top = fmaxf(top, est[u]);
+        top = warp_max(top);
+        const float least = top > 1e-30f && top < FLT_MAX ? top * (1.0f - 0x1p-19f) : -1.0f;
+#pragma unroll
+        for (int u = 0; u < kReportRows; u++) {
+            const int64_t i = i0 + u * kMpThreads, g = j * ss + i * rs;
+            if (i < n && est[u] >= least) {
+                double rowsum = fabs(c[g]);
+                if (a && i >= 2) rowsum += fabs(a[g]);
+                if (i >= 1) rowsum += fabs(b[g]);
+                if (i + 1 < n) rowsum += fabs(d[g]);
+                if (e && i + 2 < n) rowsum += fabs(e[g]);
+                fold_max(am, rowsum);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            rm = max(rm, __shfl_xor_sync(0xffffffffu, rm, o));
+            am = max(am, __shfl_xor_sync(0xffffffffu, am, o));
+            xm = max(xm, __shfl_xor_sync(0xffffffffu, xm, o));
+        }
+        if ((threadIdx.x & 31) == 0) {
+            atomic_max_pos(&rn[j], (float)__longlong_as_double((long long)rm));
+            atomic_max_pos(&an[j], (float)__longlong_as_double((long long)am));
+            atomic_max_pos(&xn[j], (float)__longlong_as_double((long long)xm));
+        }
     }
 }
 
-// Per system: max |r_i|, max_i sum_k |A_ik| and max |x_i| (float bit patterns).
-// X and r are contiguous; the bands use the caller's layout.
+// The batch's report from the per-system values (one CTA)
 __global__ void __launch_bounds__(kMpThreads)
-resid_norm_kernel(const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
-                  const double* __restrict__ d, const double* __restrict__ e,
-                  const double* __restrict__ X, const double* __restrict__ r, int64_t m, int64_t n,
-                  int64_t ss, int64_t rs, unsigned* __restrict__ rn, unsigned* __restrict__ an,
-                  unsigned* __restrict__ xn)
+summary_kernel(MpArgs p, const unsigned* __restrict__ rn, MpSummary* out)
 {
-    const int64_t tiles = (n + 1023) / 1024;
-    const int64_t j = blockIdx.x / tiles, tile = blockIdx.x - j * tiles;
-    float rm = 0.0f, am = 0.0f, xm = 0.0f;
-    const int64_t iend = min((tile + 1) * 1024, n);
-    for (int64_t i = tile * 1024 + threadIdx.x; i < iend; i += blockDim.x) {
-        const int64_t g = j * ss + i * rs;
-        double rowsum = fabs(c[g]);
-        if (a && i >= 2) rowsum += fabs(a[g]);
-        if (i >= 1) rowsum += fabs(b[g]);
-        if (i + 1 < n) rowsum += fabs(d[g]);
-        if (e && i + 2 < n) rowsum += fabs(e[g]);
-        rm = fmaxf(rm, (float)fabs(r[j * n + i]));
-        am = fmaxf(am, (float)rowsum);
-        xm = fmaxf(xm, (float)fabs(X[j * n + i]));
+    __shared__ MpSummary part[kMpThreads / 32];
+    MpSummary s{0, 1, 0.0f, 0, 0.0};
+    auto fold = [&](int sweeps, int converged, float est, double resid) {
+        s.sweeps = max(s.sweeps, sweeps);
+        s.converged &= converged;
+        s.est = est > s.est ? est : s.est;
+        s.resid = resid > s.resid ? resid : s.resid;
+    };
+    for (int64_t j = threadIdx.x; j < p.m; j += kMpThreads) {
+        const float rj = __uint_as_float(rn[j]), aj = __uint_as_float(rn[p.m + j]), xj = __uint_as_float(rn[2 * p.m + j]);
+        const double den = (double)aj * (double)xj;
+        fold(p.fin[j], p.status[j] == 1, p.est[j], den > 0.0 ? rj / den : (rj > 0.0f ? 1.0 : 0.0));
     }
-    rm = warp_max(rm); am = warp_max(am); xm = warp_max(xm);
-    if ((threadIdx.x & 31) == 0) {
-        atomic_max_pos(&rn[j], rm); atomic_max_pos(&an[j], am); atomic_max_pos(&xn[j], xm);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        fold(__shfl_xor_sync(0xffffffffu, s.sweeps, o), __shfl_xor_sync(0xffffffffu, s.converged, o),
+             __shfl_xor_sync(0xffffffffu, s.est, o), __shfl_xor_sync(0xffffffffu, s.resid, o));
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < kMpThreads / 32; k++) fold(part[k].sweeps, part[k].converged, part[k].est, part[k].resid);
+        s.gave_up = p.err ? *p.err : 0;
+        *out = s;
     }
 }
 
@@ -1248,11 +1334,14 @@ cudaError_t launch_mp_small(const MpArgs& p, cudaStream_t s)
                                          (int)mp_pass_smem(kMpMaxRows));
     if (e != cudaSuccess) return e;
     // large tiles hold two CTAs per SM (shared memory): twice the threads per
-    // CTA keep as many warps resident as four CTAs of small tiles; systems of
-    // fewer than 256 block rows get one thread per block row (whole warps),
-    // so small systems fill the SM with more CTAs instead of idle threads
-    const int threads = nb >= 1024 ? kMpSmallThreadsMax
-                        : nb >= kMpThreads ? kMpThreads : (int)std::max<int64_t>(32, (nb + 31) / 32 * 32);
+    // CTA keep as many warps resident as four CTAs of small tiles; tiles of at
+    // most kMpNarrow block rows get 128 threads, so that more systems run at
+    // once while each waits for its barriers (m=1024 n=512, interleaved: 8
+    // instead of 4 CTAs per SM, one wave instead of two, 45.2 -> 38.3 us; at
+    // n=2000 256 threads 154 us, 128 210); systems of fewer than 128 block
+    // rows one thread per block row (whole warps)
+    const int threads = nb >= 1024 ? kMpSmallThreadsMax : nb > kMpNarrow ? kMpThreads
+                        : (int)std::min<int64_t>(128, std::max<int64_t>(32, (nb + 31) / 32 * 32));
     const int64_t blocks = std::min<int64_t>(p.m, mp_grid_cap((const void*)kern, threads, smem));
     e = launch_dependent(kern, (unsigned)blocks, threads, smem, s, p);
     count_launch();
@@ -1305,21 +1394,14 @@ cudaError_t launch_residual(const double* a, const double* b, const double* c, c
     return cudaGetLastError();
 }
 
-cudaError_t launch_copy_out(const double* X, double* y, int64_t m, int64_t n, int64_t ss, int64_t rs, cudaStream_t s)
+cudaError_t launch_report(const MpArgs& p, const double* X, unsigned* norms, MpSummary* out, cudaStream_t s)
 {
-    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((m * n + kMpThreads - 1) / kMpThreads, 152 * 16));
-    copy_out_kernel<<<(unsigned)blocks, kMpThreads, 0, s>>>(X, y, m, n, ss, rs);
+    const int64_t tiles = (p.n + kReportRows * kMpThreads - 1) / (kReportRows * kMpThreads);
+    const int64_t blocks = std::min<int64_t>(p.m * tiles, mp_grid_cap((const void*)report_kernel, kMpThreads, 0));
+    report_kernel<<<(unsigned)blocks, kMpThreads, 0, s>>>(p.a, p.b, p.c, p.d, p.e, X, p.y, p.m, p.n, p.ss, p.rs, norms,
+                                                          norms + p.m, norms + 2 * p.m);
     count_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_resid_norm(const double* a, const double* b, const double* c, const double* d, const double* e,
-                              const double* X, const double* r, int64_t m, int64_t n, int64_t ss,
-                              int64_t rs, unsigned* rn, unsigned* an, unsigned* xn, cudaStream_t s)
-{
-    const int64_t blocks = m * ((n + 1023) / 1024);
-    if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    resid_norm_kernel<<<(unsigned)blocks, kMpThreads, 0, s>>>(a, b, c, d, e, X, r, m, n, ss, rs, rn, an, xn);
+    summary_kernel<<<1, kMpThreads, 0, s>>>(p, norms, out);
     count_launch();
     return cudaGetLastError();
 }

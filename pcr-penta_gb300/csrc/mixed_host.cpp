@@ -51,7 +51,7 @@ MpPlan mp_plan(int64_t nb, const pcrp_opts* o)
 
 struct MpLayout {
     size_t S0, R, Mi, P0, P1, dx, X0, Yc, Xout, ctr, ndx, nx, fin, status, est, trunc, ndx_pre, live, fail, nfail, dnorm,
-        err, rbuf, rn, total;
+        err, sum, rn, total;
 };
 
 MpLayout mp_layout(int64_t m, int64_t n, int max_sweeps, const MpPlan& pl, bool info)
@@ -82,7 +82,7 @@ MpLayout mp_layout(int64_t m, int64_t n, int max_sweeps, const MpPlan& pl, bool 
     L.nfail = take(sizeof(int));
     L.dnorm = take(2 * (size_t)m * sizeof(unsigned));
     L.err = take(sizeof(int));
-    L.rbuf = info ? take((size_t)m * n * sizeof(double)) : 0;
+    L.sum = info ? take(sizeof(MpSummary)) : 0;
     L.rn = info ? take(3 * m * sizeof(unsigned)) : 0;
     L.total = off;
     return L;
@@ -461,7 +461,10 @@ pcrp_status mixed_enqueue(const double* a, const double* b, const double* c, con
     A.ctr = reinterpret_cast<int*>(base + WL.ctr);
 
     cudaError_t ce;
-    const int gm = keep_x ? 0 : graph_mode(st);
+    // (a report synchronises: not inside a caller's capture)
+    int gm = graph_mode(st);
+    const bool waiting_forbidden = gm == 2;
+    if (keep_x && gm == 2) gm = 0;
     if (gm == 1) {
         const pcrp_status grc = launch_sweep_graph(A, S, st);
         if (grc != PCRP_ENOTSUP) {
@@ -488,6 +491,15 @@ pcrp_status mixed_enqueue(const double* a, const double* b, const double* c, con
     for (int s = 0; s < max_sweeps; s++) {
         const pcrp_status rc = enqueue_sweep(A, S, s, st);
         if (rc != PCRP_OK) return rc;
+        // a report waits for the solve in any case: stop once no system runs
+        // instead of enqueueing sweeps that return at once
+        if (keep_x && s >= 1 && s + 1 < max_sweeps && !waiting_forbidden) {
+            int running = 0;
+            ce = cudaMemcpyAsync(&running, A.live + s + 1, sizeof running, cudaMemcpyDeviceToHost, st);
+            if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+            if (ce != cudaSuccess) return cuda_error(ce, "mixed sweep count");
+            if (running == 0) break;
+        }
     }
     if (out) *out = A;
     return PCRP_OK;
@@ -561,52 +573,25 @@ extern "C" pcrp_status pcrp_solve_mixed(const double* a, const double* b, const 
 
     if (!info) return adapt_out();
 
-    // report: y still holds the rhs (the iterate was kept in X); final
-    // residual r = y - A X, its norms, then X -> y
-    double* rb = reinterpret_cast<double*>(base + WL.rbuf);
+    // report: y still holds the rhs (the iterate was kept in Xout)
     unsigned* rn = U(WL.rn);
+    MpSummary* ds = reinterpret_cast<MpSummary*>(base + WL.sum);
     ce = cudaMemsetAsync(rn, 0, 3 * m * sizeof(unsigned), st);
-    if (ce != cudaSuccess) return cuda_error(ce, "cudaMemsetAsync");
-    ce = launch_residual(a, b, c, d, e, ys, A.Xout, rb, m, n, A.ss, A.rs, n, 1, st);
-    if (ce == cudaSuccess) ce = launch_resid_norm(a, b, c, d, e, A.Xout, rb, m, n, A.ss, A.rs, rn, rn + m, rn + 2 * m, st);
-    if (ce == cudaSuccess) ce = launch_copy_out(A.Xout, ys, m, n, A.ss, A.rs, st);
+    if (ce == cudaSuccess) ce = launch_report(A, A.Xout, rn, ds, st);
     if (ce != cudaSuccess) return cuda_error(ce, "mixed report launch");
     rc = adapt_out();
     if (rc != PCRP_OK) return rc;
-    std::vector<unsigned> norms(3 * m);
-    ce = cudaMemcpyAsync(norms.data(), rn, 3 * m * sizeof(unsigned), cudaMemcpyDeviceToHost, st);
-    if (ce != cudaSuccess) return cuda_error(ce, "mixed report copy");
-    std::vector<int> conv(m), sw(m);
-    std::vector<float> est(m);
-    ce = cudaMemcpyAsync(conv.data(), A.status, m * sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(sw.data(), A.fin, m * sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (ce == cudaSuccess) ce = cudaMemcpyAsync(est.data(), A.est, m * sizeof(float), cudaMemcpyDeviceToHost, st);
-    int waits_gave_up = 0;
-    if (ce == cudaSuccess && A.err)
-        ce = cudaMemcpyAsync(&waits_gave_up, A.err, sizeof(int), cudaMemcpyDeviceToHost, st);
+    MpSummary sum{};
+    ce = cudaMemcpyAsync(&sum, ds, sizeof sum, cudaMemcpyDeviceToHost, st);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
     if (ce != cudaSuccess) return cuda_error(ce, "mixed report");
-    if (waits_gave_up)
+    if (sum.gave_up)
         return set_error(PCRP_ETIMEOUT, "%s: a staging wait of the fused first sweeps gave up (time limit)", who);
-    int all = 1, maxsw = 0;
-    float maxest = 0.0f;
-    for (int64_t j = 0; j < m; j++) {
-        all &= conv[j] == 1;
-        maxsw = std::max(maxsw, sw[j]);
-        maxest = std::max(maxest, est[j]);
-    }
-    info->sweeps = maxsw;
-    info->converged = all;
-    info->fwd_err_est = maxest;
-    double worst = 0.0;
-    for (int64_t j = 0; j < m; j++) {
-        float rj, aj, xj;
-        std::memcpy(&rj, &norms[j], 4); std::memcpy(&aj, &norms[m + j], 4); std::memcpy(&xj, &norms[2 * m + j], 4);
-        const double den = (double)aj * (double)xj;
-        const double v = den > 0.0 ? rj / den : (rj > 0.0f ? 1.0 : 0.0);
-        worst = std::max(worst, v);
-    }
-    info->resid = worst;
+    info->sweeps = sum.sweeps;
+    info->converged = sum.converged;
+    info->fwd_err_est = sum.est;
+    info->resid = sum.resid;
+    const int all = sum.converged;
     if (!all) return set_error(PCRP_ENOCONV, "%s: not every system reached tol=%g in %d sweeps", who, tol, max_sweeps);
     return PCRP_OK;
 }

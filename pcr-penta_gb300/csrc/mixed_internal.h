@@ -181,9 +181,14 @@ cudaError_t launch_mp_gate(const MpArgs& p, cudaGraphConditionalHandle h, cudaSt
 cudaError_t launch_residual(const double* a, const double* b, const double* c, const double* d, const double* e,
                             const double* y, const double* x, double* r, int64_t m, int64_t n, int64_t ss,
                             int64_t rs, int64_t xss, int64_t xrs, cudaStream_t s);
-cudaError_t launch_copy_out(const double* X, double* y, int64_t m, int64_t n, int64_t ss, int64_t rs, cudaStream_t s);
-cudaError_t launch_resid_norm(const double* a, const double* b, const double* c, const double* d, const double* e,
-                              const double* X, const double* r, int64_t m, int64_t n, int64_t ss,
-                              int64_t rs, unsigned* rn, unsigned* an, unsigned* xn, cudaStream_t s);
+// Report of a solve whose iterate X (contiguous) was kept apart: residual
+// norms against the rhs in p.y, X -> p.y, and the batch's summary.
+struct MpSummary {
+    int sweeps, converged;
+    float est;
+    int gave_up;                        // a bounded wait of the fused kernel gave up
+    double resid;
+};
+cudaError_t launch_report(const MpArgs& p, const double* X, unsigned* norms, MpSummary* out, cudaStream_t s);
 
 }  // namespace pcrp
