@@ -234,31 +234,49 @@ __device__ __forceinline__ PairRow load_pair(const MpArgs& p, int64_t j, int64_t
 // The FP32 row-scaled diagonal block and couplings of block row k (rows
 // i0 = 2k, i1 = 2k+1) of a system with n rows.  Row i1 = n (odd n) is a
 // dummy identity row.  Out-of-range band slots are never read as values.
-struct BlockRow { M2 D, L, U; int sh0, sh1; };
+struct BlockRow { M2 D, L, U; float y0, y1; };
 
 __device__ __forceinline__ BlockRow block_of(const PairRow& P, int64_t i0, int64_t n)
 {
     BlockRow B;
     const int64_t i1 = i0 + 1;
-    B.sh0 = d_exponent(P.c0);
-    const float a0 = i0 >= 2 ? d2f_scaled(P.a0, B.sh0) : 0.0f;
-    const float b0 = i0 >= 1 ? d2f_scaled(P.b0, B.sh0) : 0.0f;
-    const float d0 = i0 + 1 < n ? d2f_scaled(P.d0, B.sh0) : 0.0f;
-    const float e0 = i0 + 2 < n ? d2f_scaled(P.e0, B.sh0) : 0.0f;
-    const float cf0 = d2f_scaled(P.c0, B.sh0);
+    const int sh0 = d_exponent(P.c0);
+    const float a0 = i0 >= 2 ? d2f_scaled(P.a0, sh0) : 0.0f;
+    const float b0 = i0 >= 1 ? d2f_scaled(P.b0, sh0) : 0.0f;
+    const float d0 = i0 + 1 < n ? d2f_scaled(P.d0, sh0) : 0.0f;
+    const float e0 = i0 + 2 < n ? d2f_scaled(P.e0, sh0) : 0.0f;
+    const float cf0 = d2f_scaled(P.c0, sh0);
     float a1 = 0.0f, b1 = 0.0f, cf1 = 1.0f, d1 = 0.0f, e1 = 0.0f;
-    B.sh1 = 0;
+    B.y0 = d2f_scaled(P.y0, sh0);
+    B.y1 = 0.0f;
     if (i1 < n) {
-        B.sh1 = d_exponent(P.c1);
-        a1 = i1 >= 2 ? d2f_scaled(P.a1, B.sh1) : 0.0f;
-        b1 = d2f_scaled(P.b1, B.sh1);
-        cf1 = d2f_scaled(P.c1, B.sh1);
-        d1 = i1 + 1 < n ? d2f_scaled(P.d1, B.sh1) : 0.0f;
-        e1 = i1 + 2 < n ? d2f_scaled(P.e1, B.sh1) : 0.0f;
+        const int sh1 = d_exponent(P.c1);
+        a1 = i1 >= 2 ? d2f_scaled(P.a1, sh1) : 0.0f;
+        b1 = d2f_scaled(P.b1, sh1);
+        cf1 = d2f_scaled(P.c1, sh1);
+        d1 = i1 + 1 < n ? d2f_scaled(P.d1, sh1) : 0.0f;
+        e1 = i1 + 2 < n ? d2f_scaled(P.e1, sh1) : 0.0f;
+        B.y1 = d2f_scaled(P.y1, sh1);
     }
     B.D = {cf0, d0, b1, cf1};
     B.L = {a0, b0, 0.0f, a1};
     B.U = {e0, 0.0f, d1, e1};
+    return B;
+}
+
+// The same for a block row with all its band slots inside the system; values
+// beyond the row conversion's range take the general form.
+__device__ __forceinline__ BlockRow block_inner(const PairRow& P, int64_t i0, int64_t n)
+{
+    const RowScale s0 = row_scale(P.c0), s1 = row_scale(P.c1);
+    int top = 0;
+    BlockRow B;
+    B.D = {d2f_row(P.c0, s0, top), d2f_row(P.d0, s0, top), d2f_row(P.b1, s1, top), d2f_row(P.c1, s1, top)};
+    B.L = {d2f_row(P.a0, s0, top), d2f_row(P.b0, s0, top), 0.0f, d2f_row(P.a1, s1, top)};
+    B.U = {d2f_row(P.e0, s0, top), 0.0f, d2f_row(P.d1, s1, top), d2f_row(P.e1, s1, top)};
+    B.y0 = d2f_row(P.y0, s0, top);
+    B.y1 = d2f_row(P.y1, s1, top);
+    if (!(s0.ok && s1.ok && row_fits(top))) B = block_of(P, i0, n);
     return B;
 }
 
@@ -269,19 +287,23 @@ __device__ __forceinline__ BlockRow block_of(const PairRow& P, int64_t i0, int64
 // the normalised couplings and rhs.
 struct PrepRow { M2 L, U, Mi; float2 Y; double2 y; };   // y: the two FP64 rhs values (0 past the system)
 
-template <bool RG>
-__device__ __forceinline__ PrepRow prep_row(const MpArgs& p, int64_t j, int64_t k, Keep keep = Keep::normal)
+__device__ __forceinline__ PrepRow prep_of(const BlockRow& B)
 {
-    const PairRow P = load_pair<RG>(p, j, 2 * k, keep);
-    const BlockRow B = block_of(P, 2 * k, p.n);
     PrepRow r;
     r.Mi = minv(B.D);
     r.L = mmul(r.Mi, B.L);
     r.U = mmul(r.Mi, B.U);
-    const float y0 = d2f_scaled(P.y0, B.sh0);
-    const float y1 = 2 * k + 1 < p.n ? d2f_scaled(P.y1, B.sh1) : 0.0f;
-    r.Y = make_float2(fmaf(r.Mi.m0, y0, r.Mi.m1 * y1), fmaf(r.Mi.m2, y0, r.Mi.m3 * y1));
-    r.y = make_double2(P.y0, 2 * k + 1 < p.n ? P.y1 : 0.0);
+    r.Y = make_float2(fmaf(r.Mi.m0, B.y0, r.Mi.m1 * B.y1), fmaf(r.Mi.m2, B.y0, r.Mi.m3 * B.y1));
+    return r;
+}
+
+template <bool RG>
+__device__ __forceinline__ PrepRow prep_row(const MpArgs& p, int64_t j, int64_t k, Keep keep = Keep::normal)
+{
+    const PairRow P = load_pair<RG>(p, j, 2 * k, keep);
+    const int64_t i0 = 2 * k;
+    PrepRow r = prep_of(i0 >= 2 && i0 + 3 < p.n ? block_inner(P, i0, p.n) : block_of(P, i0, p.n));
+    r.y = make_double2(P.y0, i0 + 1 < p.n ? P.y1 : 0.0);
     return r;
 }
 
