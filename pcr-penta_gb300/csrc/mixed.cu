@@ -66,64 +66,62 @@ __device__ __forceinline__ void x_write(double* __restrict__ x, int64_t ss, int6
     if (i < g.y) x[g.x + i] = v;
 }
 
+// Where sweep s reads x_{s-1} and writes x_s.  x_0 is a float (the first
+// correction itself), kept as one in X0f (m*n, contiguous) when more sweeps
+// follow: srcf (sweep 1) and dstf (sweep 0) then stand in for src and dst.
+struct XView {
+    const double* src; int64_t sss, srs; const longlong2* srg;
+    double* dst; int64_t dss, drs; const longlong2* drg;
+    const float* srcf; float* dstf;
+};
+
 // x_s of row i of system j (FP32 correction d), with the maxima of |dx| and
 // |x| folded into dmax and xbits.
-__device__ __forceinline__ double x_update(const double* __restrict__ xsrc, int64_t xss, int64_t xrs,
-                                           const longlong2* srg, double* __restrict__ xdst, int64_t dss, int64_t drs,
-                                           const longlong2* drg, int64_t j, int64_t i, float d, float& dmax,
-                                           unsigned long long& xbits)
+__device__ __forceinline__ void x_update(const XView& v, int64_t n, int64_t j, int64_t i, float d, float& dmax,
+                                         unsigned long long& xbits)
 {
     const double dd = f2d(d);
-    const double x = xsrc ? __dadd_rn(x_read(xsrc, xss, xrs, srg, j, i), dd) : dd;
-    x_write(xdst, dss, drs, drg, j, i, x);
+    double x = dd;
+    if (v.srcf) x = __dadd_rn(f2d(v.srcf[j * n + i]), dd);
+    else if (v.src) x = __dadd_rn(x_read(v.src, v.sss, v.srs, v.srg, j, i), dd);
+    if (v.dstf) v.dstf[j * n + i] = d;
+    else x_write(v.dst, v.dss, v.drs, v.drg, j, i, x);
     dmax = fmaxf(dmax, fabsf(d));
     xbits = max(xbits, absbits(x));
-    return x;
 }
 
 // Rows i0 (even) and i0 + 1 < n of system j: as two x_update calls, with
-// one 16-byte load and store when both iterates are contiguous there and
-// 16-byte aligned (same values).
-__device__ __forceinline__ void x_update_pair(const double* __restrict__ xsrc, int64_t xss, int64_t xrs,
-                                              const longlong2* srg, double* __restrict__ xdst, int64_t dss,
-                                              int64_t drs, const longlong2* drg, int64_t j, int64_t i0, float2 d,
-                                              float& dmax, unsigned long long& xbits)
+// paired loads and stores for sweep 1 of a contiguous batch where they are
+// aligned (same values).
+__device__ __forceinline__ void x_update_pair(const XView& v, int64_t n, int64_t j, int64_t i0, float2 d, float& dmax,
+                                              unsigned long long& xbits)
 {
-    if (!srg && !drg && xrs == 1 && drs == 1) {
-        const double* s = xsrc ? xsrc + j * xss + i0 : nullptr;
-        double* t = xdst + j * dss + i0;
-        if (((reinterpret_cast<uintptr_t>(s) | reinterpret_cast<uintptr_t>(t)) & 15) == 0) {
-            const double2 dd = make_double2(f2d(d.x), f2d(d.y));
-            double2 x = dd;
-            if (s) {
-                const double2 xs = *reinterpret_cast<const double2*>(s);
-                x = make_double2(__dadd_rn(xs.x, dd.x), __dadd_rn(xs.y, dd.y));
-            }
+    if (v.srcf && !v.dstf && !v.drg && v.drs == 1) {
+        const float* s = v.srcf + j * n + i0;
+        double* t = v.dst + j * v.dss + i0;
+        if (((reinterpret_cast<uintptr_t>(s) & 7) | (reinterpret_cast<uintptr_t>(t) & 15)) == 0) {
+            const float2 xs = *reinterpret_cast<const float2*>(s);
+            const double2 x = make_double2(__dadd_rn(f2d(xs.x), f2d(d.x)), __dadd_rn(f2d(xs.y), f2d(d.y)));
             *reinterpret_cast<double2*>(t) = x;
             dmax = fmaxf(dmax, fmaxf(fabsf(d.x), fabsf(d.y)));
             xbits = max(xbits, max(absbits(x.x), absbits(x.y)));
             return;
         }
     }
-    x_update(xsrc, xss, xrs, srg, xdst, dss, drs, drg, j, i0, d.x, dmax, xbits);
-    x_update(xsrc, xss, xrs, srg, xdst, dss, drs, drg, j, i0 + 1, d.y, dmax, xbits);
+    x_update(v, n, j, i0, d.x, dmax, xbits);
+    x_update(v, n, j, i0 + 1, d.y, dmax, xbits);
 }
 
-// Iterates of sweep s: x_0 in X0 when more sweeps follow, every later x_s in
+// Iterates of sweep s: x_0 in X0f when more sweeps follow, every later x_s in
 // the output; x_{s-1} is read from where sweep s-1 wrote it.
 // The output of a ragged batch is addressed through rg.
-struct XView { const double* src; int64_t sss, srs; const longlong2* srg; double* dst; int64_t dss, drs; const longlong2* drg; };
-
-__device__ __forceinline__ XView x_view(int s, int max_sweeps, const double* X0, double* xout, int64_t n,
-                                        int64_t oss, int64_t ors, const longlong2* rg)
+__device__ __forceinline__ XView x_view(int s, int max_sweeps, float* X0f, double* xout, int64_t oss, int64_t ors,
+                                        const longlong2* rg)
 {
-    XView v;
-    v.srg = nullptr; v.drg = nullptr;
-    if (s == 0) { v.src = nullptr; v.sss = 0; v.srs = 0; }
-    else if (s == 1) { v.src = X0; v.sss = n; v.srs = 1; }
-    else { v.src = xout; v.sss = oss; v.srs = ors; v.srg = rg; }
-    if (s == 0 && max_sweeps >= 2) { v.dst = const_cast<double*>(X0); v.dss = n; v.drs = 1; }
-    else { v.dst = xout; v.dss = oss; v.drs = ors; v.drg = rg; }
+    XView v{nullptr, oss, ors, rg, xout, oss, ors, rg, nullptr, nullptr};
+    if (s == 1) v.srcf = X0f;
+    else if (s > 1) v.src = xout;
+    if (s == 0 && max_sweeps >= 2) v.dstf = X0f;
     return v;
 }
 
@@ -132,11 +130,7 @@ __device__ __forceinline__ XView x_view(int s, int max_sweeps, const double* X0,
 // starts).  No-ops for host-driven launches.
 __device__ __forceinline__ void mp_resolve(MpArgs& p)
 {
-    if (!p.ctr) return;
-    p.sweep = *p.ctr;
-    const XView v = x_view(p.sweep, p.max_sweeps, p.X0, p.xout, p.n, p.oss, p.ors, p.rg);
-    p.xsrc = v.src; p.xsrc_ss = v.sss; p.xsrc_rs = v.srs; p.xsrc_rg = v.srg;
-    p.xdst = v.dst; p.xdst_ss = v.dss; p.xdst_rs = v.drs; p.xdst_rg = v.drg;
+    if (p.ctr) p.sweep = *p.ctr;
 }
 
 __device__ __forceinline__ void mp_resolve(MpPassArgs& p)
@@ -151,12 +145,7 @@ __device__ __forceinline__ void mp_resolve(MpPassArgs& p)
         p.ndx_pre_in = p.pass > 0 ? pre + (size_t)(p.pass - 1) * p.m : nullptr;
         p.ndx_pre_out = p.final_step ? nullptr : pre + (size_t)p.pass * p.m;
     }
-    if (p.nx0) {
-        p.nx = p.nx0 + (size_t)s * p.m;
-        const XView v = x_view(s, p.max_sweeps, p.X0, p.xout, p.n, p.oss, p.ors, p.rg);
-        p.xsrc = v.src; p.xsrc_ss = v.sss; p.xsrc_rs = v.srs; p.xsrc_rg = v.srg;
-        p.xdst = v.dst; p.xdst_ss = v.dss; p.xdst_rs = v.drs; p.xdst_rg = v.drg;
-    }
+    if (p.nx0) p.nx = p.nx0 + (size_t)s * p.m;
 }
 
 // The six FP64 values of rows i0 = 2k and i1 = 2k+1 of system j (i1 may be
@@ -297,6 +286,17 @@ __device__ __forceinline__ PrepRow prep_of(const BlockRow& B)
     return r;
 }
 
+// The inverse of the row-scaled FP32 diagonal block of a block row, as prep_of
+// forms it.
+__device__ __forceinline__ M2 diag_inverse(const PairRow& P, int64_t i0, int64_t n)
+{
+    const RowScale s0 = row_scale(P.c0), s1 = row_scale(P.c1);
+    int top = 0;
+    M2 D = {d2f_row(P.c0, s0, top), d2f_row(P.d0, s0, top), d2f_row(P.b1, s1, top), d2f_row(P.c1, s1, top)};
+    if (!(i0 + 1 < n && s0.ok && s1.ok && row_fits(top))) D = block_of(P, i0, n).D;
+    return minv(D);
+}
+
 template <bool RG>
 __device__ __forceinline__ PrepRow prep_row(const MpArgs& p, int64_t j, int64_t k, Keep keep = Keep::normal)
 {
@@ -325,8 +325,6 @@ __device__ __forceinline__ void prep_store(const MpArgs& p, int64_t q, const Pre
     // (the rhs copy Yc is written by the callers, which have y in hand)
     p.S0[2 * q] = make_float4(r.L.m0, r.L.m1, r.L.m2, r.L.m3);
     p.S0[2 * q + 1] = make_float4(r.U.m0, r.U.m1, r.U.m2, r.U.m3);
-    p.Mi[q] = make_float4(r.Mi.m0, r.Mi.m1, r.Mi.m2, r.Mi.m3);
-    p.R[0][q] = r.Y;
 }
 
 // per-system flags and norms of a solve
@@ -358,9 +356,27 @@ mp_prep_kernel(MpArgs p)
         const int64_t j = q / nb, k = q - j * nb;
         const PrepRow r = prep_row<RG>(p, j, k);
         prep_store(p, q, r);
+        p.R[0][q] = r.Y;
         store_rhs_pair(p, j, 2 * k, r.y);
     }
     pdl_release();                                // (multi-wave grid: release once this CTA is done)
+}
+
+// The first right-hand side of the systems the windowed sweep 0 leaves to the
+// general passes (the windows keep theirs in shared memory; 4 bytes per row
+// that no other system's solve would read).
+template <bool RG>
+__global__ void __launch_bounds__(kMpThreads)
+mp_rhs_kernel(MpArgs p)
+{
+    pdl_wait();
+    pdl_release();                                // one wave of persistent CTAs: the successor may queue now
+    if (__ldg(p.nfail) == 0) return;
+    const int64_t nb = (p.n + 1) / 2;
+    for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < p.m * nb; q += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t j = q / nb;
+        if (__ldg(p.fail + j)) p.R[0][q] = prep_row<RG>(p, j, q - j * nb).Y;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -578,18 +594,14 @@ __device__ __forceinline__ void try_solve(const MpPassArgs& p, const TryTile& t,
     // fails, the general passes redo these rows with values equal to within
     // the truncation, so the maxima stand either way.
     const int klo = (int)(t.wlo - t.t0), khi = (int)(t.whi - t.t0);
+    const XView xv = x_view(p.sweep, p.max_sweeps, p.X0f, p.xout, p.oss, p.ors, p.rg);
     float dmax = 0.0f;
     unsigned long long xbits = 0ull;
     for (int k = klo + threadIdx.x; k < khi; k += blockDim.x) {
         const int64_t i0 = 2 * (t.t0 + k);
         const float2 v = sY[swz(k)];
-        if (i0 + 1 < p.n) {
-            x_update_pair(p.xsrc, p.xsrc_ss, p.xsrc_rs, p.xsrc_rg, p.xdst, p.xdst_ss, p.xdst_rs, p.xdst_rg, t.j, i0,
-                          v, dmax, xbits);
-        } else {
-            x_update(p.xsrc, p.xsrc_ss, p.xsrc_rs, p.xsrc_rg, p.xdst, p.xdst_ss, p.xdst_rs, p.xdst_rg, t.j, i0, v.x,
-                     dmax, xbits);
-        }
+        if (i0 + 1 < p.n) x_update_pair(xv, p.n, t.j, i0, v, dmax, xbits);
+        else x_update(xv, p.n, t.j, i0, v.x, dmax, xbits);
     }
     dmax = warp_max(dmax);
     const float xmax = warp_max(d2f_scaled(__longlong_as_double((long long)xbits), 0));
@@ -626,12 +638,12 @@ mp_try_kernel(MpPassArgs p)
 // Sweep 0 fused (prep, windowed cyclic reduction and the first refinement),
 // for windows that decouple (or hold the whole system).  Per window tile:
 //  1. FP64 bands and y of the tile's block rows -> row-scaled, normalised FP32
-//     blocks in shared memory; the window's own rows also go to S0, Mi and
-//     R[0] for the later sweeps and the general passes;
+//     blocks in shared memory; the window's own rows also go to S0 for the
+//     later sweeps and the general passes;
 //  2. cyclic reduction and back substitution (as mp_try_item): dx_0;
 //  3. x_0 = dx_0 on the window's rows and one block row each side (exact
 //     there: the valid region of the tile reaches 2 block rows beyond the
-//     window), written to X[0]; norms of dx_0 and x_0;
+//     window), written to X0f; norms of dx_0 and x_0;
 //  4. r_0 = y - A x_0 in FP64 for the window's rows (bands and y read again,
 //     from L2), row-scaled and normalised -> R[1].
 // No decision is needed in sweep 0, so nothing waits for other windows.  A
@@ -672,27 +684,28 @@ __device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, 
     double2* sX = reinterpret_cast<double2*>(sL);
     const int xlo = max(klo - 1, 0), xhi = min(khi + 1, TR);
     float dmax = 0.0f;
-    unsigned long long xbits = 0ull;
+    bool nan = false;
     for (int k = xlo + tid; k < xhi; k += bd) {
         const float2 v = sY[swz(k)];
         const double2 x = make_double2(f2d(v.x), f2d(v.y));
         sX[swz(k)] = x;
         if (k >= klo && k < khi) {
+            // x_0 = dx_0: one maximum for both norms
             const int64_t i0 = 2 * (t0 + k), q = j * n + i0;
             dmax = fmaxf(dmax, fabsf(v.x));
-            xbits = max(xbits, absbits(x.x));
+            nan |= v.x != v.x;
             if (i0 + 1 < n) {
-                if ((q & 1) == 0) *reinterpret_cast<double2*>(p.X0 + q) = x;   // (X0 is 256-byte aligned)
-                else { p.X0[q] = x.x; p.X0[q + 1] = x.y; }
+                if ((q & 1) == 0) *reinterpret_cast<float2*>(p.X0f + q) = v;   // (X0f is 256-byte aligned)
+                else { p.X0f[q] = v.x; p.X0f[q + 1] = v.y; }
                 dmax = fmaxf(dmax, fabsf(v.y));
-                xbits = max(xbits, absbits(x.y));
+                nan |= v.y != v.y;
             } else {
-                p.X0[q] = x.x;
+                p.X0f[q] = v.x;
             }
         }
     }
+    const float xmax = warp_max(nan ? __int_as_float(0x7FC00000) : dmax);
     dmax = warp_max(dmax);
-    float xmax = warp_max(d2f_scaled(__longlong_as_double((long long)xbits), 0));
     if ((tid & 31) == 0) {
         atomic_max_pos(&p.ndx[j], dmax);
         atomic_max_pos(&p.nx[j], xmax);
@@ -725,8 +738,8 @@ __device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, 
             rf1 = d2f_scaled(r1, d_exponent(P.c1));
         }
         const float rf0 = d2f_scaled(r0, d_exponent(P.c0));
-        const float4 Mi = p.Mi[j * nb + kb];
-        p.R[1][j * nb + kb] = make_float2(fmaf(Mi.x, rf0, Mi.y * rf1), fmaf(Mi.z, rf0, Mi.w * rf1));
+        const M2 Mi = diag_inverse(P, i0, n);     // (formed again: cheaper than keeping it)
+        p.R[1][j * nb + kb] = make_float2(fmaf(Mi.m0, rf0, Mi.m1 * rf1), fmaf(Mi.m2, rf0, Mi.m3 * rf1));
     }
 }
 
@@ -796,11 +809,10 @@ mp_pass_kernel(MpPassArgs p)
 // ---------------------------------------------------------------------------
 // refinement: x_s = x_{s-1} + dx_s (FP64), decide, r_s = y - A x_s
 // ---------------------------------------------------------------------------
-// Iterates: sweep 0 writes x_0 to X0 (workspace), every later sweep reads
+// Iterates: sweep 0 writes x_0 to X0f (workspace), every later sweep reads
 // x_{s-1} and writes x_s in the output (the caller's y, or Xout when the
 // report keeps y): a system that finishes in sweep s already holds its
-// answer there, and the rhs is read from the copy Yc.  The host passes each
-// sweep's source and destination (xsrc, xdst with their strides).
+// answer there, and the rhs is read from the copy Yc (x_view).
 
 // Systems whose dx came from the general passes (all of them when no cyclic-
 // reduction pass ran): x_s = x_{s-1} + dx_s and max |x_s|.
@@ -814,6 +826,7 @@ mp_xupdate_kernel(MpArgs p)
     const int s = p.sweep;
     if (__ldg(p.live + s) == 0) return;           // every system finished in an earlier sweep
     if (p.cr_mode && __ldg(p.nfail) == 0) return; // the cyclic-reduction passes updated every system
+    const XView xv = x_view(s, p.max_sweeps, p.X0f, p.xout, p.oss, p.ors, p.rg);
     constexpr int XT = 4 * kMpThreads;            // rows per tile
     const int64_t n = p.n, tiles = (n + XT - 1) / XT;
     for (int64_t blk = blockIdx.x; blk < p.m * tiles; blk += gridDim.x) {
@@ -825,8 +838,7 @@ mp_xupdate_kernel(MpArgs p)
 #pragma unroll
         for (int u = 0; u < 4; u++) {
             const int64_t i = t0 + threadIdx.x + u * kMpThreads;
-            if (i < n) x_update(p.xsrc, p.xsrc_ss, p.xsrc_rs, p.xsrc_rg, p.xdst, p.xdst_ss, p.xdst_rs, p.xdst_rg, j,
-                                i, p.dx[j * n + i], dmax, xbits);
+            if (i < n) x_update(xv, n, j, i, p.dx[j * n + i], dmax, xbits);
         }
         float xmax = warp_max(d2f_scaled(__longlong_as_double((long long)xbits), 0));
         if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = xmax;
@@ -879,7 +891,7 @@ mp_decide_kernel(MpArgs p)
 // the rest of the batch between sweeps and the whole solve is one launch.
 // Per system:
 //  1. FP64 bands and y -> row-scaled, normalised FP32 blocks (prep_row): in
-//     shared memory for the first solve, and in S0, Mi for the later ones;
+//     shared memory for the first solve, and in S0 for the later ones;
 //  2. per sweep: cyclic reduction to the top and back substitution (dx_s),
 //     x_s = x_{s-1} + dx_s in FP64 (X0, contiguous), the maxima of |dx_s| and
 //     |x_s| over the CTA, the stopping rule; if another sweep follows,
@@ -928,7 +940,6 @@ mp_small_kernel(MpArgs p)
             const int64_t q = j * nb + k;
             p.S0[2 * q] = f4(r.L);
             p.S0[2 * q + 1] = f4(r.U);
-            p.Mi[q] = f4(r.Mi);
             const int sk = swz(k);
             sL[sk] = f4(r.L); sU[sk] = f4(r.U); sY[sk] = r.Y;
         }
@@ -983,9 +994,9 @@ mp_small_kernel(MpArgs p)
                     if (p.e && i0 + 3 < n) r1 = fma(-P.e1, x3, r1);
                     rf1 = d2f_scaled(r1, d_exponent(P.c1));
                 }
-                const float4 Mi = p.Mi[q];
+                const M2 Mi = diag_inverse(P, i0, n);
                 const int sk = swz(k);
-                sY[sk] = make_float2(fmaf(Mi.x, rf0, Mi.y * rf1), fmaf(Mi.z, rf0, Mi.w * rf1));
+                sY[sk] = make_float2(fmaf(Mi.m0, rf0, Mi.m1 * rf1), fmaf(Mi.m2, rf0, Mi.m3 * rf1));
                 sL[sk] = p.S0[2 * q];
                 sU[sk] = p.S0[2 * q + 1];
             }
@@ -1000,10 +1011,11 @@ mp_small_kernel(MpArgs p)
 // r_s = y - A x_s (FP64, FMA chain) for the systems still running, row-scaled
 // to FP32 by the power of two of the main diagonal; the odd row of a block
 // row reaches the even lane by a shuffle, which normalises the pair by the
-// block's diagonal inverse -> R[(s+1) & 1], the rhs of sweep s+1.
+// block's diagonal inverse (formed again from the bands it has in hand) ->
+// R[(s+1) & 1], the rhs of sweep s+1.
 template <bool RG>
-__device__ __forceinline__ void residual_tile(const MpArgs& p, int s, const double* __restrict__ x, int64_t xss,
-                                              int64_t xrs, const longlong2* xrg, int64_t j, int64_t tile, double* sx)
+__device__ __forceinline__ void residual_tile(const MpArgs& p, int s, const XView& xv, int64_t j, int64_t tile,
+                                              double* sx)
 {
     const int tid = threadIdx.x;
     const int64_t n = p.n;
@@ -1015,7 +1027,9 @@ __device__ __forceinline__ void residual_tile(const MpArgs& p, int s, const doub
     // identity rows beyond, and its slots coupling to them are zero)
     int64_t base = j * p.ss, rs = p.rs, nj = n;
     if (RG) { const longlong2 g = __ldg(p.rg + j); base = g.x; rs = 1; nj = g.y; }
-    else xrg = nullptr;
+    auto x_at = [&](int64_t i) {
+        return xv.dstf ? f2d(xv.dstf[j * n + i]) : x_read(xv.dst, xv.dss, xv.drs, RG ? xv.drg : nullptr, j, i);
+    };
     double ba[XR], bb[XR], bc[XR], bd[XR], be[XR], by[XR];
 #pragma unroll
     for (int u = 0; u < XR; u++) {
@@ -1029,10 +1043,10 @@ __device__ __forceinline__ void residual_tile(const MpArgs& p, int s, const doub
                 if (p.e && i + 2 < nj) be[u] = p.e[g];
             }
             by[u] = p.Yc[j * n + i];
-            sx[tid + u * kMpThreads + 2] = x_read(x, xss, xrs, xrg, j, i);
+            sx[tid + u * kMpThreads + 2] = x_at(i);
         }
     }
-    if (halo) sx[ih - t0 + 2] = x_read(x, xss, xrs, xrg, j, ih);
+    if (halo) sx[ih - t0 + 2] = x_at(ih);
     __syncthreads();
 
     const int64_t nb = (n + 1) / 2;
@@ -1042,8 +1056,13 @@ __device__ __forceinline__ void residual_tile(const MpArgs& p, int s, const doub
         const int r0 = tid + u * kMpThreads;               // row within the tile (even lanes: first row of a block row)
         const int64_t i = t0 + r0;
         const bool even = (r0 & 1) == 0;
-        float4 Mi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (even && i < t1) Mi = p.Mi[j * nb + (i >> 1)];
+        // the row's part of the diagonal block, scaled as in the prep (an
+        // identity row past an odd system's end)
+        const int sh = d_exponent(bc[u]);
+        const bool in = i < t1;
+        const float dc = in ? d2f_scaled(bc[u], sh) : 1.0f;
+        const float dn = in && (!even || i + 1 < n) ? d2f_scaled(even ? bd[u] : bb[u], sh) : 0.0f;
+        const float dc1 = __shfl_xor_sync(0xffffffffu, dc, 1), dn1 = __shfl_xor_sync(0xffffffffu, dn, 1);
         float rf = 0.0f;
         if (i < t1) {
             const int li = r0 + 2;
@@ -1060,13 +1079,15 @@ __device__ __forceinline__ void residual_tile(const MpArgs& p, int s, const doub
                 if (i + 1 < n) r = fma(-bd[u], sx[li + 1], r);
                 if (p.e && i + 2 < n) r = fma(-be[u], sx[li + 2], r);
             }
-            rf = d2f_scaled(r, d_exponent(bc[u]));
+            rf = d2f_scaled(r, sh);
         }
         // (the partner of row n-1 of an odd system is the identity row of the
         // padded block, r = 0: its lane lies past t1 and keeps rf = 0)
         const float rf1 = __shfl_xor_sync(0xffffffffu, rf, 1);
-        if (even && i < t1)
-            p.R[(s + 1) & 1][j * nb + (i >> 1)] = make_float2(fmaf(Mi.x, rf, Mi.y * rf1), fmaf(Mi.z, rf, Mi.w * rf1));
+        if (even && in) {
+            const M2 Mi = minv({dc, dn, dn1, dc1});
+            p.R[(s + 1) & 1][j * nb + (i >> 1)] = make_float2(fmaf(Mi.m0, rf, Mi.m1 * rf1), fmaf(Mi.m2, rf, Mi.m3 * rf1));
+        }
     }
 }
 
@@ -1080,13 +1101,7 @@ mp_residual_kernel(MpArgs p)
     pdl_release();                                // one wave of persistent CTAs: the successor may queue now
     // (resolved into locals: the argument block itself stays read-only)
     const int s = p.ctr ? *p.ctr : p.sweep;
-    const double* x = p.xdst;
-    int64_t xss = p.xdst_ss, xrs = p.xdst_rs;
-    const longlong2* xrg = p.xdst_rg;
-    if (p.ctr) {
-        const XView v = x_view(s, p.max_sweeps, p.X0, p.xout, p.n, p.oss, p.ors, p.rg);
-        x = v.dst; xss = v.dss; xrs = v.drs; xrg = v.drg;
-    }
+    const XView xv = x_view(s, p.max_sweeps, p.X0f, p.xout, p.oss, p.ors, p.rg);
     if (__ldg(p.live + s + 1) == 0) return;       // every system has finished
     const bool fused0 = p.first_fused && s == 0;  // the fused sweep 0 formed r_0 of the systems it solved
     if (fused0 && __ldg(p.nfail) == 0) return;
@@ -1095,7 +1110,7 @@ mp_residual_kernel(MpArgs p)
         const int64_t j = blk / tiles;
         if (__ldg(p.fin + j) != 0) continue;
         if (fused0 && !__ldg(p.fail + j)) continue;
-        residual_tile<RG>(p, s, x, xss, xrs, xrg, j, blk - j * tiles, sx);
+        residual_tile<RG>(p, s, xv, j, blk - j * tiles, sx);
         __syncthreads();
     }
 }
@@ -1310,6 +1325,16 @@ cudaError_t launch_mp_prep(const MpArgs& p, cudaStream_t s)
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((p.m * nb + kMpThreads - 1) / kMpThreads, 152 * 16));
     const cudaError_t e = launch_dependent(p.rg ? mp_prep_kernel<true> : mp_prep_kernel<false>, (unsigned)blocks,
                                            kMpThreads, 0, s, p);
+    count_launch();
+    return e;
+}
+
+cudaError_t launch_mp_rhs(const MpArgs& p, cudaStream_t s)
+{
+    auto kern = p.rg ? mp_rhs_kernel<true> : mp_rhs_kernel<false>;
+    const int64_t need = (p.m * ((p.n + 1) / 2) + kMpThreads - 1) / kMpThreads;
+    const int64_t blocks = std::min<int64_t>(need, mp_grid_cap((const void*)kern, kMpThreads, 0));
+    const cudaError_t e = launch_dependent(kern, (unsigned)blocks, kMpThreads, 0, s, p);
     count_launch();
     return e;
 }

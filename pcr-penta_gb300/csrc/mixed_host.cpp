@@ -50,7 +50,7 @@ MpPlan mp_plan(int64_t nb, const pcrp_opts* o)
 }
 
 struct MpLayout {
-    size_t S0, R, Mi, P0, P1, dx, X0, Yc, Xout, ctr, ndx, nx, fin, status, est, trunc, ndx_pre, live, fail, nfail, dnorm,
+    size_t S0, R, P0, P1, dx, X0, Yc, Xout, ctr, ndx, nx, fin, status, est, trunc, ndx_pre, live, fail, nfail, dnorm,
         err, sum, rn, total;
 };
 
@@ -62,7 +62,6 @@ MpLayout mp_layout(int64_t m, int64_t n, int max_sweeps, const MpPlan& pl, bool 
     auto take = [&](size_t bytes) { size_t o = off; off += (bytes + 255) / 256 * 256; return o; };
     L.S0 = take(2 * T * sizeof(float4));
     L.R = take(2 * T * sizeof(float2));
-    L.Mi = take(T * sizeof(float4));
     L.P0 = pl.s1 > 0 ? take(2 * T * sizeof(float4) + T * sizeof(float2)) : 0;
     L.P1 = pl.npass > 1 ? take(2 * T * sizeof(float4) + T * sizeof(float2)) : 0;
     L.dx = take((size_t)m * n * sizeof(float));
@@ -112,12 +111,6 @@ pcrp_status enqueue_sweep(MpArgs A, const SweepPlan& S, int s, cudaStream_t st)
     cudaError_t ce;
     if (!dev) {
         A.sweep = s;
-        A.xsrc_rg = nullptr; A.xdst_rg = nullptr;
-        if (s == 0) { A.xsrc = nullptr; A.xsrc_ss = 0; A.xsrc_rs = 0; }
-        else if (s == 1) { A.xsrc = A.X0; A.xsrc_ss = n; A.xsrc_rs = 1; }
-        else { A.xsrc = A.xout; A.xsrc_ss = A.oss; A.xsrc_rs = A.ors; A.xsrc_rg = A.rg; }
-        if (s == 0 && A.max_sweeps >= 2) { A.xdst = A.X0; A.xdst_ss = n; A.xdst_rs = 1; }
-        else { A.xdst = A.xout; A.xdst_ss = A.oss; A.xdst_rs = A.ors; A.xdst_rg = A.rg; }
     }
 
     // FP32 block solve of the normalised system with rhs R[s & 1]
@@ -125,9 +118,9 @@ pcrp_status enqueue_sweep(MpArgs A, const SweepPlan& S, int s, cudaStream_t st)
     p.srcLU = A.S0;
     p.dx = A.dx; p.fin = A.fin; p.ndx = A.ndx;
     p.m = m; p.n = n; p.nb = nb; p.G = 1;
+    p.X0f = A.X0f; p.xout = A.xout; p.oss = A.oss; p.ors = A.ors; p.rg = A.rg; p.max_sweeps = A.max_sweeps;
     if (dev) {
         p.ctr = A.ctr; p.live0 = A.live; p.R0 = A.R[0]; p.R1 = A.R[1]; p.pre0 = A.ndx_pre;
-        p.X0 = A.X0; p.xout = A.xout; p.oss = A.oss; p.ors = A.ors; p.rg = A.rg; p.max_sweeps = A.max_sweeps;
     } else {
         p.sweep = s; p.srcY = A.R[s & 1]; p.live = A.live + s;
     }
@@ -142,8 +135,6 @@ pcrp_status enqueue_sweep(MpArgs A, const SweepPlan& S, int s, cudaStream_t st)
         if (dev) {
             t.pre0 = nullptr; t.level0 = 1; t.nx0 = A.nx; t.skip0 = S.fused;
         } else {
-            t.xsrc = A.xsrc; t.xsrc_ss = A.xsrc_ss; t.xsrc_rs = A.xsrc_rs; t.xsrc_rg = A.xsrc_rg;
-            t.xdst = A.xdst; t.xdst_ss = A.xdst_ss; t.xdst_rs = A.xdst_rs; t.xdst_rg = A.xdst_rg;
             t.nx = A.nx + (size_t)s * m;
         }
         ce = launch_mp_try(t, st);
@@ -259,6 +250,7 @@ bool capture_sweep_loop(const MpArgs& A, const SweepPlan& S, cudaStream_t st)
     if (S.duo && (launch_mp_duo(A, S.D, st) != cudaSuccess || launch_mp_duo_finish(A, st) != cudaSuccess))
         return false;
     if ((S.fused ? launch_mp_first(A, S.W, st) : launch_mp_prep(A, st)) != cudaSuccess) return false;
+    if (S.fused && launch_mp_rhs(A, st) != cudaSuccess) return false;
     if (S.duo && launch_mp_gate(A, h, st) != cudaSuccess) return false;
     if (cudaStreamGetCaptureInfo(st, &status, nullptr, &g, &deps, nullptr, &ndeps) != cudaSuccess ||
         status != cudaStreamCaptureStatusActive)
@@ -393,9 +385,9 @@ pcrp_status mixed_enqueue(const double* a, const double* b, const double* c, con
     A.S0 = reinterpret_cast<float4*>(base + WL.S0);
     A.R[0] = reinterpret_cast<float2*>(base + WL.R);
     A.R[1] = A.R[0] + T;
-    A.Mi = reinterpret_cast<float4*>(base + WL.Mi);
     A.dx = F(WL.dx);
     A.X0 = reinterpret_cast<double*>(base + WL.X0);
+    A.X0f = reinterpret_cast<float*>(A.X0);
     A.Yc = reinterpret_cast<double*>(base + WL.Yc);
     A.Xout = keep_x ? reinterpret_cast<double*>(base + WL.Xout) : nullptr;
     A.ndx = U(WL.ndx); A.nx = U(WL.nx);
@@ -487,6 +479,7 @@ pcrp_status mixed_enqueue(const double* a, const double* b, const double* c, con
         if (ce != cudaSuccess) return cuda_error(ce, "mixed fused-sweeps launch");
     }
     ce = S.fused ? launch_mp_first(A, S.W, st) : launch_mp_prep(A, st);
+    if (ce == cudaSuccess && S.fused) ce = launch_mp_rhs(A, st);
     if (ce != cudaSuccess) return cuda_error(ce, S.fused ? "mixed first-sweep launch" : "mixed prep launch");
     for (int s = 0; s < max_sweeps; s++) {
         const pcrp_status rc = enqueue_sweep(A, S, s, st);

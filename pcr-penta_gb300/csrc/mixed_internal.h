@@ -24,17 +24,11 @@ struct MpArgs {
                                         // there; null: uniform batch addressed by (ss, rs)
     float4* S0;                         // level-0 normalised L,U: [2*q] = L, [2*q+1] = U, q < m*nb
     float2* R[2];                       // normalised rhs Y of block row q: sweep s reads R[s & 1]
-    float4* Mi;                         // inverse of the row-scaled FP32 diagonal block of block row q
     float* dx;                          // FP32 correction, m*n (contiguous)
-    double* X0;                         // x_0, m*n contiguous (sweep 0 of a multi-sweep solve)
+    double* X0;                         // iterate of the whole-system kernel / x_1 of the fused first sweeps, m*n
+    float* X0f;                         // x_0 (a float: the first correction), m*n contiguous (the same memory)
     double* Xout;                       // iterates when the caller asked for a report (keep_x), else y
     double* Yc;                         // copy of the rhs, m*n contiguous (y may hold the iterate)
-    const double* xsrc;                 // this sweep's x_{s-1} (null in sweep 0) ...
-    int64_t xsrc_ss, xsrc_rs;           //   ... and its system / row strides
-    const longlong2* xsrc_rg;           //   ... or its ragged rows (rg, when xsrc is the output)
-    double* xdst;                       // this sweep's x_s ...
-    int64_t xdst_ss, xdst_rs;
-    const longlong2* xdst_rg;
     double* xout;                       // the output iterate (y or Xout) and its strides: x_s of sweeps >= 1
     int64_t oss, ors;
     int* ctr;                           // device sweep counter (graph-driven sweeps), or null: `sweep` and the
@@ -77,15 +71,9 @@ struct MpPassArgs {
     int* fail;                          // per system: the windowed cyclic-reduction pass did not decouple it
                                         // (null: no such pass; general passes then run for every system)
     int* nfail;                         // number of systems with fail set
-    const double* xsrc;                 // cyclic-reduction passes: x_{s-1} (null in sweep 0) ...
-    int64_t xsrc_ss, xsrc_rs;
-    const longlong2* xsrc_rg;
-    double* xdst;                       //   ... and x_s = x_{s-1} + dx_s (null: write dx instead)
-    int64_t xdst_ss, xdst_rs;
-    const longlong2* xdst_rg;
-    unsigned* nx;                       //   ... and max |x_s|
+    unsigned* nx;                       // cyclic-reduction passes: max |x_s|
     // Graph-driven sweeps: the fields above that change from sweep to sweep
-    // (sweep, live, srcY at level 0, ndx_pre_in/out, xsrc, xdst, nx) are
+    // (sweep, live, srcY at level 0, ndx_pre_in/out, nx) are
     // derived on the device from the sweep counter and these:
     const int* ctr;                     // device sweep counter, or null (host-set fields)
     const int* live0;
@@ -93,7 +81,7 @@ struct MpPassArgs {
     const float2* R1;
     unsigned* pre0;                     // ndx_pre base
     unsigned* nx0;                      // nx base (cyclic-reduction pass)
-    const double* X0;
+    float* X0f;                         // iterates (see MpArgs)
     double* xout;
     int64_t oss, ors;
     const longlong2* rg;                // ragged output rows (see MpArgs::rg)
@@ -163,6 +151,7 @@ pcrp_status mixed_enqueue(const double* a, const double* b, const double* c, con
 cudaError_t launch_mp_init(const MpArgs& p, cudaStream_t s);
 cudaError_t launch_mp_first(const MpArgs& p, const MpWindows& g, cudaStream_t s);
 cudaError_t launch_mp_prep(const MpArgs& p, cudaStream_t s);
+cudaError_t launch_mp_rhs(const MpArgs& p, cudaStream_t s);
 cudaError_t launch_mp_pass(const MpPassArgs& p, cudaStream_t s);
 cudaError_t launch_mp_small(const MpArgs& p, cudaStream_t s);   // whole systems, every sweep in one CTA
 cudaError_t launch_mp_try(const MpPassArgs& p, cudaStream_t s);
