@@ -307,6 +307,52 @@ __device__ __forceinline__ PrepRow prep_row(const MpArgs& p, int64_t j, int64_t 
     return r;
 }
 
+// A run of block rows of one system whose band slots all lie inside it
+// (contiguous rows, every pair 16-byte aligned): the arrays from the run's
+// first row on, a null outer band zero.  One address per array and run instead
+// of the general row's index arithmetic and tests.
+struct PairRun { const double *a, *b, *c, *d, *e, *y; };
+
+__device__ __forceinline__ PairRun pair_run(const MpArgs& p, int64_t row)
+{
+    return {p.a ? p.a + row : nullptr, p.b + row, p.c + row, p.d + row, p.e ? p.e + row : nullptr, p.y + row};
+}
+
+__device__ __forceinline__ PairRow load_run(const PairRun& s, int k, Keep keep, uint64_t pol)
+{
+    const double2 z = make_double2(0.0, 0.0);
+    const double2 a = s.a ? ldg2(s.a + 2 * k, keep, pol) : z;
+    const double2 b = ldg2(s.b + 2 * k, keep, pol), c = ldg2(s.c + 2 * k, keep, pol);
+    const double2 d = ldg2(s.d + 2 * k, keep, pol);
+    const double2 e = s.e ? ldg2(s.e + 2 * k, keep, pol) : z;
+    const double2 y = ldg2(s.y + 2 * k, keep, pol);
+    return {a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, e.x, e.y, y.x, y.y};
+}
+
+// r = y - A x of a block row whose band slots all lie inside the system
+// (x_{i0-2..i0+3} = xm, xc, xp; the FMA order of residual_kernel), row-scaled
+// and normalised by its diagonal block's inverse (formed again: cheaper than
+// keeping it): the next right-hand side.
+__device__ __forceinline__ float2 residual_inner(const PairRow& P, bool has_a, bool has_e, double2 xm, double2 xc,
+                                                 double2 xp, int64_t i0, int64_t n)
+{
+    double r0 = fma(-P.c0, xc.x, P.y0), r1 = fma(-P.c1, xc.y, P.y1);
+    if (has_a) { r0 = fma(-P.a0, xm.x, r0); r1 = fma(-P.a1, xm.y, r1); }
+    r0 = fma(-P.b0, xm.y, r0); r1 = fma(-P.b1, xc.x, r1);
+    r0 = fma(-P.d0, xc.y, r0); r1 = fma(-P.d1, xp.x, r1);
+    if (has_e) { r0 = fma(-P.e0, xp.x, r0); r1 = fma(-P.e1, xp.y, r1); }
+    const RowScale s0 = row_scale(P.c0), s1 = row_scale(P.c1);
+    int top = 0;
+    M2 D = {d2f_row(P.c0, s0, top), d2f_row(P.d0, s0, top), d2f_row(P.b1, s1, top), d2f_row(P.c1, s1, top)};
+    float f0 = d2f_row(r0, s0, top), f1 = d2f_row(r1, s1, top);
+    if (!(s0.ok && s1.ok && row_fits(top))) {
+        D = block_of(P, i0, n).D;
+        f0 = d2f_scaled(r0, d_exponent(P.c0)); f1 = d2f_scaled(r1, d_exponent(P.c1));
+    }
+    const M2 Mi = minv(D);
+    return make_float2(fmaf(Mi.m0, f0, Mi.m1 * f1), fmaf(Mi.m2, f0, Mi.m3 * f1));
+}
+
 // Rows i0 = 2k, i0 + 1 of the rhs of system j (loaded by prep_row) -> the
 // contiguous copy Yc, one 16-byte store where the pair is aligned.
 __device__ __forceinline__ void store_rhs_pair(const MpArgs& p, int64_t j, int64_t i0, double2 y)
@@ -649,6 +695,38 @@ mp_try_kernel(MpPassArgs p)
 // No decision is needed in sweep 0, so nothing waits for other windows.  A
 // window whose system stays coupled marks it and stops after step 1; the
 // general passes and the refinement kernel then take the whole system.
+// (steps 1 and 4 of an inner tile)
+__device__ __forceinline__ void first_prep(const MpArgs& p, const PairRun& run, int64_t j, int64_t t0, int TR, int klo,
+                                           int khi, float4* sL, float4* sU, float2* sY)
+{
+    const int64_t nb = (p.n + 1) / 2;
+    float4* __restrict__ S0 = p.S0 + 2 * (j * nb + t0);
+    double* __restrict__ Yc = p.Yc + j * p.n + 2 * t0;
+    const uint64_t pol = tma::policy_evict_last();
+    for (int k = threadIdx.x; k < TR; k += blockDim.x) {
+        const PairRow P = load_run(run, k, Keep::last, pol);
+        const PrepRow r = prep_of(block_inner(P, 2 * (t0 + k), p.n));
+        const int sk = swz(k);
+        sL[sk] = f4(r.L); sU[sk] = f4(r.U); sY[sk] = r.Y;
+        if (k >= klo && k < khi) {
+            S0[2 * k] = f4(r.L);
+            S0[2 * k + 1] = f4(r.U);
+            *reinterpret_cast<double2*>(Yc + 2 * k) = make_double2(P.y0, P.y1);
+        }
+    }
+}
+
+__device__ __forceinline__ void first_residual(const MpArgs& p, const PairRun& run, int64_t j, int64_t t0, int klo,
+                                               int khi, const double2* sX)
+{
+    float2* __restrict__ R = p.R[1] + j * ((p.n + 1) / 2) + t0;
+    const uint64_t pol = tma::policy_evict_first();
+    for (int k = klo + (int)threadIdx.x; k < khi; k += blockDim.x) {
+        const PairRow P = load_run(run, k, Keep::first, pol);
+        R[k] = residual_inner(P, run.a != nullptr, run.e != nullptr, sX[k - 1], sX[k], sX[k + 1], 2 * (t0 + k), p.n);
+    }
+}
+
 template <bool RG>
 __device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, int64_t item,
                                            float4* sL, float4* sU, float2* sY)
@@ -661,7 +739,12 @@ __device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, 
     const int TR = (int)(t1 - t0);
     const bool whole = t0 == 0 && t1 == nb;
 
-    for (int k = tid; k < TR; k += bd) {
+    // an inner tile: one aligned run of rows, every band slot in the system
+    int64_t base = j * p.ss, nj = n;
+    if (RG) { const longlong2 r = __ldg(p.rg + j); base = r.x; nj = r.y; }
+    const bool inner = (RG || p.rs == 1) && t0 >= 1 && 2 * t1 + 2 <= nj && p.vec && ((base | (j * n)) & 1) == 0;
+    if (inner) first_prep(p, pair_run(p, base + 2 * t0), j, t0, TR, (int)(wlo - t0), (int)(whi - t0), sL, sU, sY);
+    else for (int k = tid; k < TR; k += bd) {
         const int64_t kb = t0 + k;
         const PrepRow r = prep_row<RG>(p, j, kb, Keep::last);
         const int sk = swz(k);
@@ -687,8 +770,7 @@ __device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, 
     bool nan = false;
     for (int k = xlo + tid; k < xhi; k += bd) {
         const float2 v = sY[swz(k)];
-        const double2 x = make_double2(f2d(v.x), f2d(v.y));
-        sX[swz(k)] = x;
+        sX[k] = make_double2(f2d(v.x), f2d(v.y));
         if (k >= klo && k < khi) {
             // x_0 = dx_0: one maximum for both norms
             const int64_t i0 = 2 * (t0 + k), q = j * n + i0;
@@ -714,12 +796,13 @@ __device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, 
 
     // r_0 = y - A x_0 on the window's block rows (FP64, same FMA order as the
     // refinement kernel), row-scaled and normalised -> the rhs of sweep 1
+    if (inner) { first_residual(p, pair_run(p, base + 2 * t0), j, t0, klo, khi, sX); return; }
     for (int k = klo + tid; k < khi; k += bd) {
         const int64_t kb = t0 + k, i0 = 2 * kb;
         const PairRow P = load_pair<RG>(p, j, i0, Keep::first);
-        const double2 xm = k > 0 ? sX[swz(k - 1)] : make_double2(0.0, 0.0);
-        const double2 xc = sX[swz(k)];
-        const double2 xp = k + 1 < TR ? sX[swz(k + 1)] : make_double2(0.0, 0.0);
+        const double2 xm = k > 0 ? sX[k - 1] : make_double2(0.0, 0.0);
+        const double2 xc = sX[k];
+        const double2 xp = k + 1 < TR ? sX[k + 1] : make_double2(0.0, 0.0);
         double r0 = P.y0;                          // row i0: x_{i0-2..i0+2} = xm.x xm.y xc.x xc.y xp.x
         r0 = fma(-P.c0, xc.x, r0);
         if (p.a && i0 >= 2) r0 = fma(-P.a0, xm.x, r0);
