@@ -232,6 +232,7 @@ pcrp_status f64_solve(const double* a, const double* b, const double* c, const d
         p.src_ss = n; p.src_rs = 1; p.src_sub = 1;
         cur ^= 1;
         p.G <<= K;
+        p.lg += K;
     }
 
     // shared-memory finish on whole subsystems of at most smem_rows rows

@@ -54,11 +54,8 @@ __global__ void __launch_bounds__(kMaxThreads, CAP > 1024 ? 1 : CAP > 544 ? 2 : 
 pcr_pass_kernel(const PcrPassArgs p)
 {
     extern __shared__ __align__(16) unsigned char pcr_smem[];
-    const int64_t blk  = blockIdx.x;
-    const int64_t item = blk / p.nwin;
-    const int64_t w    = blk - item * p.nwin;
-    const int64_t j    = item / p.G;
-    const int64_t r    = item - j * p.G;
+    const uint32_t blk = blockIdx.x, nwin = (uint32_t)p.nwin, item = blk / nwin, w = blk - item * nwin;
+    const uint32_t j = item >> p.lg, r = item & ((1u << p.lg) - 1);
     pcr_tile<CAP, false, kFew>(p, j, r, w, *reinterpret_cast<TileRows<CAP>*>(pcr_smem));
 }
 

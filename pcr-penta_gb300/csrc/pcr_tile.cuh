@@ -411,23 +411,26 @@ __device__ __forceinline__ double gload(const double* p) {
 // kFew: the launch leaves most of the SM's warp slots empty; every row takes
 // the general form.
 template <int CAP, bool kL2Only = false, bool kFew = false>
-__device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_t r, int64_t w, TileRows<CAP>& T)
+__device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32_t r, uint32_t w, TileRows<CAP>& T)
 {
+    // row numbers inside a system fit 32 bits (n <= 2^31), and G = 2^lg: a
+    // 64-bit division is ~80 instructions, and every thread runs this code for
+    // two rows of a tile
+    const int lg = p.lg;
     const int64_t sbase = p.offsets ? p.offsets[j] : j * p.src_ss;
     const int64_t dbase = p.offsets ? p.offsets[j] : j * p.dst_ss;
-    const int64_t nsys = p.offsets ? (p.offsets[j + 1] - p.offsets[j]) : p.n;
+    const uint32_t nsys = (uint32_t)(p.offsets ? (p.offsets[j + 1] - p.offsets[j]) : p.n);
     if (r >= nsys) return;
-    const int64_t nr  = (nsys - 1 - r) / p.G + 1;           // rows of subsystem r
-    const int64_t wlo = w * (int64_t)p.L;
+    const uint32_t nr = ((nsys - 1 - r) >> lg) + 1;          // rows of subsystem r
+    const uint32_t wlo = w * (uint32_t)p.L;
     if (wlo >= nr) return;
-    const int64_t whi = min(wlo + (int64_t)p.L, nr);
-    const int64_t t0  = max(wlo - (int64_t)p.H, (int64_t)0);
-    const int64_t t1  = min(whi + (int64_t)p.H, nr);
+    const uint32_t whi = min(wlo + (uint32_t)p.L, nr);
+    const uint32_t t0 = wlo - min(wlo, (uint32_t)p.H), t1 = min(whi + (uint32_t)p.H, nr);
     const int TR = (int)(t1 - t0);
     const int tid = threadIdx.x, bd = blockDim.x;
     // distance of local rows t, t+1 and local row 0 of the source
     const int64_t sstep = p.src_sub ? 1 : p.G * p.src_rs;
-    const int64_t soff = p.src_sub ? sbase + r * (nsys / p.G) + min(r, nsys % p.G) : sbase + r * p.src_rs;
+    const int64_t soff = p.src_sub ? sbase + r * (nsys >> lg) + min(r, nsys & ((1u << lg) - 1)) : sbase + r * p.src_rs;
     const int64_t dstep = p.G * p.dst_rs;
     const int64_t doff = dbase + r * p.dst_rs;
     // a null outer band (a tridiagonal batch, first pass only) is +0.0
@@ -486,7 +489,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_
     } else {
 #pragma unroll 2
         for (int k = tid; k < TR; k += bd) {
-            const int64_t gi = (t0 + k) * sstep;
+            const int64_t gi = (int64_t)(t0 + k) * sstep;
             const double a = has_a ? gload<kL2Only>(ga + gi) : 0.0;
             const double e = has_e ? gload<kL2Only>(ge + gi) : 0.0;
             const double b = gload<kL2Only>(gb + gi), c = gload<kL2Only>(gc + gi);
@@ -496,14 +499,14 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_
     }
     if (p.rem == 1)
         for (int k = tid, q = 0; k < TR; k += bd, q++) {
-            const int64_t gi = soff + (t0 + k) * sstep;
+            const int64_t gi = soff + (int64_t)(t0 + k) * sstep;
             kept1[q] = p.src[AL1_] ? gload<kL2Only>(p.src[AL1_] + gi) : 0.0;
             kept2[q] = p.src[AL1_] ? gload<kL2Only>(p.src[AL2_] + gi) : 0.0;
         }
     // local rows of the subsystem's ends: row k of the tile has a neighbour at
     // distance x iff k - x >= kfirst / k + x <= klast (32-bit: ends further
     // away than any distance of the tile are moved in to 2^14 rows)
-    const int kfirst = -(int)min(t0, (int64_t)16384), klast = (int)min(nr - 1 - t0, (int64_t)16384);
+    const int kfirst = -(int)min(t0, 16384u), klast = (int)min(nr - 1 - t0, 16384u);
 
     // A whole subsystem whose rows are all decoupled (a = b = d = e = 0, c and
     // y away from the ends of the exponent range): every further stride only
@@ -518,11 +521,10 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_
         const int dl = 1 << s;
         // rows this stride must produce: the window widened by the halo the
         // remaining strides of the pass still consume (everything if final).
-        int klo, khi;
-        if (p.final_step) { klo = 0; khi = TR; }
-        else {
-            const int64_t rem = 2 * ((int64_t(1) << p.K) - (int64_t(2) << s));
-            klo = (int)(max(wlo - rem, (int64_t)0) - t0); khi = (int)(min(whi + rem, nr) - t0);
+        int klo = 0, khi = TR;
+        if (!p.final_step) {
+            const int rem = 2 * ((1 << p.K) - (2 << s));
+            klo = max((int)(wlo - t0) - rem, kfirst); khi = min((int)(whi - t0) + rem, klast + 1);
         }
         // the rows whose T(m) those need, all in the tile
         const int Alo = max(klo - dl, 0), Ahi = min(khi + dl, TR);
@@ -615,15 +617,15 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, int64_
     } else {
         // subsystem-major output: row t of subsystem r is row t >> K of
         // subsystem r + (t mod 2^K) G at the next level's stride G 2^K
-        const int64_t G2 = p.G << p.K, q2 = nsys / G2, rem2 = nsys % G2;
-        const int64_t kmask = (int64_t(1) << p.K) - 1;
+        const int lg2 = lg + p.K;
+        const uint32_t q2 = nsys >> lg2, rem2 = nsys & ((1u << lg2) - 1), kmask = (1u << p.K) - 1;
         for (int k = tid, q = 0; k < TR; k += bd, q++) {
-            const int64_t t = t0 + k;
+            const uint32_t t = t0 + k;
             if (t >= wlo && t < whi) {
                 int64_t gi;
                 if (p.dst_sub) {
-                    const int64_t r2 = r + (t & kmask) * p.G;
-                    gi = dbase + r2 * q2 + min(r2, rem2) + (t >> p.K);
+                    const uint32_t r2 = r + ((t & kmask) << lg);
+                    gi = dbase + (r2 * q2 + min(r2, rem2) + (t >> p.K));    // (r2 * q2 <= nsys)
                 } else {
                     gi = doff + t * dstep;
                 }

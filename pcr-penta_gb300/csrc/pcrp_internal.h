@@ -54,8 +54,9 @@ struct PcrPassArgs {
     int64_t dst_ss, dst_rs;      // addressing of dst and x
     int64_t n;                   // rows of each full system (uniform batch)
     int64_t m;                   // systems
-    int64_t G;                   // gather stride = 2^(strides already done)
+    int64_t G;                   // gather stride = 2^lg, lg = strides already done
     int64_t nwin;                // windows per subsystem
+    int lg;
     int K;                       // strides run by this pass (local deltas 1..2^(K-1))
     int rem;                     // strides the subsystems have left, this pass's included; the AL1_/AL2_ arrays
                                  // are written by a pass that leaves one stride and read by the next

@@ -47,7 +47,7 @@ constexpr long long kSpinLimitInjected = 1LL << 14;   // ~4 ms: the failure-dete
 struct RgLevel {
     int64_t G, nwin;                       // gather stride before the level, windows per subsystem
     int K, H, Lw, P;                       // strides, halo, tile rows; P: the system's global levels
-    int rem;                               // strides left at the level's start
+    int rem, lg;                           // strides left at the level's start, done before it (G = 2^lg)
 };
 
 struct RgArgs {
@@ -107,6 +107,7 @@ __global__ void rg_plan_kernel(RgArgs a)
         for (int l = 0; l <= P; l++) {
             RgLevel v;
             v.rem = rem;
+            v.lg = ref_strides(n) - rem;
             rem -= K[l];
             v.G = G[l]; v.nwin = nwin[l]; v.K = K[l]; v.H = H[l]; v.Lw = Lw[l]; v.P = P;
             a.lv[(int64_t)l * a.nsys + k] = v;
@@ -195,7 +196,7 @@ rg_persistent_kernel(RgArgs a)
         }
         __syncthreads();
         const int64_t lo = s_slot;
-        const int lvl = (int)(lo / a.nsys);
+        const int lvl = (int)((uint32_t)lo / (uint32_t)a.nsys);   // (nsys <= 2^24: 32-bit slots)
         const int64_t k = lo - (int64_t)lvl * a.nsys;
         const int64_t i = item - a.start[lo];
         const int64_t n = a.offsets[k + 1] - a.offsets[k];
@@ -228,7 +229,7 @@ rg_persistent_kernel(RgArgs a)
             p.x = a.y;
             p.offsets = a.offsets;
             p.src_ss = 0; p.src_rs = 1; p.dst_ss = 0; p.dst_rs = 1;
-            p.n = n; p.m = a.nsys; p.G = lv.G;
+            p.n = n; p.m = a.nsys; p.G = lv.G; p.lg = lv.lg;
             p.K = lv.K; p.rem = lv.rem; p.final_step = fin ? 1 : 0; p.L = lv.Lw; p.H = lv.H;
             p.nwin = lv.nwin;
             p.TRmax = a.cap;
@@ -240,8 +241,8 @@ rg_persistent_kernel(RgArgs a)
             p.src_sub = lvl > 0 ? 1 : 0;
             p.dst_sub = fin ? 0 : 1;
             p.bulk = 0;                               // (per-thread loads through L2: data of this launch)
-            const int64_t r = fin ? i : i / lv.nwin;
-            const int64_t w = fin ? 0 : i - r * lv.nwin;
+            const uint32_t nwin = (uint32_t)lv.nwin, r = fin ? (uint32_t)i : (uint32_t)i / nwin;
+            const uint32_t w = fin ? 0u : (uint32_t)i - r * nwin;
             pcr_tile<kRgCap, true>(p, k, r, w, *reinterpret_cast<RgTile*>(pcr_smem));
         }
         __syncthreads();
