@@ -90,28 +90,6 @@ __device__ __forceinline__ void x_update(const XView& v, int64_t n, int64_t j, i
     xbits = max(xbits, absbits(x));
 }
 
-// Rows i0 (even) and i0 + 1 < n of system j: as two x_update calls, with
-// paired loads and stores for sweep 1 of a contiguous batch where they are
-// aligned (same values).
-__device__ __forceinline__ void x_update_pair(const XView& v, int64_t n, int64_t j, int64_t i0, float2 d, float& dmax,
-                                              unsigned long long& xbits)
-{
-    if (v.srcf && !v.dstf && !v.drg && v.drs == 1) {
-        const float* s = v.srcf + j * n + i0;
-        double* t = v.dst + j * v.dss + i0;
-        if (((reinterpret_cast<uintptr_t>(s) & 7) | (reinterpret_cast<uintptr_t>(t) & 15)) == 0) {
-            const float2 xs = *reinterpret_cast<const float2*>(s);
-            const double2 x = make_double2(__dadd_rn(f2d(xs.x), f2d(d.x)), __dadd_rn(f2d(xs.y), f2d(d.y)));
-            *reinterpret_cast<double2*>(t) = x;
-            dmax = fmaxf(dmax, fmaxf(fabsf(d.x), fabsf(d.y)));
-            xbits = max(xbits, max(absbits(x.x), absbits(x.y)));
-            return;
-        }
-    }
-    x_update(v, n, j, i0, d.x, dmax, xbits);
-    x_update(v, n, j, i0 + 1, d.y, dmax, xbits);
-}
-
 // Iterates of sweep s: x_0 in X0f when more sweeps follow, every later x_s in
 // the output; x_{s-1} is read from where sweep s-1 wrote it.
 // The output of a ragged batch is addressed through rg.
@@ -634,20 +612,45 @@ __device__ __forceinline__ void try_solve(const MpPassArgs& p, const TryTile& t,
         if (threadIdx.x == 0 && atomicOr(&p.fail[t.j], 1) == 0) atomicAdd(p.nfail, 1);
         return;
     }
-    cr_substitute(sL, sU, sY, t.TR, top);
     // x_s = x_{s-1} + dx_s on the window's rows, straight from the tile.  The
     // norms go straight into the sweep's: if another window of the system
     // fails, the general passes redo these rows with values equal to within
     // the truncation, so the maxima stand either way.
     const int klo = (int)(t.wlo - t.t0), khi = (int)(t.whi - t.t0);
     const XView xv = x_view(p.sweep, p.max_sweeps, p.X0f, p.xout, p.oss, p.ors, p.rg);
+    // sweep 1 of a contiguous batch with aligned pairs: one address per array
+    // and tile, and x_0 on its way from memory during the substitution (the
+    // last row of an odd system goes the general way below)
+    const float* __restrict__ xs = xv.srcf + t.j * p.n + 2 * t.t0;
+    double* __restrict__ xd = xv.dst + t.j * xv.dss + 2 * t.t0;
+    const bool run = xv.srcf && !xv.drg && xv.drs == 1 &&
+                     ((reinterpret_cast<uintptr_t>(xs) & 7) | (reinterpret_cast<uintptr_t>(xd) & 15)) == 0;
+    const int done = run ? (int)(min(t.whi, p.n / 2) - t.t0) : klo;
+    float2 x0[kMpTryRows / kMpTryThreads];
+#pragma unroll
+    for (int u = 0; u < kMpTryRows / kMpTryThreads; u++) {
+        const int k = klo + (int)threadIdx.x + u * kMpTryThreads;
+        if (k < done) x0[u] = reinterpret_cast<const float2*>(xs)[k];
+    }
+    cr_substitute(sL, sU, sY, t.TR, top);
     float dmax = 0.0f;
     unsigned long long xbits = 0ull;
-    for (int k = klo + threadIdx.x; k < khi; k += blockDim.x) {
+#pragma unroll
+    for (int u = 0; u < kMpTryRows / kMpTryThreads; u++) {
+        const int k = klo + (int)threadIdx.x + u * kMpTryThreads;
+        if (k < done) {
+            const float2 d = sY[swz(k)];
+            const double2 x = make_double2(__dadd_rn(f2d(x0[u].x), f2d(d.x)), __dadd_rn(f2d(x0[u].y), f2d(d.y)));
+            reinterpret_cast<double2*>(xd)[k] = x;
+            dmax = fmaxf(dmax, fmaxf(fabsf(d.x), fabsf(d.y)));
+            xbits = max(xbits, max(absbits(x.x), absbits(x.y)));
+        }
+    }
+    for (int k = done + (int)threadIdx.x; k < khi; k += blockDim.x) {
         const int64_t i0 = 2 * (t.t0 + k);
         const float2 v = sY[swz(k)];
-        if (i0 + 1 < p.n) x_update_pair(xv, p.n, t.j, i0, v, dmax, xbits);
-        else x_update(xv, p.n, t.j, i0, v.x, dmax, xbits);
+        x_update(xv, p.n, t.j, i0, v.x, dmax, xbits);
+        if (i0 + 1 < p.n) x_update(xv, p.n, t.j, i0 + 1, v.y, dmax, xbits);
     }
     dmax = warp_max(dmax);
     const float xmax = warp_max(d2f_scaled(__longlong_as_double((long long)xbits), 0));
@@ -766,6 +769,9 @@ __device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, 
     // x_0 pairs, kept as double2 in the L slots for the residual's neighbours
     double2* sX = reinterpret_cast<double2*>(sL);
     const int xlo = max(klo - 1, 0), xhi = min(khi + 1, TR);
+    float* __restrict__ X0 = p.X0f + j * n + 2 * t0;
+    const bool even = ((j * n) & 1) == 0;
+    const int pairs = (int)(n / 2 - t0);          // block rows of two rows
     float dmax = 0.0f;
     bool nan = false;
     for (int k = xlo + tid; k < xhi; k += bd) {
@@ -773,17 +779,12 @@ __device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, 
         sX[k] = make_double2(f2d(v.x), f2d(v.y));
         if (k >= klo && k < khi) {
             // x_0 = dx_0: one maximum for both norms
-            const int64_t i0 = 2 * (t0 + k), q = j * n + i0;
+            const bool two = k < pairs;
+            if (two && even) *reinterpret_cast<float2*>(X0 + 2 * k) = v;      // (X0f is 256-byte aligned)
+            else { X0[2 * k] = v.x; if (two) X0[2 * k + 1] = v.y; }
             dmax = fmaxf(dmax, fabsf(v.x));
             nan |= v.x != v.x;
-            if (i0 + 1 < n) {
-                if ((q & 1) == 0) *reinterpret_cast<float2*>(p.X0f + q) = v;   // (X0f is 256-byte aligned)
-                else { p.X0f[q] = v.x; p.X0f[q + 1] = v.y; }
-                dmax = fmaxf(dmax, fabsf(v.y));
-                nan |= v.y != v.y;
-            } else {
-                p.X0f[q] = v.x;
-            }
+            if (two) { dmax = fmaxf(dmax, fabsf(v.y)); nan |= v.y != v.y; }
         }
     }
     const float xmax = warp_max(nan ? __int_as_float(0x7FC00000) : dmax);
