@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sys
 from typing import Optional, Sequence
 
 from . import build as _build
@@ -140,11 +141,34 @@ def _check_tensor(x, count: int, dtype: str) -> None:
         raise ValueError(f"tensor of {x.numel()} elements where {count} are read")
 
 
+# torch, once it is known to be loaded, and what the argument checks ask of it
+# on every call: six tensors and a stream per solve of a few short systems took
+# 12 us of host time by way of dtype names and torch.cuda.current_stream(),
+# about as long as the kernel
+_torch = None
+_dtypes: dict = {}
+_raw_stream = None
+
+
+def _bind_torch():
+    global _torch, _raw_stream
+    t = sys.modules.get("torch")
+    if t is not None and hasattr(t, "Tensor") and hasattr(t, "cuda"):
+        _dtypes.update(float64=t.float64, int64=t.int64)
+        _raw_stream = getattr(t._C, "_cuda_getCurrentRawStream", None)
+        _torch = t
+    return _torch
+
+
 def _ptr(x, count: int = 0, dtype: str = "float64") -> Optional[int]:
     """Raw device pointer of a CUDA tensor (contiguous, of `dtype`, at least
     `count` elements) or an int (an address, taken as it is)."""
     if x is None:
         return None
+    t = _torch or _bind_torch()
+    if t is not None and type(x) is t.Tensor and x.dtype is _dtypes[dtype] and x.is_cuda and x.numel() >= count \
+            and x.is_contiguous():
+        return x.data_ptr()
     if isinstance(x, int):
         return x
     if hasattr(x, "data_ptr"):
@@ -161,6 +185,9 @@ def _count(m: int, n: int) -> int:
 
 def _stream(s) -> Optional[int]:
     if s is None:
+        t = _torch or _bind_torch()
+        if t is not None and _raw_stream is not None and t.cuda.is_initialized():
+            return _raw_stream(t.cuda.current_device())
         try:
             import torch
             if torch.cuda.is_available():
@@ -177,11 +204,15 @@ def _opts(opts: Optional[Opts]):
     return ctypes.byref(opts) if opts is not None else None
 
 
+_F64_PATHS = {"auto": "pcrp_solve_f64", "small": "pcrp_solve_f64_small", "split": "pcrp_solve_f64_split"}
+
+
 def solve_f64(a, b, c, d, e, y, m: int, n: int, layout: int = CONTIGUOUS,
               opts: Optional[Opts] = None, stream=None, path: str = "auto") -> None:
     """FP64 PCR-Penta solve in place on y (pcrp_solve_f64 / _small / _split)."""
-    fn = {"auto": "pcrp_solve_f64", "small": "pcrp_solve_f64_small", "split": "pcrp_solve_f64_split"}[path]
-    rc = getattr(lib(), fn)(*[_ptr(v, _count(m, n)) for v in (a, b, c, d, e, y)], m, n, layout,
+    fn = _F64_PATHS[path]
+    k = _count(m, n)
+    rc = getattr(lib(), fn)(_ptr(a, k), _ptr(b, k), _ptr(c, k), _ptr(d, k), _ptr(e, k), _ptr(y, k), m, n, layout,
                             _opts(opts), _stream(stream))
     _check(rc, fn)
 
