@@ -59,15 +59,18 @@ pcr_pass_kernel(const PcrPassArgs p)
     pcr_tile<CAP, false, kFew>(p, j, r, w, *reinterpret_cast<TileRows<CAP>*>(pcr_smem));
 }
 
-constexpr int kShortRows = 320;
+constexpr int kShortRows = 2048;          // rows of a short system
 
 template <int CAP, bool kFew>
 cudaError_t launch_tiles(const PcrPassArgs& p, int threads, int64_t blocks, cudaStream_t s)
 {
-    // per-device attribute; cheap, and legal while a stream is being captured
-    cudaError_t e = cudaFuncSetAttribute(pcr_pass_kernel<CAP, kFew>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sizeof(TileRows<CAP>));
-    if (e != cudaSuccess) return e;
+    // per-device attribute, for more than the default 48 KB; cheap, and legal
+    // while a stream is being captured
+    if (sizeof(TileRows<CAP>) > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(pcr_pass_kernel<CAP, kFew>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)sizeof(TileRows<CAP>));
+        if (e != cudaSuccess) return e;
+    }
     pcr_pass_kernel<CAP, kFew><<<(unsigned)blocks, threads, sizeof(TileRows<CAP>), s>>>(p);
     count_launch();
     return cudaGetLastError();
@@ -80,17 +83,18 @@ cudaError_t launch_cap(const PcrPassArgs& p, int threads, int64_t blocks, cudaSt
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    // The general rows for launches of at most two warps per SM sub-partition,
-    // where a row's latency counts and the FP64 pipe is not full (us, general /
-    // per-case rows: 8 systems of 100 rows 29 / 43, of 512 rows 71 / 81; 32
-    // systems of 4096 rows, six warps, 152 / 136), and for whole short
-    // pentadiagonal systems, most of whose rows are near an end in the late
-    // strides and would each load another case's code (4000 systems of 100
-    // rows 229 / 316, 2000 of 320 rows 388 / 397, of 384 rows 458 / 438).
-    // Tridiagonal batches never (their rows issue little FP64 work: 8 systems
-    // of 512 rows 71 / 50).
+    // One row case for all rows (zeros among the operands selected) for
+    // launches of at most two warps per SM sub-partition, where a row's latency
+    // counts and the FP64 pipe is not full (us, one case / per-case rows: 8
+    // systems of 512 rows 58 / 81; 32 systems of 4096 rows, six warps,
+    // 152 / 136), and for short pentadiagonal systems, many of whose rows are
+    // near an end in the late strides and would each load another case's code
+    // (4000 systems of 100 rows 157 / 316, 2000 of 512 464 / 511, 2000 of 1000
+    // 968 / 1135, 500 of 2000 581 / 609, 300 of 4000 737 / 708).  Tridiagonal
+    // batches never: their rows issue little FP64 work (8 systems of 512 rows
+    // 71 / 50).
     const bool few = blocks * (threads / 32) <= 8 * (int64_t)sms;
-    const bool shorts = p.G == 1 && p.final_step && p.TRmax <= kShortRows;
+    const bool shorts = p.n <= kShortRows;
     if ((few || shorts) && !p.tri) return launch_tiles<CAP, true>(p, threads, blocks, s);
     return launch_tiles<CAP, false>(p, threads, blocks, s);
 }

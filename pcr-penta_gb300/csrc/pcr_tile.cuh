@@ -328,6 +328,81 @@ __device__ __forceinline__ bool row_b_none(TileRows<CAP>& t, int k, int dl, bool
     return true;
 }
 
+// Rows near the ends of a (sub)system, where sides are missing and the
+// neighbouring rows hold structural zeros: any operand may be a zero, the
+// others are inside the window; integer quotients and products with the zeros
+// selected, sums on the FP64 pipe.
+struct Multiplier {
+    ieee::Factor f;
+    double x;
+    bool active;                        // nonzero: products by ieee::mul
+};
+__device__ __forceinline__ unsigned off_or_zero(double x) { return nz(x) ? ieee::off(x) : 0u; }
+__device__ __forceinline__ Multiplier multiplier(double num, double piv, uint32_t G, bool active, bool zero)
+{
+    Multiplier m;
+    m.x = ieee::div(num, piv, G);
+    m.active = active;
+    if (!active) m.x = zero ? szero(hiw(num) ^ hiw(piv)) : 0.0;
+    m.f = ieee::factor(m.x);
+    return m;
+}
+__device__ __forceinline__ double times(const Multiplier& m, double y)
+{
+    const double p = ieee::mul(m.f, y);
+    return m.active && nz(y) ? p : szero(hiw(m.x) ^ hiw(y));
+}
+
+template <int CAP>
+__device__ __forceinline__ bool row_a_zeros(TileRows<CAP>& t, int k, int dl, bool hasL, bool has2L, bool hasR,
+                                            bool has2R, double& cT)
+{
+    const int l = hasL ? k - dl : k, r = hasR ? k + dl : k;
+    const double am = neg(t.a[k]), em = neg(t.e[k]);
+    const double aL = t.a[l], bL = t.b[l], cL = t.c[l], dL = t.d[l], eL = t.e[l];
+    const double aR = t.a[r], bR = t.b[r], cR = t.c[r], dR = t.d[r], eR = t.e[r];
+    if (!ieee::fits(off_or_zero(am) | off_or_zero(em) | off_or_zero(aL) | off_or_zero(bL) | off_or_zero(cL) |
+                    off_or_zero(dL) | off_or_zero(eL) | off_or_zero(aR) | off_or_zero(bR) | off_or_zero(cR) |
+                    off_or_zero(dR) | off_or_zero(eR))) return false;
+    const bool piv1 = has2L && nz(bL), piv2 = has2R && nz(dR);
+    const Multiplier m1 = multiplier(am, bL, ieee::recip(bL), piv1 && nz(am), piv1);
+    const Multiplier m2 = multiplier(em, dR, ieee::recip(dR), piv2 && nz(em), piv2);
+    const double m0 = szero(~0u);                 // (a missing side adds -0, which changes nothing)
+    cT = add(add(hasL ? times(m1, dL) : m0, t.c[k]), hasR ? times(m2, bR) : m0);
+    t.Tc[k] = cT;
+    t.Tr[k] = ieee::recip(cT);
+    t.Tb[k] = hasL ? add(add(times(m1, cL), t.b[k]), hasR ? times(m2, aR) : m0) : 0.0;
+    t.Td[k] = hasR ? add(add(hasL ? times(m1, eL) : m0, t.d[k]), times(m2, cR)) : 0.0;
+    t.Ty[k] = add(add(hasL ? mul(m1.x, t.y[l]) : m0, t.y[k]), hasR ? mul(m2.x, t.y[r]) : m0);
+    t.Ta[k] = hasL ? times(m1, aL) : 0.0;
+    t.Te[k] = hasR ? times(m2, eR) : 0.0;
+    return true;
+}
+
+template <int CAP>
+__device__ __forceinline__ bool row_b_zeros(TileRows<CAP>& t, int k, int dl, bool hasL, bool hasR, double& f1, double& f2)
+{
+    const int l = hasL ? k - dl : k, r = hasR ? k + dl : k;
+    const double bi = t.b[k], di = t.d[k], cL = hasL ? t.Tc[l] : 1.0, cR = hasR ? t.Tc[r] : 1.0;
+    const double aL = hasL ? t.Ta[l] : 0.0, bL = hasL ? t.Tb[l] : 0.0, dL = hasL ? t.Td[l] : 0.0, eL = hasL ? t.Te[l] : 0.0;
+    const double aR = hasR ? t.Ta[r] : 0.0, bR = hasR ? t.Tb[r] : 0.0, dR = hasR ? t.Td[r] : 0.0, eR = hasR ? t.Te[r] : 0.0;
+    if (!ieee::fits(off_or_zero(bi) | off_or_zero(di) | ieee::off(cL) | ieee::off(cR) | off_or_zero(aL) | off_or_zero(bL) |
+                    off_or_zero(dL) | off_or_zero(eL) | off_or_zero(aR) | off_or_zero(bR) | off_or_zero(dR) |
+                    off_or_zero(eR))) return false;
+    const Multiplier m1 = multiplier(bi, cL, t.Tr[l], hasL && nz(bi), hasL);
+    const Multiplier m2 = multiplier(di, cR, t.Tr[r], hasR && nz(di), hasR);
+    // (a missing side's products are +0: its factors are)
+    const double ny = add(sub(hasL ? mul(m1.x, t.Ty[l]) : 0.0, t.y[k]), hasR ? mul(m2.x, t.Ty[r]) : 0.0);
+    const double nb = add(sub(times(m1, bL), t.a[k]), times(m2, aR));
+    const double nc = add(sub(times(m1, dL), t.c[k]), times(m2, bR));
+    const double nd = add(sub(times(m1, eL), t.e[k]), times(m2, dR));
+    t.y[k] = ny; t.b[k] = nb; t.c[k] = nc; t.d[k] = nd;
+    t.a[k] = times(m1, aL);
+    t.e[k] = times(m2, eR);
+    f1 = m1.x; f2 = m2.x;
+    return true;
+}
+
 // The general forms: every operation on the FP64 pipe but the quotients whose
 // operands are inside the integer quotient's guard.
 template <int CAP>
@@ -408,8 +483,8 @@ __device__ __forceinline__ double gload(const double* p) {
 
 // One CTA's work: window w of subsystem r of system j (whole subsystem when
 // p.final_step).  Every thread of the CTA must call it with the same (j, r, w).
-// kFew: the launch leaves most of the SM's warp slots empty; every row takes
-// the general form.
+// kFew: one case for all rows (row_a_zeros, row_b_zeros), then the general
+// form; else a case per kind of row (launch_cap chooses).
 template <int CAP, bool kL2Only = false, bool kFew = false>
 __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32_t r, uint32_t w, TileRows<CAP>& T)
 {
@@ -542,7 +617,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
             // structural zeros, take the general form at once
             double cT;
             bool done = false;
-            if (kFew) done = false;
+            if (kFew) done = row_a_zeros(T, k, dl, hasL, has2L, hasR, has2R, cT);
             else if (!left && !right) done = row_a_none(T, k, dl, hasL, has2L, hasR, has2R, cT);
             else if (has2L && has2R) {
                 if (left && right) done = row_a_both(T, k, dl, cT);
@@ -580,7 +655,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
             const bool left = hasL && nz(T.b[k]), right = hasR && nz(T.d[k]);
             double f1 = 0.0, f2 = 0.0;
             bool done = false;
-            if (kFew) done = false;
+            if (kFew) done = row_b_zeros(T, k, dl, hasL, hasR, f1, f2);
             else if (!left && !right) done = row_b_none(T, k, dl, hasL, hasR, f1, f2);
             else if (k - 3 * dl >= kfirst && k + 3 * dl <= klast) {
                 if (left && right) {
