@@ -109,6 +109,10 @@ cudaError_t launch_pcr_pass(const PcrPassArgs& p, int threads, cudaStream_t s)
     threads = (threads + 31) / 32 * 32;
     if (p.TRmax < threads) threads = (p.TRmax + 31) / 32 * 32;   // small (sub)systems: no idle warps
     while ((p.TRmax + threads - 1) / threads > kMaxRowsPerThread && threads < kMaxThreads) threads += 32;
+    // as many warps as the rows per thread need (376 rows: two rounds of 192
+    // threads, not of 256)
+    const int rounds = (p.TRmax + threads - 1) / threads;
+    threads = ((p.TRmax + rounds - 1) / rounds + 31) / 32 * 32;
     if (p.TRmax > pcr_max_smem_rows()) return cudaErrorInvalidValue;
     const int64_t blocks = p.m * p.G * p.nwin;
     if (blocks <= 0) return cudaSuccess;
@@ -117,6 +121,7 @@ cudaError_t launch_pcr_pass(const PcrPassArgs& p, int threads, cudaStream_t s)
     if (p.TRmax <= 64) return launch_cap<64>(p, threads, blocks, s);
     if (p.TRmax <= 128) return launch_cap<128>(p, threads, blocks, s);
     if (p.TRmax <= 256) return launch_cap<256>(p, threads, blocks, s);
+    if (p.TRmax <= 384) return launch_cap<384>(p, threads, blocks, s);
     if (p.TRmax <= 544) return launch_cap<544>(p, threads, blocks, s);
     if (p.TRmax <= 1024) return launch_cap<1024>(p, threads, blocks, s);
     return launch_cap<1920>(p, threads, blocks, s);
