@@ -391,11 +391,19 @@ mp_prep_kernel(MpArgs p)
 // that no other system's solve would read).
 template <bool RG>
 __global__ void __launch_bounds__(kMpThreads)
-mp_rhs_kernel(MpArgs p)
+mp_rhs_kernel(MpArgs p, cudaGraphConditionalHandle windows, cudaGraphConditionalHandle full, bool gate)
 {
     pdl_wait();
     pdl_release();                                // one wave of persistent CTAs: the successor may queue now
-    if (__ldg(p.nfail) == 0) return;
+    const bool left = __ldg(p.nfail) != 0;
+    if (gate && blockIdx.x == 0 && threadIdx.x == 0) {
+        // no system left: the sweeps go on with sweep 1 (sweep 0 takes no
+        // decision when more than one may run, and they are two at least)
+        *p.ctr = left ? 0 : 1;
+        cudaGraphSetConditional(windows, left ? 0u : 1u);
+        cudaGraphSetConditional(full, left ? 1u : 0u);
+    }
+    if (!left) return;
     const int64_t nb = (p.n + 1) / 2;
     for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < p.m * nb; q += (int64_t)gridDim.x * blockDim.x) {
         const int64_t j = q / nb;
@@ -958,9 +966,13 @@ mp_decide_kernel(MpArgs p)
     bool finish = false;
     if (j < p.m && p.fin[j] == 0) {
         const UpDecision D = up_decide(p, j);
-        if (D.last) {
-            p.est[j] = D.est;
-            p.status[j] = D.done ? 1 : 2;         // 2: stopped at max_sweeps
+        // A sweep without general passes takes the blocks of sweep 0, which
+        // decoupled then, through the same reduction; should a window differ
+        // all the same, its system stops here and is not called converged.
+        const bool lost = p.windows_only && __ldg(p.fail + j) != 0;
+        if (D.last || lost) {
+            p.est[j] = lost ? __uint_as_float(0x7F800000u) : D.est;
+            p.status[j] = D.done && !lost ? 1 : 2;    // 2: stopped at max_sweeps
             p.fin[j] = s + 1;
             finish = true;
         }
@@ -1413,12 +1425,13 @@ cudaError_t launch_mp_prep(const MpArgs& p, cudaStream_t s)
     return e;
 }
 
-cudaError_t launch_mp_rhs(const MpArgs& p, cudaStream_t s)
+cudaError_t launch_mp_rhs(const MpArgs& p, cudaGraphConditionalHandle windows, cudaGraphConditionalHandle full, bool gate,
+                          cudaStream_t s)
 {
     auto kern = p.rg ? mp_rhs_kernel<true> : mp_rhs_kernel<false>;
     const int64_t need = (p.m * ((p.n + 1) / 2) + kMpThreads - 1) / kMpThreads;
     const int64_t blocks = std::min<int64_t>(need, mp_grid_cap((const void*)kern, kMpThreads, 0));
-    const cudaError_t e = launch_dependent(kern, (unsigned)blocks, kMpThreads, 0, s, p);
+    const cudaError_t e = launch_dependent(kern, (unsigned)blocks, kMpThreads, 0, s, p, windows, full, gate);
     count_launch();
     return e;
 }

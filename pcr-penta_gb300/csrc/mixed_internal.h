@@ -50,6 +50,8 @@ struct MpArgs {
     int vec;                            // 1: all six caller arrays are 16-byte aligned (paired loads allowed)
     int first_fused;                    // sweep 0 ran as mp_first_kernel (the refinement of sweep 0 only
                                         // takes the systems it left to the general passes)
+    bool windows_only;                  // this sweep runs without general passes: every system decoupled in
+                                        // the windows of sweep 0
     int cr_mode;                        // a cyclic-reduction pass updates x of the systems it solves
     float tol;
 };
@@ -151,7 +153,11 @@ pcrp_status mixed_enqueue(const double* a, const double* b, const double* c, con
 cudaError_t launch_mp_init(const MpArgs& p, cudaStream_t s);
 cudaError_t launch_mp_first(const MpArgs& p, const MpWindows& g, cudaStream_t s);
 cudaError_t launch_mp_prep(const MpArgs& p, cudaStream_t s);
-cudaError_t launch_mp_rhs(const MpArgs& p, cudaStream_t s);
+// R[0] of the systems the windows of sweep 0 left coupled; with `gate`, also
+// opens the while node of the sweeps without general passes (windows) or, if
+// any system is left, the one with them (full).
+cudaError_t launch_mp_rhs(const MpArgs& p, cudaGraphConditionalHandle windows, cudaGraphConditionalHandle full, bool gate,
+                          cudaStream_t s);
 cudaError_t launch_mp_pass(const MpPassArgs& p, cudaStream_t s);
 cudaError_t launch_mp_small(const MpArgs& p, cudaStream_t s);   // whole systems, every sweep in one CTA
 cudaError_t launch_mp_try(const MpPassArgs& p, cudaStream_t s);
