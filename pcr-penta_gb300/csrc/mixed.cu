@@ -155,7 +155,7 @@ __device__ __forceinline__ double2 ldg2(const double* q, Keep keep, uint64_t pol
 // RG: the batch is ragged (p.rg non-null); the uniform kernels are compiled
 // without the ragged addressing.
 template <bool RG>
-__device__ __forceinline__ PairRow load_pair(const MpArgs& p, int64_t j, int64_t i0, Keep keep = Keep::normal)
+__device__ __forceinline__ PairRow load_pair(const MpArgs& p, int64_t j, int64_t i0, Keep keep, bool has_a, bool has_e)
 {
     PairRow P;
     int64_t n = p.n, rs = p.rs, base = j * p.ss;
@@ -172,20 +172,20 @@ __device__ __forceinline__ PairRow load_pair(const MpArgs& p, int64_t j, int64_t
     if (p.vec && rs == 1 && ((g0 & 1) == 0) && i0 + 1 < n) {
         const uint64_t pol = keep == Keep::last ? tma::policy_evict_last()
                              : keep == Keep::first ? tma::policy_evict_first() : 0;
-        const double2 a = p.a ? ldg2(p.a + g0, keep, pol) : z;
+        const double2 a = has_a ? ldg2(p.a + g0, keep, pol) : z;
         const double2 b = ldg2(p.b + g0, keep, pol);
         const double2 c = ldg2(p.c + g0, keep, pol);
         const double2 d = ldg2(p.d + g0, keep, pol);
-        const double2 e = p.e ? ldg2(p.e + g0, keep, pol) : z;
+        const double2 e = has_e ? ldg2(p.e + g0, keep, pol) : z;
         const double2 y = ldg2(p.y + g0, keep, pol);
         P = {a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y, e.x, e.y, y.x, y.y};
     } else {
-        P.a0 = p.a ? p.a[g0] : 0.0; P.b0 = p.b[g0]; P.c0 = p.c[g0]; P.d0 = p.d[g0];
-        P.e0 = p.e ? p.e[g0] : 0.0; P.y0 = p.y[g0];
+        P.a0 = has_a ? p.a[g0] : 0.0; P.b0 = p.b[g0]; P.c0 = p.c[g0]; P.d0 = p.d[g0];
+        P.e0 = has_e ? p.e[g0] : 0.0; P.y0 = p.y[g0];
         if (i0 + 1 < n) {
             const int64_t g1 = g0 + rs;
-            P.a1 = p.a ? p.a[g1] : 0.0; P.b1 = p.b[g1]; P.c1 = p.c[g1]; P.d1 = p.d[g1];
-            P.e1 = p.e ? p.e[g1] : 0.0; P.y1 = p.y[g1];
+            P.a1 = has_a ? p.a[g1] : 0.0; P.b1 = p.b[g1]; P.c1 = p.c[g1]; P.d1 = p.d[g1];
+            P.e1 = has_e ? p.e[g1] : 0.0; P.y1 = p.y[g1];
         } else {
             P.a1 = 0.0; P.b1 = 0.0; P.c1 = 1.0; P.d1 = 0.0; P.e1 = 0.0; P.y1 = 0.0;
         }
@@ -196,6 +196,12 @@ __device__ __forceinline__ PairRow load_pair(const MpArgs& p, int64_t j, int64_t
         if (i0 + 3 >= n) P.e1 = 0.0;
     }
     return P;
+}
+
+template <bool RG>
+__device__ __forceinline__ PairRow load_pair(const MpArgs& p, int64_t j, int64_t i0, Keep keep = Keep::normal)
+{
+    return load_pair<RG>(p, j, i0, keep, p.a != nullptr, p.e != nullptr);
 }
 
 // The FP32 row-scaled diagonal block and couplings of block row k (rows
@@ -469,8 +475,9 @@ __device__ __forceinline__ void mp_pass_item(const MpPassArgs& p, int64_t j, int
             const int k = tid + q * bd;
             if (k >= klo && k < khi) {
                 const int km = max(k - dl, 0), kp = min(k + dl, TR - 1);
+                M2 Mi;
                 reduce_row(Lr[q], Ur[q], Yr[q], m2(sL[km]), m2(sU[km]), sY[km], m2(sL[kp]), m2(sU[kp]), sY[kp],
-                           Lr[q], Ur[q], Yr[q]);
+                           Lr[q], Ur[q], Yr[q], Mi);
             }
         }
         __syncthreads();                                   // every read of this stride is done
@@ -986,15 +993,22 @@ mp_decide_kernel(MpArgs p)
 // one CTA): all sweeps of a system run inside its CTA, so nothing waits for
 // the rest of the batch between sweeps and the whole solve is one launch.
 // Per system:
-//  1. FP64 bands and y -> row-scaled, normalised FP32 blocks (prep_row): in
-//     shared memory for the first solve, and in S0 for the later ones;
-//  2. per sweep: cyclic reduction to the top and back substitution (dx_s),
-//     x_s = x_{s-1} + dx_s in FP64 (X0, contiguous), the maxima of |dx_s| and
-//     |x_s| over the CTA, the stopping rule; if another sweep follows,
-//     r_s = y - A x_s in FP64, row-scaled and normalised into the tile's rhs,
-//     and the level-0 blocks back from S0 (the reduction overwrote them);
+//  1. FP64 bands and y -> row-scaled, normalised FP32 blocks in shared memory;
+//  2. per sweep: cyclic reduction to the top (sweep 0, which keeps the factors
+//     of its steps; later sweeps replay them on their rhs) and back
+//     substitution (dx_s), x_s = x_{s-1} + dx_s in FP64, the maxima of |dx_s|
+//     and |x_s| over the CTA, the stopping rule; if another sweep follows,
+//     r_s = y - A x_s in FP64, row-scaled and normalised into the tile's rhs;
 //  3. x -> the output, status, sweeps and estimate.
 // y keeps the rhs until the final copy, so no copy of it is needed.
+//
+// Bound by latency: two CTAs of 512 threads fill an SM's registers at n=4096
+// (FP64 pipe 40 %, ALU 47 %, issue 51 %; L2 and barrier waits).  Measured:
+// reducing the matrix again in every sweep, from a copy of the blocks in S0,
+// m=4096 n=4096 ADI 931 us, m=2048 n=2000 154; the factors kept instead, and
+// zero outer bands skipped, 887 and 133 (same bits).  Keeping the diagonal
+// inverses as well costs more L2 traffic than the instructions it saves (933
+// and 146); the iterate as 16-byte pairs changes nothing.
 __device__ __forceinline__ void block_max(unsigned& dmb, unsigned long long& xb, unsigned* red_d,
                                           unsigned long long* red_x)
 {
@@ -1021,6 +1035,7 @@ mp_small_kernel(MpArgs p)
     extern __shared__ float4 fsm[];
     __shared__ unsigned red_d[kMpSmallThreadsMax / 32];
     __shared__ unsigned long long red_x[kMpSmallThreadsMax / 32];
+    __shared__ float4 s_last[3 * kCrLevels];
     pdl_wait();
     pdl_release();
     const int64_t n = p.n, nb = (n + 1) / 2;
@@ -1029,22 +1044,33 @@ mp_small_kernel(MpArgs p)
     float4* sU = fsm + TRs;
     float2* sY = reinterpret_cast<float2*>(fsm + 2 * TRs);
     const int tid = threadIdx.x, bd = blockDim.x;
+    // this CTA's part of the workspace, the same for every system it solves
+    // (what it writes stays in L2): the iterate, and the factors in the memory
+    // of S0 and R[], which follow each other (48 bytes per block row)
+    double* __restrict__ X = p.X0 + blockIdx.x * n;
+    const CrFactors F{p.S0 + 3 * nb * blockIdx.x, s_last};
     for (int64_t j = blockIdx.x; j < p.m; j += gridDim.x) {
-        double* __restrict__ X = p.X0 + j * n;
+        unsigned any_a = 0u, any_e = 0u;          // bits of the outer bands inside the system
         for (int k = tid; k < TR; k += bd) {
-            const PrepRow r = prep_row<RG>(p, j, k);
-            const int64_t q = j * nb + k;
-            p.S0[2 * q] = f4(r.L);
-            p.S0[2 * q + 1] = f4(r.U);
+            const int64_t i0 = 2 * (int64_t)k;
+            const PairRow P = load_pair<RG>(p, j, i0);
+            const PrepRow r = prep_of(i0 >= 2 && i0 + 3 < n ? block_inner(P, i0, n) : block_of(P, i0, n));
+            if (i0 >= 2) any_a |= magbits(P.a0) | magbits(P.a1);
+            if (i0 + 2 < n) any_e |= magbits(P.e0);
+            if (i0 + 3 < n) any_e |= magbits(P.e1);
             const int sk = swz(k);
             sL[sk] = f4(r.L); sU[sk] = f4(r.U); sY[sk] = r.Y;
         }
-        __syncthreads();
+        // an outer band that is zero in the whole system (one-sided operators)
+        // is treated like a missing one: neither read nor multiplied again
+        const bool has_a = __syncthreads_or(any_a != 0u), has_e = __syncthreads_or(any_e != 0u);
         float ndp = 0.0f, nxp = 0.0f;
         UpDecision D{false, false, 0.0f};
-        int s = 0;
+        int s = 0, top = 0;
         for (;; s++) {
-            const int top = cr_reduce(sL, sU, sY, TR, 31, 0, TR);   // a whole system: never -1
+            // (a whole system: never -1)
+            if (s == 0) top = cr_reduce<true>(sL, sU, sY, TR, 31, 0, TR, F);
+            else cr_replay(F, sY, TR, top);
             cr_substitute(sL, sU, sY, TR, top);
             unsigned dmb = 0u;
             unsigned long long xb = 0ull;
@@ -1070,33 +1096,29 @@ mp_small_kernel(MpArgs p)
             if (D.last) break;
             ndp = nd; nxp = nx;
             for (int k = tid; k < TR; k += bd) {
-                const int64_t i0 = 2 * (int64_t)k, q = j * nb + k;
-                const PairRow P = load_pair<RG>(p, j, i0);
+                const int64_t i0 = 2 * (int64_t)k;
+                const PairRow P = load_pair<RG>(p, j, i0, Keep::normal, has_a, has_e);
                 const double xm2 = i0 >= 2 ? X[i0 - 2] : 0.0, xm1 = i0 >= 1 ? X[i0 - 1] : 0.0, x0 = X[i0];
                 const double x1 = i0 + 1 < n ? X[i0 + 1] : 0.0, x2 = i0 + 2 < n ? X[i0 + 2] : 0.0;
                 const double x3 = i0 + 3 < n ? X[i0 + 3] : 0.0;
                 double r0 = fma(-P.c0, x0, P.y0);
-                if (p.a && i0 >= 2) r0 = fma(-P.a0, xm2, r0);
+                if (has_a && i0 >= 2) r0 = fma(-P.a0, xm2, r0);
                 if (i0 >= 1) r0 = fma(-P.b0, xm1, r0);
                 if (i0 + 1 < n) r0 = fma(-P.d0, x1, r0);
-                if (p.e && i0 + 2 < n) r0 = fma(-P.e0, x2, r0);
+                if (has_e && i0 + 2 < n) r0 = fma(-P.e0, x2, r0);
                 const float rf0 = d2f_scaled(r0, d_exponent(P.c0));
                 float rf1 = 0.0f;                 // the identity row of an odd system's last block row
                 if (i0 + 1 < n) {
                     double r1 = fma(-P.c1, x1, P.y1);
-                    if (p.a && i0 >= 1) r1 = fma(-P.a1, xm1, r1);
+                    if (has_a && i0 >= 1) r1 = fma(-P.a1, xm1, r1);
                     r1 = fma(-P.b1, x0, r1);
                     if (i0 + 2 < n) r1 = fma(-P.d1, x2, r1);
-                    if (p.e && i0 + 3 < n) r1 = fma(-P.e1, x3, r1);
+                    if (has_e && i0 + 3 < n) r1 = fma(-P.e1, x3, r1);
                     rf1 = d2f_scaled(r1, d_exponent(P.c1));
                 }
                 const M2 Mi = diag_inverse(P, i0, n);
-                const int sk = swz(k);
-                sY[sk] = make_float2(fmaf(Mi.m0, rf0, Mi.m1 * rf1), fmaf(Mi.m2, rf0, Mi.m3 * rf1));
-                sL[sk] = p.S0[2 * q];
-                sU[sk] = p.S0[2 * q + 1];
+                sY[swz(k)] = make_float2(fmaf(Mi.m0, rf0, Mi.m1 * rf1), fmaf(Mi.m2, rf0, Mi.m3 * rf1));
             }
-            __syncthreads();
         }
         for (int64_t i = tid; i < n; i += bd) x_write(p.xout, p.oss, p.ors, RG ? p.rg : nullptr, j, i, X[i]);
         if (tid == 0) { p.fin[j] = s + 1; p.status[j] = D.done ? 1 : 2; p.est[j] = D.est; }

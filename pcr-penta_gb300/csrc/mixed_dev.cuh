@@ -132,6 +132,11 @@ __device__ __forceinline__ unsigned long long absbits(double x) {
     return r;
 }
 
+// Bits of x other than the sign, folded into one word: zero exactly for +-0.
+__device__ __forceinline__ unsigned magbits(double x) {
+    return ((unsigned)__double2hiint(x) << 1) | (unsigned)__double2loint(x);
+}
+
 // ---------------------------------------------------------------------------
 // 2x2 helpers (row-major m[0] m[1] / m[2] m[3])
 // ---------------------------------------------------------------------------
@@ -154,28 +159,34 @@ __device__ __forceinline__ float amaxm(const M2& a) {
 __device__ __forceinline__ M2 m2(const float4& v) { return {v.x, v.y, v.z, v.w}; }
 __device__ __forceinline__ float4 f4(const M2& a) { return make_float4(a.m0, a.m1, a.m2, a.m3); }
 
+// The rhs of a block reduction step (reduce_row): Y' = D'^-1 (Y_k - L_k Y_m - U_k Y_p).
+__device__ __forceinline__ float2 reduce_rhs(const M2& Lk, const M2& Uk, float2 Yk, float2 ym, float2 yp, const M2& Mi)
+{
+    const float y0 = fmaf(-Uk.m1, yp.y, fmaf(-Uk.m0, yp.x, fmaf(-Lk.m1, ym.y, fmaf(-Lk.m0, ym.x, Yk.x))));
+    const float y1 = fmaf(-Uk.m3, yp.y, fmaf(-Uk.m2, yp.x, fmaf(-Lk.m3, ym.y, fmaf(-Lk.m2, ym.x, Yk.y))));
+    return make_float2(fmaf(Mi.m0, y0, Mi.m1 * y1), fmaf(Mi.m2, y0, Mi.m3 * y1));
+}
+
 // One block reduction step of a normalised row k (D = I) with its neighbours
 // m = k-d and p = k+d (PCR stride and cyclic-reduction level alike):
 //     D' = I - L_k U_m - U_k L_p,  L' = -D'^-1 L_k L_m,  U' = -D'^-1 U_k U_p,
-//     Y' = D'^-1 (Y_k - L_k Y_m - U_k Y_p).
+//     Y' = D'^-1 (Y_k - L_k Y_m - U_k Y_p);   Mi = D'^-1.
 __device__ __forceinline__ void reduce_row(const M2& Lk, const M2& Uk, float2 Yk,
                                            const M2& Lm, const M2& Um, float2 ym,
                                            const M2& Lp, const M2& Up, float2 yp,
-                                           M2& Lo, M2& Uo, float2& Yo)
+                                           M2& Lo, M2& Uo, float2& Yo, M2& Mi)
 {
     M2 Dn;
     Dn.m0 = fmaf(-Uk.m1, Lp.m2, fmaf(-Uk.m0, Lp.m0, fmaf(-Lk.m1, Um.m2, fmaf(-Lk.m0, Um.m0, 1.0f))));
     Dn.m1 = fmaf(-Uk.m1, Lp.m3, fmaf(-Uk.m0, Lp.m1, fmaf(-Lk.m1, Um.m3, -Lk.m0 * Um.m1)));
     Dn.m2 = fmaf(-Uk.m3, Lp.m2, fmaf(-Uk.m2, Lp.m0, fmaf(-Lk.m3, Um.m2, -Lk.m2 * Um.m0)));
     Dn.m3 = fmaf(-Uk.m3, Lp.m3, fmaf(-Uk.m2, Lp.m1, fmaf(-Lk.m3, Um.m3, fmaf(-Lk.m2, Um.m1, 1.0f))));
-    const float y0 = fmaf(-Uk.m1, yp.y, fmaf(-Uk.m0, yp.x, fmaf(-Lk.m1, ym.y, fmaf(-Lk.m0, ym.x, Yk.x))));
-    const float y1 = fmaf(-Uk.m3, yp.y, fmaf(-Uk.m2, yp.x, fmaf(-Lk.m3, ym.y, fmaf(-Lk.m2, ym.x, Yk.y))));
     const M2 LL = mmul(Lk, Lm), UU = mmul(Uk, Up);
-    const M2 Mi = minv(Dn);
+    Mi = minv(Dn);
+    Yo = reduce_rhs(Lk, Uk, Yk, ym, yp, Mi);      // (the results may be the operands of row k)
     const M2 Mn = {-Mi.m0, -Mi.m1, -Mi.m2, -Mi.m3};
     Lo = mmul(Mn, LL);
     Uo = mmul(Mn, UU);
-    Yo = make_float2(fmaf(Mi.m0, y0, Mi.m1 * y1), fmaf(Mi.m2, y0, Mi.m3 * y1));
 }
 
 // Shared-memory position of row k of a cyclic-reduction tile: an XOR swizzle
@@ -183,6 +194,15 @@ __device__ __forceinline__ void reduce_row(const M2& Lk, const M2& Uk, float2 Yk
 // cyclic reduction hit distinct banks (16-byte slots) for 8 consecutive
 // lanes.  The arrays are allocated for whole groups of 8 rows (mp_pass_rows).
 __device__ __forceinline__ int swz(int k) { return k ^ (((k >> 3) ^ (k >> 6) ^ (k >> 9)) & 7); }
+
+// What the rhs of the reduction steps of a tile depends on, kept by one
+// reduction for later right-hand sides: per survivor L_k, U_k and D'^-1, as
+// three arrays per level.  A survivor with a right neighbour is counted by it
+// (each row but row 0 is one, at one level: TR - 1 entries of three in all,
+// in global memory); the last survivor of a level may have none and has its
+// place in shared memory.
+constexpr int kCrLevels = 12;            // levels of a tile of at most 4096 rows
+struct CrFactors { float4 *g, *last; };  // [3 (TR-1)], [3 kCrLevels]
 
 // Forward block cyclic reduction of the TR rows held (swizzled) in shared
 // memory: level l turns the rows k = 0 mod 2^(l+1) into the reduced system
@@ -194,28 +214,74 @@ __device__ __forceinline__ int swz(int k) { return k ^ (((k >> 3) ^ (k >> 6) ^ (
 // reduced rows that rows [clo, chi) depend on are decoupled (|L|,|U| <
 // kTrunc, truncated reduction) and returns the number of levels; returns -1
 // if they are still coupled after kmax levels.  A barrier must separate the
-// loads from the call.
-__device__ __forceinline__ int cr_reduce(float4* sL, float4* sU, float2* sY, int TR, int kmax, int clo, int chi)
+// loads from the call.  With kKeep, what the rhs of every step depends on goes
+// to F (cr_replay).
+template <bool kKeep = false>
+__device__ __forceinline__ int cr_reduce(float4* sL, float4* sU, float2* sY, int TR, int kmax, int clo, int chi,
+                                         CrFactors F = {})
 {
     const int tid = threadIdx.x, bd = blockDim.x;
+    int base = 0;
     for (int l = 0; l < kmax && (1 << l) < TR; l++) {
         const int d = 1 << l, d2 = 2 * d;
         const int lo = clo - d2 + 1, hi = chi + d2 - 1;
         bool coupled = false;
         for (int k = tid * d2; k < TR; k += bd * d2) {
             const int sk = swz(k), sm = swz(max(k - d, 0)), sp = swz(min(k + d, TR - 1));
-            M2 Lo, Uo;
+            M2 Lo, Uo, Mi;
             float2 Yo;
-            reduce_row(m2(sL[sk]), m2(sU[sk]), sY[sk], m2(sL[sm]), m2(sU[sm]), sY[sm], m2(sL[sp]), m2(sU[sp]), sY[sp],
-                       Lo, Uo, Yo);
+            const M2 Lk = m2(sL[sk]), Uk = m2(sU[sk]);
+            reduce_row(Lk, Uk, sY[sk], m2(sL[sm]), m2(sU[sm]), sY[sm], m2(sL[sp]), m2(sU[sp]), sY[sp], Lo, Uo, Yo, Mi);
+            if (kKeep) {
+                const int i = k >> (l + 1);
+                float4* const g = k + d < TR ? F.g + 3 * base + i : F.last + l;
+                const int step = k + d < TR ? (TR - d + d2 - 1) >> (l + 1) : kCrLevels;
+                g[0] = f4(Lk); g[step] = f4(Uk); g[2 * step] = f4(Mi);
+            }
             sL[sk] = f4(Lo); sU[sk] = f4(Uo); sY[sk] = Yo;
             if (k >= lo && k < hi) coupled |= fmaxf(amaxm(Lo), amaxm(Uo)) >= kTrunc;
         }
+        base += (TR - d + d2 - 1) >> (l + 1);
         // the barrier reduces the test: (nan entries do not count; a nan
         // solution is reported by the refinement)
         if (!__syncthreads_or(coupled)) return l + 1;
     }
     return TR <= 1 ? 0 : -1;
+}
+
+// The reduction of another rhs (in sY) by the steps that cr_reduce<true> kept:
+// the same operations on the rhs, so the same bits as reducing the matrix
+// again, at 12 of ~70 FMAs and 24 of 120 bytes of shared memory per step.
+// A level's factors do not depend on the level before: each thread's first
+// ones are on their way during the barrier.
+__device__ __forceinline__ void cr_replay(const CrFactors& F, float2* sY, int TR, int top)
+{
+    const int tid = threadIdx.x, bd = blockDim.x;
+    int base = 0, count = TR / 2;                 // survivors of a level with a right neighbour
+    const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 fL = z, fU = z, fM = z;
+    if (tid < count) { fL = F.g[tid]; fU = F.g[count + tid]; fM = F.g[2 * count + tid]; }
+    __syncthreads();                              // the rhs is complete
+    for (int l = 0; l < top; l++) {
+        const int d = 1 << l, d2 = 2 * d;
+        for (int i = tid; i * d2 < TR; i += bd) {
+            const int k = i * d2;
+            if (i != tid || i >= count) {
+                const float4* const g = i < count ? F.g + 3 * base + i : F.last + l;
+                const int step = i < count ? count : kCrLevels;
+                fL = g[0]; fU = g[step]; fM = g[2 * step];
+            }
+            const int sk = swz(k);
+            sY[sk] = reduce_rhs(m2(fL), m2(fU), sY[sk], sY[swz(max(k - d, 0))], sY[swz(min(k + d, TR - 1))], m2(fM));
+        }
+        base += count;
+        count = (TR - d2 + 2 * d2 - 1) >> (l + 2);
+        if (l + 1 < top && tid < count) {
+            const float4* const g = F.g + 3 * base + tid;
+            fL = g[0]; fU = g[count]; fM = g[2 * count];
+        }
+        __syncthreads();
+    }
 }
 
 // Back substitution after cr_reduce: the rows left at level `top` hold
