@@ -539,7 +539,7 @@ __device__ __forceinline__ void cr_load(const MpPassArgs& p, int64_t j, int64_t 
     for (int k = threadIdx.x; k < TR; k += blockDim.x) {
         const int64_t gi = g0 + (t0 + k) * p.G;
         const int s = swz(k);
-        sL[s] = p.srcLU[2 * gi]; sU[s] = p.srcLU[2 * gi + 1]; sY[s] = p.srcY[gi];
+        sL[s] = p.srcLU[2 * gi]; sU[s] = p.srcLU[2 * gi + 1]; sY[swzy(k)] = p.srcY[gi];
     }
     __syncthreads();
 }
@@ -552,7 +552,7 @@ __device__ __forceinline__ void cr_store(const MpPassArgs& p, int64_t j, int64_t
     float xmx = 0.0f;
     for (int k = klo + threadIdx.x; k < khi; k += blockDim.x) {
         const int64_t i0 = 2 * (r + (t0 + k) * p.G);      // first row of the block row
-        const float2 xv = sY[swz(k)];
+        const float2 xv = sY[swzy(k)];
         p.dx[j * p.n + i0] = xv.x;
         xmx = fmaxf(xmx, fabsf(xv.x));
         if (i0 + 1 < p.n) { p.dx[j * p.n + i0 + 1] = xv.y; xmx = fmaxf(xmx, fabsf(xv.y)); }
@@ -654,7 +654,7 @@ __device__ __forceinline__ void try_solve(const MpPassArgs& p, const TryTile& t,
     for (int u = 0; u < kMpTryRows / kMpTryThreads; u++) {
         const int k = klo + (int)threadIdx.x + u * kMpTryThreads;
         if (k < done) {
-            const float2 d = sY[swz(k)];
+            const float2 d = sY[swzy(k)];
             const double2 x = make_double2(__dadd_rn(f2d(x0[u].x), f2d(d.x)), __dadd_rn(f2d(x0[u].y), f2d(d.y)));
             reinterpret_cast<double2*>(xd)[k] = x;
             dmax = fmaxf(dmax, fmaxf(fabsf(d.x), fabsf(d.y)));
@@ -663,7 +663,7 @@ __device__ __forceinline__ void try_solve(const MpPassArgs& p, const TryTile& t,
     }
     for (int k = done + (int)threadIdx.x; k < khi; k += blockDim.x) {
         const int64_t i0 = 2 * (t.t0 + k);
-        const float2 v = sY[swz(k)];
+        const float2 v = sY[swzy(k)];
         x_update(xv, p.n, t.j, i0, v.x, dmax, xbits);
         if (i0 + 1 < p.n) x_update(xv, p.n, t.j, i0 + 1, v.y, dmax, xbits);
     }
@@ -725,7 +725,7 @@ __device__ __forceinline__ void first_prep(const MpArgs& p, const PairRun& run, 
         const PairRow P = load_run(run, k, Keep::last, pol);
         const PrepRow r = prep_of(block_inner(P, 2 * (t0 + k), p.n));
         const int sk = swz(k);
-        sL[sk] = f4(r.L); sU[sk] = f4(r.U); sY[sk] = r.Y;
+        sL[sk] = f4(r.L); sU[sk] = f4(r.U); sY[swzy(k)] = r.Y;
         if (k >= klo && k < khi) {
             S0[2 * k] = f4(r.L);
             S0[2 * k + 1] = f4(r.U);
@@ -766,7 +766,7 @@ __device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, 
         const int64_t kb = t0 + k;
         const PrepRow r = prep_row<RG>(p, j, kb, Keep::last);
         const int sk = swz(k);
-        sL[sk] = f4(r.L); sU[sk] = f4(r.U); sY[sk] = r.Y;
+        sL[sk] = f4(r.L); sU[sk] = f4(r.U); sY[swzy(k)] = r.Y;
         if (kb >= wlo && kb < whi) {
             prep_store(p, j * nb + kb, r);
             store_rhs_pair(p, j, 2 * kb, r.y);
@@ -790,7 +790,7 @@ __device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, 
     float dmax = 0.0f;
     bool nan = false;
     for (int k = xlo + tid; k < xhi; k += bd) {
-        const float2 v = sY[swz(k)];
+        const float2 v = sY[swzy(k)];
         sX[k] = make_double2(f2d(v.x), f2d(v.y));
         if (k >= klo && k < khi) {
             // x_0 = dx_0: one maximum for both norms
@@ -1059,7 +1059,7 @@ mp_small_kernel(MpArgs p)
             if (i0 + 2 < n) any_e |= magbits(P.e0);
             if (i0 + 3 < n) any_e |= magbits(P.e1);
             const int sk = swz(k);
-            sL[sk] = f4(r.L); sU[sk] = f4(r.U); sY[sk] = r.Y;
+            sL[sk] = f4(r.L); sU[sk] = f4(r.U); sY[swzy(k)] = r.Y;
         }
         // an outer band that is zero in the whole system (one-sided operators)
         // is treated like a missing one: neither read nor multiplied again
@@ -1075,7 +1075,7 @@ mp_small_kernel(MpArgs p)
             unsigned dmb = 0u;
             unsigned long long xb = 0ull;
             for (int k = tid; k < TR; k += bd) {
-                const float2 v = sY[swz(k)];
+                const float2 v = sY[swzy(k)];
                 const int64_t i0 = 2 * (int64_t)k;
                 const double x0 = s ? __dadd_rn(X[i0], f2d(v.x)) : f2d(v.x);
                 X[i0] = x0;
@@ -1117,7 +1117,7 @@ mp_small_kernel(MpArgs p)
                     rf1 = d2f_scaled(r1, d_exponent(P.c1));
                 }
                 const M2 Mi = diag_inverse(P, i0, n);
-                sY[swz(k)] = make_float2(fmaf(Mi.m0, rf0, Mi.m1 * rf1), fmaf(Mi.m2, rf0, Mi.m3 * rf1));
+                sY[swzy(k)] = make_float2(fmaf(Mi.m0, rf0, Mi.m1 * rf1), fmaf(Mi.m2, rf0, Mi.m3 * rf1));
             }
         }
         for (int64_t i = tid; i < n; i += bd) x_write(p.xout, p.oss, p.ors, RG ? p.rg : nullptr, j, i, X[i]);

@@ -15,9 +15,9 @@ namespace {
 
 constexpr float kTrunc = 1e-10f;
 
-// rows allocated per shared-memory array of the pass kernel (whole groups of
-// 8, the span of the swizzle of the whole-subsystem pass)
-__host__ __device__ __forceinline__ int mp_pass_rows(int rows) { return (rows + 7) & ~7; }
+// rows allocated per shared-memory array of a tile (whole groups of 16, the
+// span of the swizzles of cyclic reduction)
+__host__ __device__ __forceinline__ int mp_pass_rows(int rows) { return (rows + 15) & ~15; }
 
 // CTAs of one wave of a kernel (the pass kernel strides over its items with
 // one wave, so that sweeps of mostly finished systems stay cheap)
@@ -189,11 +189,19 @@ __device__ __forceinline__ void reduce_row(const M2& Lk, const M2& Uk, float2 Yk
     Uo = mmul(Mn, UU);
 }
 
-// Shared-memory position of row k of a cyclic-reduction tile: an XOR swizzle
-// inside each aligned group of 8 rows, so that the power-of-two strides of
-// cyclic reduction hit distinct banks (16-byte slots) for 8 consecutive
-// lanes.  The arrays are allocated for whole groups of 8 rows (mp_pass_rows).
-__device__ __forceinline__ int swz(int k) { return k ^ (((k >> 3) ^ (k >> 6) ^ (k >> 9)) & 7); }
+// Shared-memory positions of row k of a cyclic-reduction tile, in the float4
+// arrays (swz: L and U) and in the float2 array (swzy: Y): XOR swizzles inside
+// each aligned group of 8 (16) rows, with which the power-of-two strides of the
+// first levels, which hold most rows, hit distinct banks for the 8 (16) lanes
+// that one wavefront serves.  Two operations each, as these kernels are short
+// of integer instructions: against one swizzle of five operations for all
+// arrays and levels (conflict-free for L and U at every level, two-way
+// conflicts for Y: 27 % of mp_try_kernel's wavefronts) m=64 n=2^20 2133 ->
+// 2081 us, m=256 n=65536 572 -> 557; a nine-operation swizzle without any
+// conflict was 7 % slower, none at all for Y 11 %.
+// The arrays are allocated for whole groups of 16 rows (mp_pass_rows).
+__device__ __forceinline__ int swz(int k) { return k ^ ((k >> 3) & 7); }
+__device__ __forceinline__ int swzy(int k) { return k ^ ((k >> 4) & 15); }
 
 // What the rhs of the reduction steps of a tile depends on, kept by one
 // reduction for later right-hand sides: per survivor L_k, U_k and D'^-1, as
@@ -227,18 +235,19 @@ __device__ __forceinline__ int cr_reduce(float4* sL, float4* sU, float2* sY, int
         const int lo = clo - d2 + 1, hi = chi + d2 - 1;
         bool coupled = false;
         for (int k = tid * d2; k < TR; k += bd * d2) {
-            const int sk = swz(k), sm = swz(max(k - d, 0)), sp = swz(min(k + d, TR - 1));
+            const int km = max(k - d, 0), kp = min(k + d, TR - 1);
+            const int sk = swz(k), sm = swz(km), sp = swz(kp), yk = swzy(k), ym = swzy(km), yp = swzy(kp);
             M2 Lo, Uo, Mi;
             float2 Yo;
             const M2 Lk = m2(sL[sk]), Uk = m2(sU[sk]);
-            reduce_row(Lk, Uk, sY[sk], m2(sL[sm]), m2(sU[sm]), sY[sm], m2(sL[sp]), m2(sU[sp]), sY[sp], Lo, Uo, Yo, Mi);
+            reduce_row(Lk, Uk, sY[yk], m2(sL[sm]), m2(sU[sm]), sY[ym], m2(sL[sp]), m2(sU[sp]), sY[yp], Lo, Uo, Yo, Mi);
             if (kKeep) {
                 const int i = k >> (l + 1);
                 float4* const g = k + d < TR ? F.g + 3 * base + i : F.last + l;
                 const int step = k + d < TR ? (TR - d + d2 - 1) >> (l + 1) : kCrLevels;
                 g[0] = f4(Lk); g[step] = f4(Uk); g[2 * step] = f4(Mi);
             }
-            sL[sk] = f4(Lo); sU[sk] = f4(Uo); sY[sk] = Yo;
+            sL[sk] = f4(Lo); sU[sk] = f4(Uo); sY[yk] = Yo;
             if (k >= lo && k < hi) coupled |= fmaxf(amaxm(Lo), amaxm(Uo)) >= kTrunc;
         }
         base += (TR - d + d2 - 1) >> (l + 1);
@@ -271,8 +280,8 @@ __device__ __forceinline__ void cr_replay(const CrFactors& F, float2* sY, int TR
                 const int step = i < count ? count : kCrLevels;
                 fL = g[0]; fU = g[step]; fM = g[2 * step];
             }
-            const int sk = swz(k);
-            sY[sk] = reduce_rhs(m2(fL), m2(fU), sY[sk], sY[swz(max(k - d, 0))], sY[swz(min(k + d, TR - 1))], m2(fM));
+            const int yk = swzy(k), ym = swzy(max(k - d, 0)), yp = swzy(min(k + d, TR - 1));
+            sY[yk] = reduce_rhs(m2(fL), m2(fU), sY[yk], sY[ym], sY[yp], m2(fM));
         }
         base += count;
         count = (TR - d2 + 2 * d2 - 1) >> (l + 2);
@@ -293,11 +302,11 @@ __device__ __forceinline__ void cr_substitute(const float4* sL, const float4* sU
     for (int l = top - 1; l >= 0; l--) {
         const int d = 1 << l;
         for (int k = d + tid * 2 * d; k < TR; k += bd * 2 * d) {
-            const int sk = swz(k), sm = swz(k - d), sp = swz(min(k + d, TR - 1));
+            const int sk = swz(k), yk = swzy(k);
             const M2 Lk = m2(sL[sk]), Uk = m2(sU[sk]);
-            const float2 xm = sY[sm], xp = sY[sp], yk = sY[sk];
-            sY[sk] = make_float2(fmaf(-Uk.m1, xp.y, fmaf(-Uk.m0, xp.x, fmaf(-Lk.m1, xm.y, fmaf(-Lk.m0, xm.x, yk.x)))),
-                                 fmaf(-Uk.m3, xp.y, fmaf(-Uk.m2, xp.x, fmaf(-Lk.m3, xm.y, fmaf(-Lk.m2, xm.x, yk.y)))));
+            const float2 xm = sY[swzy(k - d)], xp = sY[swzy(min(k + d, TR - 1))], y = sY[yk];
+            sY[yk] = make_float2(fmaf(-Uk.m1, xp.y, fmaf(-Uk.m0, xp.x, fmaf(-Lk.m1, xm.y, fmaf(-Lk.m0, xm.x, y.x)))),
+                                 fmaf(-Uk.m3, xp.y, fmaf(-Uk.m2, xp.x, fmaf(-Lk.m3, xm.y, fmaf(-Lk.m2, xm.x, y.y)))));
         }
         __syncthreads();
     }

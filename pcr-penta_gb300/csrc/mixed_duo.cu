@@ -86,7 +86,7 @@ constexpr int kDuoMaxLevels = 6;
 constexpr size_t kDuoSmem = (size_t)kDuoSlots * kDuoSlotDoubles * sizeof(double)   // staging ring
                             + (size_t)kDuoRows * sizeof(double2)                     // x_0
                             + (size_t)kDuoRows * (2 * sizeof(float4) + sizeof(float2));   // reduction tile
-static_assert(kDuoRows % 8 == 0 && kDuoRows == 2 * kDuoThreads, "whole swizzle groups; one survivor per thread");
+static_assert(kDuoRows % 16 == 0 && kDuoRows == 2 * kDuoThreads, "whole swizzle groups; one survivor per thread");
 
 // TMEM columns: per warp group (warps 4g..4g+3) a region of 16-column
 // factorisation entries, one per level its threads can reach (levels
@@ -309,7 +309,7 @@ __device__ __forceinline__ void put_block_half(double a, double b, double c, dou
     const int sk = swz(k);
     reinterpret_cast<float2*>(sL + sk)[h] = make_float2(mA * a0, fmaf(mA, b0, mB * a1));
     reinterpret_cast<float2*>(sU + sk)[h] = make_float2(fmaf(mA, e0, mB * d1), mB * e1);
-    reinterpret_cast<float*>(sY + sk)[h] = fmaf(mA, y0, mB * y1);
+    reinterpret_cast<float*>(sY + swzy(k))[h] = fmaf(mA, y0, mB * y1);
 }
 
 // ---------------------------------------------------------------------------
@@ -332,10 +332,11 @@ __device__ __forceinline__ int cr_reduce_keep(float4* sL, float4* sU, float2* sY
         bool coupled = false;
         float v[16];
         if (act) {
-            const int sk = swz(k), sm = swz(max(k - d, 0)), sp = swz(min(k + d, TR - 1));
+            const int km = max(k - d, 0), kp = min(k + d, TR - 1);
+            const int sk = swz(k), sm = swz(km), sp = swz(kp);
             const M2 Lk = m2(sL[sk]), Uk = m2(sU[sk]), Lm = m2(sL[sm]), Um = m2(sU[sm]);
             const M2 Lp = m2(sL[sp]), Up = m2(sU[sp]);
-            const float2 Yk = sY[sk], ym = sY[sm], yp = sY[sp];
+            const float2 Yk = sY[swzy(k)], ym = sY[swzy(km)], yp = sY[swzy(kp)];
             M2 Dn;
             Dn.m0 = fmaf(-Uk.m1, Lp.m2, fmaf(-Uk.m0, Lp.m0, fmaf(-Lk.m1, Um.m2, fmaf(-Lk.m0, Um.m0, 1.0f))));
             Dn.m1 = fmaf(-Uk.m1, Lp.m3, fmaf(-Uk.m0, Lp.m1, fmaf(-Lk.m1, Um.m3, -Lk.m0 * Um.m1)));
@@ -349,7 +350,7 @@ __device__ __forceinline__ int cr_reduce_keep(float4* sL, float4* sU, float2* sY
             const M2 Lo = mmul(Mn, LL), Uo = mmul(Mn, UU);
             sL[sk] = f4(Lo);
             sU[sk] = f4(Uo);
-            sY[sk] = make_float2(fmaf(Mi.m0, y0, Mi.m1 * y1), fmaf(Mi.m2, y0, Mi.m3 * y1));
+            sY[swzy(k)] = make_float2(fmaf(Mi.m0, y0, Mi.m1 * y1), fmaf(Mi.m2, y0, Mi.m3 * y1));
             if (k >= clo - d2 + 1 && k < chi + d2 - 1) coupled = fmaxf(amaxm(Lo), amaxm(Uo)) >= kTrunc;
             v[0] = Lk.m0; v[1] = Lk.m1; v[2] = Lk.m2; v[3] = Lk.m3;
             v[4] = Uk.m0; v[5] = Uk.m1; v[6] = Uk.m2; v[7] = Uk.m3;
@@ -380,7 +381,7 @@ __device__ __forceinline__ void cr_replay_rhs(float2* sY, int TR, int top, uint3
             tmem_ld16(tw + 16u * l, v);
             tmem_wait_ld16(v);
             if (act) {
-                const int sk = swz(k), sm = swz(max(k - d, 0)), sp = swz(min(k + d, TR - 1));
+                const int sk = swzy(k), sm = swzy(max(k - d, 0)), sp = swzy(min(k + d, TR - 1));
                 const float2 Yk = sY[sk], ym = sY[sm], yp = sY[sp];
                 const float y0 = fmaf(-v[5], yp.y, fmaf(-v[4], yp.x, fmaf(-v[1], ym.y, fmaf(-v[0], ym.x, Yk.x))));
                 const float y1 = fmaf(-v[7], yp.y, fmaf(-v[6], yp.x, fmaf(-v[3], ym.y, fmaf(-v[2], ym.x, Yk.y))));
@@ -537,7 +538,7 @@ mp_duo_kernel(MpArgs p, DuoGeom g)
         const int klo = (int)(t.wlo - t.t0), khi = (int)(t.whi - t.t0);
         unsigned xm = 0u;
         for (int k = klo0 + tid; k < khi0; k += bd) {
-            const float2 v = sY[swz(k)];
+            const float2 v = sY[swzy(k)];
             sX0[k] = make_double2(f2d(v.x), f2d(v.y));
             if (k >= klo && k < khi) xm = max(xm, max(abs_bits(v.x), abs_bits(v.y)));
         }
@@ -575,7 +576,7 @@ mp_duo_kernel(MpArgs p, DuoGeom g)
             }
             const float pf = __shfl_xor_sync(0xffffffffu, rf, 1);
             tmem_wait_ld2(mA, mB);
-            if (active) reinterpret_cast<float*>(sY + swz(k))[h] = fmaf(mA, h ? pf : rf, mB * (h ? rf : pf));
+            if (active) reinterpret_cast<float*>(sY + swzy(k))[h] = fmaf(mA, h ? pf : rf, mB * (h ? rf : pf));
             cur = nxt;
         }
         __syncthreads();
@@ -587,7 +588,7 @@ mp_duo_kernel(MpArgs p, DuoGeom g)
         unsigned dm = 0u;
         double2* X = reinterpret_cast<double2*>(p.X0 + t.j * n);
         for (int k = klo + tid; k < khi; k += bd) {
-            const float2 v = sY[swz(k)];
+            const float2 v = sY[swzy(k)];
             const double2 x0 = sX0[k];
             X[t.t0 + k] = make_double2(__dadd_rn(x0.x, f2d(v.x)), __dadd_rn(x0.y, f2d(v.y)));
             dm = max(dm, max(abs_bits(v.x), abs_bits(v.y)));
