@@ -70,6 +70,9 @@ __device__ __forceinline__ unsigned expw(double x) { return hiw(x) & 0x7FF00000u
 __device__ __forceinline__ bool finite6(double p, double q, double r, double s, double t, double u) {
     return max(max(max(expw(p), expw(q)), max(expw(r), expw(s))), max(expw(t), expw(u))) < 0x7FF00000u;
 }
+__device__ __forceinline__ bool finite4(double p, double q, double r, double s) {
+    return max(max(expw(p), expw(q)), max(expw(r), expw(s))) < 0x7FF00000u;
+}
 
 constexpr int kMaxThreads = 256;
 constexpr int kMaxRowsPerThread = 8;
@@ -239,6 +242,26 @@ __device__ __forceinline__ bool row_a_none(TileRows<CAP>& t, int k, int dl, bool
     t.Ty[k] = add_z(add_z(t.y[k], g1.y), g2.y);
     t.Ta[k] = hasL ? szero(g1.a) : 0.0;
     t.Te[k] = hasR ? szero(g2.e) : 0.0;
+    return true;
+}
+
+// The same for a row with both sides whose b, c, d and y are not zero, in a
+// tile without infinities and nans: T(m) is the row itself, and of the
+// neighbours only the signs that a and e inherit are read (12 reads and 6
+// tests of the neighbours less; tridiagonal m=777 n=3001 644 -> 615 us).
+template <int CAP>
+__device__ __forceinline__ bool row_a_self(TileRows<CAP>& t, int k, int dl, bool has2L, bool has2R, double& cT)
+{
+    const double b = t.b[k], c = t.c[k], d = t.d[k], y = t.y[k], bL = t.b[k - dl], dR = t.d[k + dl];
+    if (!(nz(b) && nz(c) && nz(d) && nz(y))) return false;
+    const unsigned s1 = has2L && nz(bL) ? hiw(t.a[k]) ^ hiw(bL) ^ 0x80000000u : 0u;
+    const unsigned s2 = has2R && nz(dR) ? hiw(t.e[k]) ^ hiw(dR) ^ 0x80000000u : 0u;
+    cT = c;
+    t.Tc[k] = c;
+    t.Tr[k] = ieee::recip(c);
+    t.Tb[k] = b; t.Td[k] = d; t.Ty[k] = y;
+    t.Ta[k] = szero(s1 ^ hiw(t.a[k - dl]));
+    t.Te[k] = szero(s2 ^ hiw(t.e[k + dl]));
     return true;
 }
 
@@ -590,6 +613,15 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
     bool apart = p.final_step != 0;
     if (apart)
         for (int k = tid; k < TR; k += bd) apart = apart && decoupled(T, k);
+    // tridiagonal batches: no row of the tile holds an infinity or a nan (kept
+    // up by phase B)
+    __shared__ int s_odd;
+    if (p.tri) {
+        bool odd = false;
+        for (int k = tid; k < TR; k += bd) odd = odd || !finite4(T.b[k], T.c[k], T.d[k], T.y[k]);
+        const bool any = __syncthreads_or(odd);
+        if (tid == 0) s_odd = any;
+    }
     const int strides = __syncthreads_and(apart) ? 0 : p.K;
 
     for (int s = 0; s < strides; s++) {
@@ -606,6 +638,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
 
         // ---- phase A: T(m) = a1*row(m-d) + row(m) + a2*row(m+d) ----------
         bool zero_pivot = false;
+        const bool tame = p.tri && s_odd == 0;
 #pragma unroll 1
         for (int k = tid; k < TR; k += bd) {
             if (k < Alo || k >= Ahi) continue;
@@ -618,7 +651,10 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
             double cT;
             bool done = false;
             if (kFew) done = row_a_zeros(T, k, dl, hasL, has2L, hasR, has2R, cT);
-            else if (!left && !right) done = row_a_none(T, k, dl, hasL, has2L, hasR, has2R, cT);
+            else if (!left && !right) {
+                if (tame && hasL && hasR) done = row_a_self(T, k, dl, has2L, has2R, cT);
+                if (!done) done = row_a_none(T, k, dl, hasL, has2L, hasR, has2R, cT);
+            }
             else if (has2L && has2R) {
                 if (left && right) done = row_a_both(T, k, dl, cT);
                 else done = row_a_one(T, k, dl, right, cT);
@@ -671,6 +707,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
                 f1 = f.x; f2 = f.y;
             }
             apart = apart && !left && !right && decoupled(T, k);
+            if (tame && !finite4(T.b[k], T.c[k], T.d[k], T.y[k])) s_odd = 1;
             if (keep) { kept1[q] = f1; kept2[q] = f2; }
         }
         if (__syncthreads_and(apart)) break;
