@@ -589,10 +589,10 @@ struct TryTile {
     bool whole;                                   // the tile holds the whole system
 };
 
-__device__ __forceinline__ TryTile try_tile(const MpPassArgs& p, int64_t item)
+__device__ __forceinline__ TryTile try_tile(const MpPassArgs& p, int64_t item, int64_t j)
 {
     TryTile t;
-    t.j = item / p.nwin;
+    t.j = j;
     const int64_t w = item - t.j * p.nwin;
     t.wlo = w * (int64_t)p.L;
     t.whi = min(t.wlo + (int64_t)p.L, p.nb);
@@ -605,10 +605,10 @@ __device__ __forceinline__ TryTile try_tile(const MpPassArgs& p, int64_t item)
 
 // next item of this CTA with work: running system, window inside it, and
 // (after sweep 0) a system the windowed pass solves
-__device__ __forceinline__ int64_t try_next(const MpPassArgs& p, int64_t item, int64_t items)
+__device__ __forceinline__ int64_t try_next(const MpPassArgs& p, int64_t item, int64_t items, int64_t& j)
 {
     for (; item < items; item += gridDim.x) {
-        const int64_t j = item / p.nwin;
+        j = item / p.nwin;
         if (__ldg(p.fin + j)) continue;
         if (p.sweep > 0 && __ldg(p.fail + j)) continue;
         if ((item - j * p.nwin) * (int64_t)p.L >= p.nb) continue;
@@ -693,8 +693,9 @@ mp_try_kernel(MpPassArgs p)
     float4* sU = fsm + TRs;
     float2* sY = reinterpret_cast<float2*>(fsm + 2 * TRs);
     const int64_t items = p.m * p.nwin;
-    for (int64_t it = try_next(p, blockIdx.x, items); it < items; it = try_next(p, it + gridDim.x, items)) {
-        try_solve(p, try_tile(p, it), sL, sU, sY);
+    int64_t j = 0;
+    for (int64_t it = try_next(p, blockIdx.x, items, j); it < items; it = try_next(p, it + gridDim.x, items, j)) {
+        try_solve(p, try_tile(p, it, j), sL, sU, sY);
         __syncthreads();
     }
 }
@@ -746,12 +747,12 @@ __device__ __forceinline__ void first_residual(const MpArgs& p, const PairRun& r
 }
 
 template <bool RG>
-__device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, int64_t item,
+__device__ __forceinline__ void first_item(const MpArgs& p, const MpWindows& g, int64_t item, int64_t j,
                                            float4* sL, float4* sU, float2* sY)
 {
     const int tid = threadIdx.x, bd = blockDim.x;
     const int64_t n = p.n, nb = (n + 1) / 2;
-    const int64_t j = item / g.nwin, w = item - j * g.nwin;
+    const int64_t w = item - j * g.nwin;
     const int64_t wlo = w * (int64_t)g.L, whi = min(wlo + (int64_t)g.L, nb);
     const int64_t t0 = max(wlo - (int64_t)g.H, (int64_t)0), t1 = min(whi + (int64_t)g.H, nb);
     const int TR = (int)(t1 - t0);
@@ -858,8 +859,9 @@ mp_first_kernel(MpArgs p, MpWindows g)
     if (__ldg(p.live) == 0) return;               // the fused first sweeps finished every system
     const int64_t items = p.m * g.nwin;
     for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
-        if (__ldg(p.fin + it / g.nwin)) continue;   // finished by the fused first sweeps
-        first_item<RG>(p, g, it, sL, sU, sY);
+        const int64_t j = it / g.nwin;
+        if (__ldg(p.fin + j)) continue;           // finished by the fused first sweeps
+        first_item<RG>(p, g, it, j, sL, sU, sY);
         __syncthreads();
     }
 }
