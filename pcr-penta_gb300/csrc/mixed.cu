@@ -1005,12 +1005,13 @@ mp_decide_kernel(MpArgs p)
 // y keeps the rhs until the final copy, so no copy of it is needed.
 //
 // Bound by latency: two CTAs of 512 threads fill an SM's registers at n=4096
-// (FP64 pipe 40 %, ALU 47 %, issue 51 %; L2 and barrier waits).  Measured:
-// reducing the matrix again in every sweep, from a copy of the blocks in S0,
-// m=4096 n=4096 ADI 931 us, m=2048 n=2000 154; the factors kept instead, and
-// zero outer bands skipped, 887 and 133 (same bits).  Keeping the diagonal
-// inverses as well costs more L2 traffic than the instructions it saves (933
-// and 146); the iterate as 16-byte pairs changes nothing.
+// (FP64 pipe 41 %, ALU 45 %, issue 51 %; L2 and barrier waits).  Measured:
+// reducing the matrix again in every sweep, from a copy of the blocks, m=4096
+// n=4096 ADI 931 us; the factors kept instead, zero outer bands skipped and
+// the tile's cheaper swizzles 870 (same bits).  Keeping the diagonal inverses
+// as well costs more L2 traffic than the instructions it saves (+5 %), the
+// factors in shared memory as generic addresses +3 %; the iterate as 16-byte
+// pairs changes nothing.
 __device__ __forceinline__ void block_max(unsigned& dmb, unsigned long long& xb, unsigned* red_d,
                                           unsigned long long* red_x)
 {
@@ -1030,7 +1031,9 @@ __device__ __forceinline__ void block_max(unsigned& dmb, unsigned long long& xb,
 constexpr int kMpNarrow = 256;                   // block rows of a system solved by 128 threads
 constexpr int kMpSmallThreadsMax = 512;          // systems of >= 1024 block rows: 512 threads
 
-template <bool RG>
+// kKeep: sweep 0 keeps the factors of the reduction and later sweeps replay
+// it; else they reduce a copy of the level-0 blocks again (launch_mp_small)
+template <bool RG, bool kKeep>
 __global__ void __launch_bounds__(kMpSmallThreadsMax, 2)
 mp_small_kernel(MpArgs p)
 {
@@ -1047,8 +1050,9 @@ mp_small_kernel(MpArgs p)
     float2* sY = reinterpret_cast<float2*>(fsm + 2 * TRs);
     const int tid = threadIdx.x, bd = blockDim.x;
     // this CTA's part of the workspace, the same for every system it solves
-    // (what it writes stays in L2): the iterate, and the factors in the memory
-    // of S0 and R[], which follow each other (48 bytes per block row)
+    // (what it writes stays in L2): the iterate, and the factors (or the blocks)
+    // in the memory of S0 and R[], which follow each other (48 bytes per block
+    // row)
     double* __restrict__ X = p.X0 + blockIdx.x * n;
     const CrFactors F{p.S0 + 3 * nb * blockIdx.x, s_last};
     for (int64_t j = blockIdx.x; j < p.m; j += gridDim.x) {
@@ -1062,6 +1066,7 @@ mp_small_kernel(MpArgs p)
             if (i0 + 3 < n) any_e |= magbits(P.e1);
             const int sk = swz(k);
             sL[sk] = f4(r.L); sU[sk] = f4(r.U); sY[swzy(k)] = r.Y;
+            if (!kKeep) { F.g[2 * k] = f4(r.L); F.g[2 * k + 1] = f4(r.U); }
         }
         // an outer band that is zero in the whole system (one-sided operators)
         // is treated like a missing one: neither read nor multiplied again
@@ -1071,7 +1076,7 @@ mp_small_kernel(MpArgs p)
         int s = 0, top = 0;
         for (;; s++) {
             // (a whole system: never -1)
-            if (s == 0) top = cr_reduce<true>(sL, sU, sY, TR, 31, 0, TR, F);
+            if (!kKeep || s == 0) top = cr_reduce<kKeep>(sL, sU, sY, TR, 31, 0, TR, F);
             else cr_replay(F, sY, TR, top);
             cr_substitute(sL, sU, sY, TR, top);
             unsigned dmb = 0u;
@@ -1120,7 +1125,12 @@ mp_small_kernel(MpArgs p)
                 }
                 const M2 Mi = diag_inverse(P, i0, n);
                 sY[swzy(k)] = make_float2(fmaf(Mi.m0, rf0, Mi.m1 * rf1), fmaf(Mi.m2, rf0, Mi.m3 * rf1));
+                if (!kKeep) {
+                    const int sk = swz(k);
+                    sL[sk] = F.g[2 * k]; sU[sk] = F.g[2 * k + 1];
+                }
             }
+            if (!kKeep) __syncthreads();
         }
         for (int64_t i = tid; i < n; i += bd) x_write(p.xout, p.oss, p.ors, RG ? p.rg : nullptr, j, i, X[i]);
         if (tid == 0) { p.fin[j] = s + 1; p.status[j] = D.done ? 1 : 2; p.est[j] = D.est; }
@@ -1497,7 +1507,13 @@ cudaError_t launch_mp_small(const MpArgs& p, cudaStream_t s)
     if (nb > kMpMaxRows) return cudaErrorInvalidValue;
     if (p.m <= 0) return cudaSuccess;
     const size_t smem = mp_pass_smem((int)nb);
-    auto kern = p.rg ? mp_small_kernel<true> : mp_small_kernel<false>;
+    // short systems wait for a level's factors longer than they take to reduce
+    // it (us, reduced again / replayed: 29583 ADI systems of 139 rows 297 / 310,
+    // 40000 of 64 rows 143 / 146, 1024 of 512 rows 36.2 / 35.7, 4000 of 1000
+    // rows 242 / 231, 4096 of 4096 rows 910 / 874)
+    const bool keep = nb > kMpNarrow;
+    auto kern = p.rg ? (keep ? mp_small_kernel<true, true> : mp_small_kernel<true, false>)
+                     : (keep ? mp_small_kernel<false, true> : mp_small_kernel<false, false>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)mp_pass_smem(kMpMaxRows));
     if (e != cudaSuccess) return e;
