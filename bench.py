@@ -49,11 +49,11 @@ BYTES_PER_UNKNOWN = 56          # 5 FP64 bands + FP64 rhs read once, FP64 x writ
 # config's own layout and the autotuned plan.  The capture commands and the
 # raw figures are kept with the ncu summaries in the repository's profiles.
 MEASURED_TRAFFIC = {
-    ("c1", "f64"): (831.0, "ncu capture m=48 n=65536, the 8 pcr_pass_kernel launches of one solve"),
-    ("c1", "mixed"): (117.5, "ncu capture m=48 n=65536, mp_first_kernel + mp_try_kernel of one solve"),
-    ("c2", "mixed"): (123.0, "ncu capture m=1024 n=4096, the mp_small_kernel launch of one solve"),
-    ("c4", "f64"): (747.7, "ncu capture m=4 n=2^20, the 7 pcr_pass_kernel launches of one solve"),
-    ("c4", "mixed"): (139.2, "ncu capture m=4 n=2^20, mp_first_kernel + mp_try_kernel of one solve"),
+    ("c1", "f64"): (290.4, "ncu capture m=48 n=65536, the 4 pcr_pass_kernel launches of one solve"),
+    ("c1", "mixed"): (93.6, "ncu capture m=48 n=65536, mp_first_kernel + mp_try_kernel of one solve"),
+    ("c2", "mixed"): (95.1, "ncu capture m=1024 n=4096, the mp_small_kernel launch of one solve"),
+    ("c4", "f64"): (387.7, "ncu capture m=4 n=2^20, the 5 pcr_pass_kernel launches of one solve"),
+    ("c4", "mixed"): (98.2, "ncu capture m=4 n=2^20, mp_first_kernel + mp_try_kernel of one solve"),
 }
 
 
@@ -406,10 +406,9 @@ def run_ours(args, world, rank, local, pg):
                      "ms_at_peak": t_peak * 1e3, "frac": t_peak / (kms_med * 1e-3),
                      "note": "the reference's FP64 products/sums (exact count on n rows) at the measured "
                              "DFMA rate plus its IEEE divisions at the measured division rate "
-                             "(pcrp_measure_fp64), over the solve's kernel time; the kernels form "
-                             "operations with a zero operand (late strides, once a and e have "
-                             "underflowed) on the integer pipe and finish two quotients from one shared "
-                             "reciprocal, so frac is the rate of the reference's operations, not the "
+                             "(pcrp_measure_fp64), over the solve's kernel time; the kernels form the "
+                             "quotients, most products and the operations with a zero operand on the "
+                             "integer pipe, so frac is the rate of the reference's operations, not the "
                              "FP64 pipe's busy share (ncu reports that)"}
 
     # end to end through the public API with host buffers (pinned): pcrp_solve_host

@@ -8,7 +8,8 @@
 // ceil(m/32) systems, so little copying precedes the first solve, and each
 // next one three times as many, up to ceil(m/4), because a solve of few
 // systems fills the GPU less well than a large one (measured on GB300, m=256
-// n=65536: 0.102 ms per system at m=8, 0.088 at 32, 0.084 at 64).  The caller's stream is joined
+// n=65536, with FP64 kernels 2.5 times slower than the present ones: 0.102 ms
+// per system at m=8, 0.088 at 32, 0.084 at 64).  The caller's stream is joined
 // at both ends with events, so the call is asynchronous like the device
 // entry points (the host arrays must stay valid until the stream reaches
 // that point; page-locked host memory lets the copies run asynchronously).
