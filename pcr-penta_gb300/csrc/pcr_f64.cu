@@ -36,7 +36,7 @@
 // the FP64 pipe 72 % and the integer ALU 55 % busy (4 CTAs of 256 threads per
 // SM; what is left is the latency of the row's dependent chains between two
 // barriers).  Measured, before and after: m=64 n=2^20 weakly dominant 91.7 ->
-// 34.6 ms, m=256 n=65536 19.8 -> 8.0 ms, m=1024 n=512 interleaved 0.535 -> 0.265
+// 34.3 ms, m=256 n=65536 19.8 -> 8.0 ms, m=1024 n=512 interleaved 0.535 -> 0.265
 // ms; a dense two-stride pass at m=4 n=2^20 1.00 -> 0.38 ms.
 //
 // The reference's multiplier registers, which outlive a stride and are reused

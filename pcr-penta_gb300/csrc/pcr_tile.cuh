@@ -110,7 +110,9 @@ struct TileRows {
 // signs (bit 31) of the products of a zero multiplier of sign s with a row
 struct Signs { unsigned a, b, c, d, e, y; };
 
-// Phase A, both multipliers active.
+// Phase A, both multipliers active.  The rhs first (its products are FP64 and
+// start that pipe while the integer products run), the reciprocal last: the
+// other order 1 % slower (m=16 n=2^20 8.67 against 8.59 ms).
 template <int CAP>
 __device__ __forceinline__ bool row_a_both(TileRows<CAP>& t, int k, int dl, double& cT)
 {
@@ -123,14 +125,14 @@ __device__ __forceinline__ bool row_a_both(TileRows<CAP>& t, int k, int dl, doub
     if (!ieee::fits(w)) return false;
     const double al1 = ieee::div(neg(am), bL, ieee::recip(bL)), al2 = ieee::div(neg(em), dR, ieee::recip(dR));
     const ieee::Factor f1 = ieee::factor(al1), f2 = ieee::factor(al2);
+    t.Ty[k] = add(add(mul(al1, t.y[l]), t.y[k]), mul(al2, t.y[r]));
     cT = add(add(ieee::mul(f1, dL), t.c[k]), ieee::mul(f2, bR));
     t.Tc[k] = cT;
-    t.Tr[k] = ieee::recip(cT);
     t.Tb[k] = add(add(ieee::mul(f1, cL), t.b[k]), ieee::mul(f2, aR));
     t.Td[k] = add(add(ieee::mul(f1, eL), t.d[k]), ieee::mul(f2, cR));
-    t.Ty[k] = add(add(mul(al1, t.y[l]), t.y[k]), mul(al2, t.y[r]));
     t.Ta[k] = ieee::mul(f1, aL);
     t.Te[k] = ieee::mul(f2, eR);
+    t.Tr[k] = ieee::recip(cT);
     return true;
 }
 
