@@ -84,12 +84,14 @@ constexpr int kMaxRowsPerThread = 8;
 // (Reductions I-III, kernel.cu:63-140) for one case of operands each; they
 // return false, with nothing written, for rows outside their case, and those
 // rows take the general form in pcr_tile.  In every case the quotients and
-// most products run on the integer pipe (ieee_int.cuh), the sums and the rhs
-// products (a rhs is often zero, which is outside the integer product's
-// guard) on the FP64 pipe: per row and stride 36 products and sums and 4
-// quotients, of which 16 sums and 4 products stay FP64.  No branch inside a
-// case: with a branch per operation the chains of a row serialise (measured:
-// 14.0 against 13.2 ms for m=16 n=2^20).
+// most products run on the integer pipe (ieee_int.cuh), the sums and phase
+// B's rhs products on the FP64 pipe: per row and stride 36 products and sums
+// and 4 quotients, of which 16 sums and 2 products stay FP64.  A rhs is often
+// zero, which is outside the integer product's guard: phase A's dense case
+// decides for its two (m=256 n=65536 7.92 -> 7.82 ms); for phase B's as well
+// the same decision gains on one-sided batches what it costs on dense ones.
+// No other branch inside a case: with a branch per operation the chains of a
+// row serialise (measured: 14.0 against 13.2 ms for m=16 n=2^20).
 //
 // A multiplier of a side (left: row - dl, right: row + dl) is "active" when
 // it is a nonzero quotient inside the guard.  Otherwise it is a zero (its
@@ -110,8 +112,7 @@ struct TileRows {
 // signs (bit 31) of the products of a zero multiplier of sign s with a row
 struct Signs { unsigned a, b, c, d, e, y; };
 
-// Phase A, both multipliers active.  The rhs first (its products are FP64 and
-// start that pipe while the integer products run), the reciprocal last: the
+// Phase A, both multipliers active.  The rhs first, the reciprocal last: the
 // other order 1 % slower (m=16 n=2^20 8.67 against 8.59 ms).
 template <int CAP>
 __device__ __forceinline__ bool row_a_both(TileRows<CAP>& t, int k, int dl, double& cT)
@@ -125,7 +126,11 @@ __device__ __forceinline__ bool row_a_both(TileRows<CAP>& t, int k, int dl, doub
     if (!ieee::fits(w)) return false;
     const double al1 = ieee::div(neg(am), bL, ieee::recip(bL)), al2 = ieee::div(neg(em), dR, ieee::recip(dR));
     const ieee::Factor f1 = ieee::factor(al1), f2 = ieee::factor(al2);
-    t.Ty[k] = add(add(mul(al1, t.y[l]), t.y[k]), mul(al2, t.y[r]));
+    const double yl = t.y[l], yr = t.y[r];
+    double y1, y2;
+    if (ieee::fits(ieee::off(yl) | ieee::off(yr))) { y1 = ieee::mul(f1, yl); y2 = ieee::mul(f2, yr); }
+    else { y1 = mul(al1, yl); y2 = mul(al2, yr); }
+    t.Ty[k] = add(add(y1, t.y[k]), y2);
     cT = add(add(ieee::mul(f1, dL), t.c[k]), ieee::mul(f2, bR));
     t.Tc[k] = cT;
     t.Tb[k] = add(add(ieee::mul(f1, cL), t.b[k]), ieee::mul(f2, aR));
