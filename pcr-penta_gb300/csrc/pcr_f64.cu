@@ -32,8 +32,8 @@
 // busy.  The integer pipe runs beside it, so the quotients and 18 of the 20
 // products are formed there (ieee_int.cuh: correctly rounded, the same bits;
 // one product 25 instructions, one quotient 40) and 16 sums and 2 products stay
-// FP64.  A dense stride now issues ~1,150 warp instructions per 32 rows, with
-// the FP64 pipe 72 % and the integer ALU 55 % busy (4 CTAs of 256 threads per
+// FP64.  A dense stride now issues ~1,200 warp instructions per 32 rows, with
+// the FP64 pipe 67 % and the integer ALU 62 % busy (4 CTAs of 256 threads per
 // SM; what is left is the latency of the row's dependent chains between two
 // barriers).  Measured, before and after: m=64 n=2^20 weakly dominant 91.7 ->
 // 34.0 ms, m=256 n=65536 19.8 -> 7.9 ms, m=1024 n=512 interleaved 0.535 -> 0.265
