@@ -49,29 +49,29 @@ namespace {
 
 // CTAs per SM the register budget is set for: as many as shared memory holds
 // (100 bytes per row), at most 1024 threads.
-template <int CAP, bool kFew>
+template <int CAP, bool kFew, bool kTri>
 __global__ void __launch_bounds__(kMaxThreads, CAP > 1024 ? 1 : CAP > 544 ? 2 : 4)
 pcr_pass_kernel(const PcrPassArgs p)
 {
     extern __shared__ __align__(16) unsigned char pcr_smem[];
     const uint32_t blk = blockIdx.x, nwin = (uint32_t)p.nwin, item = blk / nwin, w = blk - item * nwin;
     const uint32_t j = item >> p.lg, r = item & ((1u << p.lg) - 1);
-    pcr_tile<CAP, false, kFew>(p, j, r, w, *reinterpret_cast<TileRows<CAP>*>(pcr_smem));
+    pcr_tile<CAP, false, kFew, kTri>(p, j, r, w, *reinterpret_cast<TileRows<CAP>*>(pcr_smem));
 }
 
 constexpr int kShortRows = 2048;          // rows of a short system
 
-template <int CAP, bool kFew>
+template <int CAP, bool kFew, bool kTri>
 cudaError_t launch_tiles(const PcrPassArgs& p, int threads, int64_t blocks, cudaStream_t s)
 {
     // per-device attribute, for more than the default 48 KB; cheap, and legal
     // while a stream is being captured
     if (sizeof(TileRows<CAP>) > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(pcr_pass_kernel<CAP, kFew>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        const cudaError_t e = cudaFuncSetAttribute(pcr_pass_kernel<CAP, kFew, kTri>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int)sizeof(TileRows<CAP>));
         if (e != cudaSuccess) return e;
     }
-    pcr_pass_kernel<CAP, kFew><<<(unsigned)blocks, threads, sizeof(TileRows<CAP>), s>>>(p);
+    pcr_pass_kernel<CAP, kFew, kTri><<<(unsigned)blocks, threads, sizeof(TileRows<CAP>), s>>>(p);
     count_launch();
     return cudaGetLastError();
 }
@@ -91,12 +91,13 @@ cudaError_t launch_cap(const PcrPassArgs& p, int threads, int64_t blocks, cudaSt
     // near an end in the late strides and would each load another case's code
     // (4000 systems of 100 rows 157 / 316, 2000 of 512 464 / 511, 2000 of 1000
     // 968 / 1135, 500 of 2000 581 / 609, 300 of 4000 737 / 708).  Tridiagonal
-    // batches never: their rows issue little FP64 work (8 systems of 512 rows
-    // 71 / 50).
+    // batches have a kernel of their own: their rows issue little FP64 work (8
+    // systems of 512 rows 71 us by one case for all, 41 by theirs).
     const bool few = blocks * (threads / 32) <= 8 * (int64_t)sms;
     const bool shorts = p.n <= kShortRows;
-    if ((few || shorts) && !p.tri) return launch_tiles<CAP, true>(p, threads, blocks, s);
-    return launch_tiles<CAP, false>(p, threads, blocks, s);
+    if (p.tri) return launch_tiles<CAP, false, true>(p, threads, blocks, s);
+    if (few || shorts) return launch_tiles<CAP, true, false>(p, threads, blocks, s);
+    return launch_tiles<CAP, false, false>(p, threads, blocks, s);
 }
 
 }  // namespace

@@ -255,7 +255,7 @@ __device__ __forceinline__ bool row_a_none(TileRows<CAP>& t, int k, int dl, bool
 // The same for a row with both sides whose b, c, d and y are not zero, in a
 // tile without infinities and nans: T(m) is the row itself, and of the
 // neighbours only the signs that a and e inherit are read (12 reads and 6
-// tests of the neighbours less; tridiagonal m=777 n=3001 644 -> 615 us).
+// tests of the neighbours less).
 template <int CAP>
 __device__ __forceinline__ bool row_a_self(TileRows<CAP>& t, int k, int dl, bool has2L, bool has2R, double& cT)
 {
@@ -269,6 +269,30 @@ __device__ __forceinline__ bool row_a_self(TileRows<CAP>& t, int k, int dl, bool
     t.Tb[k] = b; t.Td[k] = d; t.Ty[k] = y;
     t.Ta[k] = szero(s1 ^ hiw(t.a[k - dl]));
     t.Te[k] = szero(s2 ^ hiw(t.e[k + dl]));
+    return true;
+}
+
+// The same with zeros among b and d (the ends of the system), or a side
+// missing.
+template <int CAP>
+__device__ __forceinline__ bool row_a_tri(TileRows<CAP>& t, int k, int dl, bool hasL, bool has2L, bool hasR, bool has2R, double& cT)
+{
+    const int l = hasL ? k - dl : k, r = hasR ? k + dl : k;
+    const double b = t.b[k], c = t.c[k], d = t.d[k], y = t.y[k], bL = t.b[l], dR = t.d[r];
+    if (!(nz(c) && nz(y))) return false;
+    const unsigned s1 = has2L && nz(bL) ? hiw(t.a[k]) ^ hiw(bL) ^ 0x80000000u : 0u;
+    const unsigned s2 = has2R && nz(dR) ? hiw(t.e[k]) ^ hiw(dR) ^ 0x80000000u : 0u;
+    // (a missing side adds -0)
+    const unsigned zb = (hasL ? s1 ^ hiw(t.c[l]) : ~0u) & (hasR ? s2 ^ hiw(t.a[r]) : ~0u);
+    const unsigned zd = (hasL ? s1 ^ hiw(t.e[l]) : ~0u) & (hasR ? s2 ^ hiw(t.c[r]) : ~0u);
+    cT = c;
+    t.Tc[k] = c;
+    t.Tr[k] = ieee::recip(c);
+    t.Ty[k] = y;
+    t.Tb[k] = hasL ? add_z(b, zb) : 0.0;
+    t.Td[k] = hasR ? add_z(d, zd) : 0.0;
+    t.Ta[k] = hasL ? szero(s1 ^ hiw(t.a[l])) : 0.0;
+    t.Te[k] = hasR ? szero(s2 ^ hiw(t.e[r])) : 0.0;
     return true;
 }
 
@@ -433,6 +457,37 @@ __device__ __forceinline__ bool row_b_zeros(TileRows<CAP>& t, int k, int dl, boo
     return true;
 }
 
+// The zeros case of a tridiagonal row in a tile without infinities and nans:
+// a and e of the row and of T are zeros, of which only the signs are read.
+// Rows near an end used to take the general form here, in short systems most
+// rows of the late strides (with row_a_tri and a kernel of their own, us: 35733
+// systems of 90 rows 794 -> 580, 4000 of 128 143 -> 102, 777 of 3001 634 -> 585,
+// 256 of 16384 1093 -> 1064).
+template <int CAP>
+__device__ __forceinline__ bool row_b_tri(TileRows<CAP>& t, int k, int dl, bool hasL, bool hasR, double& f1, double& f2)
+{
+    const int l = hasL ? k - dl : k, r = hasR ? k + dl : k;
+    const double bi = t.b[k], di = t.d[k], cL = hasL ? t.Tc[l] : 1.0, cR = hasR ? t.Tc[r] : 1.0;
+    const double bL = hasL ? t.Tb[l] : 0.0, dL = hasL ? t.Td[l] : 0.0;
+    const double bR = hasR ? t.Tb[r] : 0.0, dR = hasR ? t.Td[r] : 0.0;
+    if (!ieee::fits(off_or_zero(bi) | off_or_zero(di) | ieee::off(cL) | ieee::off(cR) | off_or_zero(bL) |
+                    off_or_zero(dL) | off_or_zero(bR) | off_or_zero(dR))) return false;
+    const Multiplier m1 = multiplier(bi, cL, t.Tr[l], hasL && nz(bi), hasL);
+    const Multiplier m2 = multiplier(di, cR, t.Tr[r], hasR && nz(di), hasR);
+    const unsigned s1 = hiw(m1.x), s2 = hiw(m2.x);
+    const double ny = add(sub(hasL ? mul(m1.x, t.Ty[l]) : 0.0, t.y[k]), hasR ? mul(m2.x, t.Ty[r]) : 0.0);
+    const double nc = add(sub(times(m1, dL), t.c[k]), times(m2, bR));
+    const double b1 = times(m1, bL), d2 = times(m2, dR);
+    // b1 - a + m2 * Ta(r), m1 * Te(l) - e + d2, the zeros by their signs
+    const unsigned zb = hasR ? s2 ^ hiw(t.Ta[r]) : 0u, zd = (hasL ? s1 ^ hiw(t.Te[l]) : 0u) & ~hiw(t.e[k]);
+    const double nb = add_z(nz(b1) ? b1 : szero(hiw(b1) & ~hiw(t.a[k])), zb);
+    const double nd = add_z(d2, zd);
+    const double na = szero(hasL ? s1 ^ hiw(t.Ta[l]) : 0u), ne = szero(hasR ? s2 ^ hiw(t.Te[r]) : 0u);
+    t.y[k] = ny; t.c[k] = nc; t.b[k] = nb; t.d[k] = nd; t.a[k] = na; t.e[k] = ne;
+    f1 = m1.x; f2 = m2.x;
+    return true;
+}
+
 // The general forms: every operation on the FP64 pipe but the quotients whose
 // operands are inside the integer quotient's guard.
 template <int CAP>
@@ -514,8 +569,10 @@ __device__ __forceinline__ double gload(const double* p) {
 // One CTA's work: window w of subsystem r of system j (whole subsystem when
 // p.final_step).  Every thread of the CTA must call it with the same (j, r, w).
 // kFew: one case for all rows (row_a_zeros, row_b_zeros), then the general
-// form; else a case per kind of row (launch_cap chooses).
-template <int CAP, bool kL2Only = false, bool kFew = false>
+// form; else a case per kind of row (launch_cap chooses).  kTri: a tridiagonal
+// batch (null outer bands), whose rows have cases of their own; in a kernel of
+// their own, since in the pentadiagonal one they cost it 2-3 %.
+template <int CAP, bool kL2Only = false, bool kFew = false, bool kTri = false>
 __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32_t r, uint32_t w, TileRows<CAP>& T)
 {
     // row numbers inside a system fit 32 bits (n <= 2^31), and G = 2^lg: a
@@ -623,7 +680,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
     // tridiagonal batches: no row of the tile holds an infinity or a nan (kept
     // up by phase B)
     __shared__ int s_odd;
-    if (p.tri) {
+    if (kTri) {
         bool odd = false;
         for (int k = tid; k < TR; k += bd) odd = odd || !finite4(T.b[k], T.c[k], T.d[k], T.y[k]);
         const bool any = __syncthreads_or(odd);
@@ -645,7 +702,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
 
         // ---- phase A: T(m) = a1*row(m-d) + row(m) + a2*row(m+d) ----------
         bool zero_pivot = false;
-        const bool tame = p.tri && s_odd == 0;
+        const bool tame = kTri && s_odd == 0;
 #pragma unroll 1
         for (int k = tid; k < TR; k += bd) {
             if (k < Alo || k >= Ahi) continue;
@@ -660,9 +717,10 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
             if (kFew) done = row_a_zeros(T, k, dl, hasL, has2L, hasR, has2R, cT);
             else if (!left && !right) {
                 if (tame && hasL && hasR) done = row_a_self(T, k, dl, has2L, has2R, cT);
+                if (tame && !done) done = row_a_tri(T, k, dl, hasL, has2L, hasR, has2R, cT);
                 if (!done) done = row_a_none(T, k, dl, hasL, has2L, hasR, has2R, cT);
             }
-            else if (has2L && has2R) {
+            else if (!kTri && has2L && has2R) {
                 if (left && right) done = row_a_both(T, k, dl, cT);
                 else done = row_a_one(T, k, dl, right, cT);
                 if (!done) done = row_a_tiny(T, k, dl, hasL, has2L, hasR, has2R, cT);
@@ -700,6 +758,15 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
             bool done = false;
             if (kFew) done = row_b_zeros(T, k, dl, hasL, hasR, f1, f2);
             else if (!left && !right) done = row_b_none(T, k, dl, hasL, hasR, f1, f2);
+            else if (kTri) {
+                // the dense form of inner rows in a window, one form for all in
+                // a whole subsystem, where most rows are near an end
+                const bool inner = k - 3 * dl >= kfirst && k + 3 * dl <= klast;
+                if (inner && !p.final_step && left && right && !nz(T.a[k]) && !nz(T.e[k]))
+                    done = row_b_both<true, true>(T, k, dl, f1, f2);
+                else if (tame) done = row_b_tri(T, k, dl, hasL, hasR, f1, f2);
+                if (!done && (inner || tame)) done = row_b_tiny(T, k, dl, hasL, hasR, f1, f2);
+            }
             else if (k - 3 * dl >= kfirst && k + 3 * dl <= klast) {
                 if (left && right) {
                     const bool za = !nz(T.a[k]), ze = !nz(T.e[k]);
@@ -714,7 +781,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
                 f1 = f.x; f2 = f.y;
             }
             apart = apart && !left && !right && decoupled(T, k);
-            if (tame && !finite4(T.b[k], T.c[k], T.d[k], T.y[k])) s_odd = 1;
+            if (kTri && !finite4(T.b[k], T.c[k], T.d[k], T.y[k])) s_odd = 1;
             if (keep) { kept1[q] = f1; kept2[q] = f2; }
         }
         if (__syncthreads_and(apart)) break;

@@ -153,6 +153,7 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 // four CTAs per SM: 512-row tiles (50 KB) fit shared memory four times over,
 // at 64 registers (three at 80: 24.6 against 22.8 ms for 4096 systems of 32 to
 // 65536 rows)
+template <bool kTri>
 __global__ void __launch_bounds__(kRgThreads, 4)
 rg_persistent_kernel(RgArgs a)
 {
@@ -240,11 +241,11 @@ rg_persistent_kernel(RgArgs a)
             // finish writes x in their natural order
             p.src_sub = lvl > 0 ? 1 : 0;
             p.dst_sub = fin ? 0 : 1;
-            p.tri = !a.src[A_] && !a.src[E_];
+            p.tri = kTri;
             p.bulk = 0;                               // (per-thread loads through L2: data of this launch)
             const uint32_t nwin = (uint32_t)lv.nwin, r = fin ? (uint32_t)i : (uint32_t)i / nwin;
             const uint32_t w = fin ? 0u : (uint32_t)i - r * nwin;
-            pcr_tile<kRgCap, true>(p, k, r, w, *reinterpret_cast<RgTile*>(pcr_smem));
+            pcr_tile<kRgCap, true, false, kTri>(p, k, r, w, *reinterpret_cast<RgTile*>(pcr_smem));
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -310,12 +311,18 @@ cudaError_t remember_and_launch(const GraphKey& key, cudaGraphExec_t exec, cudaS
     return cudaGraphLaunch(exec, st);
 }
 
+// the persistent kernel of a batch with outer bands a, e
+auto rg_kernel(const double* a, const double* e)
+{
+    return a || e ? rg_persistent_kernel<false> : rg_persistent_kernel<true>;
+}
+
 cudaError_t enqueue(const RgArgs& a, int grid, cudaStream_t s)
 {
     const int pg = (int)std::min<int64_t>(std::max<int64_t>(1, cdiv64(a.nsys, 256)), 1024);
     rg_plan_kernel<<<pg, 256, 0, s>>>(a);
     rg_scan_kernel<<<1, 1024, 0, s>>>(a);
-    rg_persistent_kernel<<<grid, kRgThreads, sizeof(RgTile), s>>>(a);
+    rg_kernel(a.src[A_], a.src[E_])<<<grid, kRgThreads, sizeof(RgTile), s>>>(a);
     return cudaGetLastError();
 }
 
@@ -398,10 +405,11 @@ pcrp_status ragged_f64(const double* a, const double* b, const double* c, const 
     int dev = 0;
     ce = cudaGetDevice(&dev);
     if (ce != cudaSuccess) return cuda_error(ce, "cudaGetDevice");
-    ce = cudaFuncSetAttribute(rg_persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RgTile));
+    const auto kern = rg_kernel(a, e);
+    ce = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RgTile));
     if (ce != cudaSuccess) return cuda_error(ce, "cudaFuncSetAttribute");
     int per_sm = 0, sms = 0;
-    ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, rg_persistent_kernel, kRgThreads, sizeof(RgTile));
+    ce = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kRgThreads, sizeof(RgTile));
     if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (ce != cudaSuccess) return cuda_error(ce, "occupancy query");
     const int grid = std::max(1, per_sm * sms);
