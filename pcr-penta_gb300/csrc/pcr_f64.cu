@@ -49,29 +49,29 @@ namespace {
 
 // CTAs per SM the register budget is set for: as many as shared memory holds
 // (100 bytes per row), at most 1024 threads.
-template <int CAP, bool kFew, bool kTri>
+template <int CAP, bool kFew, bool kTri, bool kWindow = false>
 __global__ void __launch_bounds__(kMaxThreads, CAP > 1024 ? 1 : CAP > 544 ? 2 : 4)
 pcr_pass_kernel(const PcrPassArgs p)
 {
     extern __shared__ __align__(16) unsigned char pcr_smem[];
     const uint32_t blk = blockIdx.x, nwin = (uint32_t)p.nwin, item = blk / nwin, w = blk - item * nwin;
     const uint32_t j = item >> p.lg, r = item & ((1u << p.lg) - 1);
-    pcr_tile<CAP, false, kFew, kTri>(p, j, r, w, *reinterpret_cast<TileRows<CAP>*>(pcr_smem));
+    pcr_tile<CAP, false, kFew, kTri, kWindow>(p, j, r, w, *reinterpret_cast<TileRows<CAP>*>(pcr_smem));
 }
 
 constexpr int kShortRows = 2048;          // rows of a short system
 
-template <int CAP, bool kFew, bool kTri>
+template <int CAP, bool kFew, bool kTri, bool kWindow = false>
 cudaError_t launch_tiles(const PcrPassArgs& p, int threads, int64_t blocks, cudaStream_t s)
 {
     // per-device attribute, for more than the default 48 KB; cheap, and legal
     // while a stream is being captured
     if (sizeof(TileRows<CAP>) > 48 * 1024) {
-        const cudaError_t e = cudaFuncSetAttribute(pcr_pass_kernel<CAP, kFew, kTri>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        const cudaError_t e = cudaFuncSetAttribute(pcr_pass_kernel<CAP, kFew, kTri, kWindow>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                    (int)sizeof(TileRows<CAP>));
         if (e != cudaSuccess) return e;
     }
-    pcr_pass_kernel<CAP, kFew, kTri><<<(unsigned)blocks, threads, sizeof(TileRows<CAP>), s>>>(p);
+    pcr_pass_kernel<CAP, kFew, kTri, kWindow><<<(unsigned)blocks, threads, sizeof(TileRows<CAP>), s>>>(p);
     count_launch();
     return cudaGetLastError();
 }
@@ -97,6 +97,9 @@ cudaError_t launch_cap(const PcrPassArgs& p, int threads, int64_t blocks, cudaSt
     const bool shorts = p.n <= kShortRows;
     if (p.tri) return launch_tiles<CAP, false, true>(p, threads, blocks, s);
     if (few || shorts) return launch_tiles<CAP, true, false>(p, threads, blocks, s);
+    // window passes of the tuned plans' tiles (512 rows) have a kernel without the finish
+    constexpr bool tuned = CAP == 544;
+    if (tuned && !p.final_step) return launch_tiles<CAP, false, false, tuned>(p, threads, blocks, s);
     return launch_tiles<CAP, false, false>(p, threads, blocks, s);
 }
 

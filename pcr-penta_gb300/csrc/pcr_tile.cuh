@@ -76,6 +76,22 @@ __device__ __forceinline__ bool finite4(double p, double q, double r, double s) 
 
 constexpr int kMaxThreads = 256;
 constexpr int kMaxRowsPerThread = 8;
+// Lanes of a warp whose rows take different cases run one after the other, and
+// a row that no case takes runs the general form after its tests.  Where such
+// rows lie among others away from the ends (scattered zeros, rows scaled far
+// apart, exact zero pivots), the general form for all rows of the warp is
+// cheaper than the cases and then that.  So the rows without a case wait for a
+// second loop, and a warp that met one away from the ends sends all its rows
+// there in the next kGeneralStrides strides of the phase, and then tries the
+// cases again (1: a third of the gain lost; for the rest of a pass: 2 % more
+// lost where outer coefficients underflow unevenly).  us, before and after:
+// 2 % zeros among a, b, d, e and y, m=300 n=2049 941 -> 515, m=256 n=4096 1420
+// -> 780, 512 ragged systems 8437 -> 4560; small integers with exact zero
+// pivots, m=256 n=4096 1188 -> 757; rows scaled by up to 2^+-400 1311 -> 958;
+// dense rows, where the second loop is mostly for those near the ends: m=300
+// n=2049 457 -> 440, m=64 n=2^20 33.9 -> 34.2 ms, 20000 ragged systems of 32
+// rows 1.43 -> 1.51 ms.
+constexpr int kGeneralStrides = 3;
 
 // ---------------------------------------------------------------------------
 // One row of a stride, straight-line per case
@@ -571,14 +587,18 @@ __device__ __forceinline__ double gload(const double* p) {
 // kFew: one case for all rows (row_a_zeros, row_b_zeros), then the general
 // form; else a case per kind of row (launch_cap chooses).  kTri: a tridiagonal
 // batch (null outer bands), whose rows have cases of their own; in a kernel of
-// their own, since in the pentadiagonal one they cost it 2-3 %.
-template <int CAP, bool kL2Only = false, bool kFew = false, bool kTri = false>
+// their own, since in the pentadiagonal one they cost it 2-3 %.  kWindow: the
+// pass is a window pass (not p.final_step), known when compiled, which leaves
+// the finish and its tests out of the kernel that long systems spend most of
+// their time in (m=64 n=2^20 34.5 -> 34.3 ms, m=256 n=65536 7.86 -> 7.81).
+template <int CAP, bool kL2Only = false, bool kFew = false, bool kTri = false, bool kWindow = false>
 __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32_t r, uint32_t w, TileRows<CAP>& T)
 {
     // row numbers inside a system fit 32 bits (n <= 2^31), and G = 2^lg: a
     // 64-bit division is ~80 instructions, and every thread runs this code for
     // two rows of a tile
     const int lg = p.lg;
+    const bool final_step = !kWindow && p.final_step != 0;
     const int64_t sbase = p.offsets ? p.offsets[j] : j * p.src_ss;
     const int64_t dbase = p.offsets ? p.offsets[j] : j * p.dst_ss;
     const uint32_t nsys = (uint32_t)(p.offsets ? (p.offsets[j + 1] - p.offsets[j]) : p.n);
@@ -612,7 +632,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
     // 2^p.rem rows.  So they are kept (in local memory) by the last stride but
     // one, and pass through global memory only if a global pass ends with it.
     double kept1[kMaxRowsPerThread], kept2[kMaxRowsPerThread];
-    if (p.bulk) {
+    if (!kWindow && p.bulk) {
         // The whole system is the tile (t0 = 0, TR = n, even): thread 0
         // stages each array with one bulk asynchronous copy straight into its
         // shared-memory row array (16-byte aligned: contiguous layout, even
@@ -674,7 +694,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
     // y away from the ends of the exponent range): every further stride only
     // changes the signs of c and y of every row, which the final step's
     // products and quotients cancel, so the remaining strides are skipped.
-    bool apart = p.final_step != 0;
+    bool apart = final_step;
     if (apart)
         for (int k = tid; k < TR; k += bd) apart = apart && decoupled(T, k);
     // tridiagonal batches: no row of the tile holds an infinity or a nan (kept
@@ -688,12 +708,21 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
     }
     const int strides = __syncthreads_and(apart) ? 0 : p.K;
 
+    // the first strides in which this warp's rows try the cases of phase A and
+    // of phase B (kGeneralStrides): not the first ones if rows with and without
+    // zeros mix (the warp's first rows are looked at)
+    int casesA = 0, casesB = 0;
+    if (!kFew && !kTri) {
+        const bool z = tid < TR && !(nz(T.a[tid]) && nz(T.b[tid]) && nz(T.d[tid]) && nz(T.e[tid]));
+        const unsigned zm = __ballot_sync(~0u, z);
+        if (zm != ~0u && __popc(zm) >= 2) casesA = casesB = kGeneralStrides;
+    }
     for (int s = 0; s < strides; s++) {
         const int dl = 1 << s;
         // rows this stride must produce: the window widened by the halo the
         // remaining strides of the pass still consume (everything if final).
         int klo = 0, khi = TR;
-        if (!p.final_step) {
+        if (!final_step) {
             const int rem = 2 * ((1 << p.K) - (2 << s));
             klo = max((int)(wlo - t0) - rem, kfirst); khi = min((int)(whi - t0) + rem, klast + 1);
         }
@@ -703,30 +732,46 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
         // ---- phase A: T(m) = a1*row(m-d) + row(m) + a2*row(m+d) ----------
         bool zero_pivot = false;
         const bool tame = kTri && s_odd == 0;
+        unsigned rest = 0u;                       // rows no case took: bit q for row tid + q*bd
 #pragma unroll 1
-        for (int k = tid; k < TR; k += bd) {
+        for (int k = tid, q = 0; k < TR; k += bd, q++) {
             if (k < Alo || k >= Ahi) continue;
             const bool hasL = k - dl >= kfirst, hasR = k + dl <= klast;
             const bool has2L = k - 2 * dl >= kfirst, has2R = k + 2 * dl <= klast;
             if (!(hasL || hasR)) continue;
             const bool left = has2L && nz(T.a[k]), right = has2R && nz(T.e[k]);   // nonzero multipliers
-            // rows near the subsystem's ends, where neighbouring rows hold
-            // structural zeros, take the general form at once
             double cT;
             bool done = false;
-            if (kFew) done = row_a_zeros(T, k, dl, hasL, has2L, hasR, has2R, cT);
-            else if (!left && !right) {
+            if (kFew) {
+                done = row_a_zeros(T, k, dl, hasL, has2L, hasR, has2R, cT);
+                if (!done) cT = row_a_general(T, k, dl, hasL, has2L, hasR, has2R);
+                done = true;
+            } else if (!left && !right) {
                 if (tame && hasL && hasR) done = row_a_self(T, k, dl, has2L, has2R, cT);
                 if (tame && !done) done = row_a_tri(T, k, dl, hasL, has2L, hasR, has2R, cT);
                 if (!done) done = row_a_none(T, k, dl, hasL, has2L, hasR, has2R, cT);
-            }
-            else if (!kTri && has2L && has2R) {
+            } else if (!kTri && s >= casesA && has2L && has2R) {
                 if (left && right) done = row_a_both(T, k, dl, cT);
                 else done = row_a_one(T, k, dl, right, cT);
                 if (!done) done = row_a_tiny(T, k, dl, hasL, has2L, hasR, has2R, cT);
             }
-            if (!done) cT = row_a_general(T, k, dl, hasL, has2L, hasR, has2R);
-            zero_pivot = zero_pivot || !nz(cT);
+            // (rows near the subsystem's ends, where neighbouring rows hold
+            // structural zeros, have no case)
+            if (done) zero_pivot = zero_pivot || !nz(cT);
+            else rest |= 1u << q;
+        }
+        if (!kFew && __any_sync(~0u, rest != 0u)) {
+            bool odd = false;                     // a row away from the ends without a case
+#pragma unroll 1
+            for (; rest != 0u; rest &= rest - 1u) {
+                const int k = tid + (__ffs(rest) - 1) * bd;
+                const bool hasL = k - dl >= kfirst, hasR = k + dl <= klast;
+                const bool has2L = k - 2 * dl >= kfirst, has2R = k + 2 * dl <= klast;
+                const double cT = row_a_general(T, k, dl, hasL, has2L, hasR, has2R);
+                if (!kTri) odd = odd || (k - 3 * dl >= kfirst && k + 3 * dl <= klast);
+                zero_pivot = zero_pivot || !nz(cT);
+            }
+            if (!kTri && __any_sync(~0u, odd) && s >= casesA) casesA = s + 1 + kGeneralStrides;
         }
         double pre1[kMaxRowsPerThread], pre2[kMaxRowsPerThread];
         if (__syncthreads_or(zero_pivot)) {
@@ -747,7 +792,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
 
         // ---- phase B: new row = b/cT(i-d)*T(i-d) - row(i) + d/cT(i+d)*T(i+d)
         // (in place: phase B reads no other row's state)
-        apart = p.final_step != 0;
+        apart = final_step;
         const bool keep = s == p.rem - 2;
 #pragma unroll 1
         for (int k = tid, q = 0; k < TR; k += bd, q++) {
@@ -756,18 +801,24 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
             const bool left = hasL && nz(T.b[k]), right = hasR && nz(T.d[k]);
             double f1 = 0.0, f2 = 0.0;
             bool done = false;
-            if (kFew) done = row_b_zeros(T, k, dl, hasL, hasR, f1, f2);
-            else if (!left && !right) done = row_b_none(T, k, dl, hasL, hasR, f1, f2);
-            else if (kTri) {
+            if (kFew) {
+                done = row_b_zeros(T, k, dl, hasL, hasR, f1, f2);
+                if (!done) {
+                    const double2 f = row_b_general(T, k, dl, hasL, hasR, pre1[q], pre2[q]);
+                    f1 = f.x; f2 = f.y;
+                    done = true;
+                }
+            } else if (!left && !right) {
+                done = row_b_none(T, k, dl, hasL, hasR, f1, f2);
+            } else if (kTri) {
                 // the dense form of inner rows in a window, one form for all in
                 // a whole subsystem, where most rows are near an end
                 const bool inner = k - 3 * dl >= kfirst && k + 3 * dl <= klast;
-                if (inner && !p.final_step && left && right && !nz(T.a[k]) && !nz(T.e[k]))
+                if (inner && !final_step && left && right && !nz(T.a[k]) && !nz(T.e[k]))
                     done = row_b_both<true, true>(T, k, dl, f1, f2);
                 else if (tame) done = row_b_tri(T, k, dl, hasL, hasR, f1, f2);
                 if (!done && (inner || tame)) done = row_b_tiny(T, k, dl, hasL, hasR, f1, f2);
-            }
-            else if (k - 3 * dl >= kfirst && k + 3 * dl <= klast) {
+            } else if (s >= casesB && k - 3 * dl >= kfirst && k + 3 * dl <= klast) {
                 if (left && right) {
                     const bool za = !nz(T.a[k]), ze = !nz(T.e[k]);
                     if (za && ze) done = row_b_both<true, true>(T, k, dl, f1, f2);
@@ -776,18 +827,33 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
                 }
                 if (!done) done = row_b_tiny(T, k, dl, hasL, hasR, f1, f2);
             }
-            if (!done) {
-                const double2 f = row_b_general(T, k, dl, hasL, hasR, pre1[q], pre2[q]);
-                f1 = f.x; f2 = f.y;
+            if (done) {
+                apart = apart && !left && !right && decoupled(T, k);
+                if (kTri && !finite4(T.b[k], T.c[k], T.d[k], T.y[k])) s_odd = 1;
+                if (keep) { kept1[q] = f1; kept2[q] = f2; }
+            } else {
+                rest |= 1u << q;
             }
-            apart = apart && !left && !right && decoupled(T, k);
-            if (kTri && !finite4(T.b[k], T.c[k], T.d[k], T.y[k])) s_odd = 1;
-            if (keep) { kept1[q] = f1; kept2[q] = f2; }
+        }
+        if (!kFew && __any_sync(~0u, rest != 0u)) {
+            bool odd = false;
+#pragma unroll 1
+            for (; rest != 0u; rest &= rest - 1u) {
+                const int q = __ffs(rest) - 1, k = tid + q * bd;
+                const bool hasL = k - dl >= kfirst, hasR = k + dl <= klast;
+                const bool left = hasL && nz(T.b[k]), right = hasR && nz(T.d[k]);
+                const double2 f = row_b_general(T, k, dl, hasL, hasR, pre1[q], pre2[q]);
+                if (!kTri) odd = odd || (k - 4 * dl >= kfirst && k + 4 * dl <= klast);
+                apart = apart && !left && !right && decoupled(T, k);
+                if (kTri && !finite4(T.b[k], T.c[k], T.d[k], T.y[k])) s_odd = 1;
+                if (keep) { kept1[q] = f.x; kept2[q] = f.y; }
+            }
+            if (!kTri && __any_sync(~0u, odd) && s >= casesB) casesB = s + 1 + kGeneralStrides;
         }
         if (__syncthreads_and(apart)) break;
     }
 
-    if (p.final_step) {
+    if (final_step) {
         // kernel.cu:145-153: pairs (i, i+delta) by Cramer's rule, singles x = y/c
         const int df = 1 << p.K;
         double* __restrict__ gx = p.x + doff;
