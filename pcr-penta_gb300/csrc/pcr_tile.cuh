@@ -504,6 +504,33 @@ __device__ __forceinline__ bool row_b_tri(TileRows<CAP>& t, int k, int dl, bool 
     return true;
 }
 
+// The same for operands outside the integer forms' window, with the products
+// on the FP64 pipe (10 FP64 operations instead of the general form's 18, and
+// no second try: rows scaled by up to 2^+-400, us, 4000 systems of 128 rows
+// 224 -> 153, 777 of 3001 1299 -> 880; every row scaled by 1e40 151 -> 107 and
+// 854 -> 620).
+template <int CAP>
+__device__ __forceinline__ bool row_b_wide(TileRows<CAP>& t, int k, int dl, bool hasL, bool hasR, double& f1, double& f2)
+{
+    const int l = hasL ? k - dl : k, r = hasR ? k + dl : k;
+    const double cL = hasL ? t.Tc[l] : 1.0, cR = hasR ? t.Tc[r] : 1.0;
+    if (!(nz(cL) && nz(cR))) return false;
+    const double g1 = hasL ? quot(t.b[k], cL, t.Tr[l]) : 0.0, g2 = hasR ? quot(t.d[k], cR, t.Tr[r]) : 0.0;
+    if (max(expw(g1), expw(g2)) >= 0x7FF00000u) return false;
+    const unsigned s1 = hiw(g1), s2 = hiw(g2);
+    const double ny = add(sub(hasL ? mul(g1, t.Ty[l]) : 0.0, t.y[k]), hasR ? mul(g2, t.Ty[r]) : 0.0);
+    const double nc = add(sub(hasL ? mul(g1, t.Td[l]) : 0.0, t.c[k]), hasR ? mul(g2, t.Tb[r]) : 0.0);
+    const double b1 = hasL ? mul(g1, t.Tb[l]) : 0.0, d2 = hasR ? mul(g2, t.Td[r]) : 0.0;
+    const unsigned zb = hasR ? s2 ^ hiw(t.Ta[r]) : 0u, zd = (hasL ? s1 ^ hiw(t.Te[l]) : 0u) & ~hiw(t.e[k]);
+    t.b[k] = add_z(nz(b1) ? b1 : szero(hiw(b1) & ~hiw(t.a[k])), zb);
+    t.d[k] = add_z(d2, zd);
+    t.a[k] = szero(hasL ? s1 ^ hiw(t.Ta[l]) : 0u);
+    t.e[k] = szero(hasR ? s2 ^ hiw(t.Te[r]) : 0u);
+    t.c[k] = nc; t.y[k] = ny;
+    f1 = g1; f2 = g2;
+    return true;
+}
+
 // The general forms: every operation on the FP64 pipe but the quotients whose
 // operands are inside the integer quotient's guard.
 template <int CAP>
@@ -817,7 +844,6 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
                 if (inner && !final_step && left && right && !nz(T.a[k]) && !nz(T.e[k]))
                     done = row_b_both<true, true>(T, k, dl, f1, f2);
                 else if (tame) done = row_b_tri(T, k, dl, hasL, hasR, f1, f2);
-                if (!done && (inner || tame)) done = row_b_tiny(T, k, dl, hasL, hasR, f1, f2);
             } else if (s >= casesB && k - 3 * dl >= kfirst && k + 3 * dl <= klast) {
                 if (left && right) {
                     const bool za = !nz(T.a[k]), ze = !nz(T.e[k]);
@@ -842,7 +868,9 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
                 const int q = __ffs(rest) - 1, k = tid + q * bd;
                 const bool hasL = k - dl >= kfirst, hasR = k + dl <= klast;
                 const bool left = hasL && nz(T.b[k]), right = hasR && nz(T.d[k]);
-                const double2 f = row_b_general(T, k, dl, hasL, hasR, pre1[q], pre2[q]);
+                double2 f;
+                if (!(tame && row_b_wide(T, k, dl, hasL, hasR, f.x, f.y)))
+                    f = row_b_general(T, k, dl, hasL, hasR, pre1[q], pre2[q]);
                 if (!kTri) odd = odd || (k - 4 * dl >= kfirst && k + 4 * dl <= klast);
                 apart = apart && !left && !right && decoupled(T, k);
                 if (kTri && !finite4(T.b[k], T.c[k], T.d[k], T.y[k])) s_odd = 1;
