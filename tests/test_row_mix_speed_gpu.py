@@ -69,6 +69,19 @@ def test_mixed_rows_cost_no_more_than_general_ones(cuda, kind, m, n):
     assert us <= 1.45 * ref
 
 
+# Short systems and few of them, where one case serves all rows: a warp's rows
+# take it or the general form together (lane by lane: 1.4 and 1.5 times; now 1.0).
+@pytest.mark.parametrize("m,n", [(8, 512), (4000, 128)])
+def test_one_case_or_the_general_form(cuda, m, n):
+    rng = np.random.default_rng(n)
+    arrs = mix("rows", rng, m, n)
+    us, x = solve_us(arrs, m, n)
+    ref, _ = solve_us(mix("scaled", rng, m, n), m, n)
+    print(f"\n[rows m={m} n={n}] {us:.1f} us, every row general {ref:.1f} us")
+    assert_bitexact(x, O.pcr(*arrs, m, n), f"rows m={m} n={n}")
+    assert us <= 1.25 * ref
+
+
 # A tridiagonal batch (null outer bands) of widely scaled rows runs 10 of the
 # pentadiagonal general form's 36 FP64 operations per row and stride and the
 # same two quotients of phase B: with the general form it took 0.85 of the
