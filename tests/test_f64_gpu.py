@@ -112,6 +112,11 @@ def test_zero_outer_bands_bitexact(cuda, n, path, opts, special, zero_d):
     assert_bitexact(x, ref, f"zero bands n={n} path={path} special={special} zero_d={zero_d}")
 
 
+# (The quotients are formed on the integer pipe since: two digits of 31 and 22
+# bits from a 32-bit reciprocal inside the exponent guard, ieee::div, and one
+# routine for operands of any size, ieee::div_any, outside it; __ddiv_rn only for
+# non-finite operands, zero and subnormal divisors and overflow.  The check is
+# the same.)
 @pytest.mark.parametrize("mode", [0, 1, 2, 3, 4])
 def test_phase_b_quotients_match_ieee_division(cuda, mode):
     """Phase B forms its two quotients from one correctly rounded reciprocal
@@ -122,6 +127,7 @@ def test_phase_b_quotients_match_ieee_division(cuda, mode):
     assert fast > (1 << 26)                       # the guard admits most pairs of every class
 
 
+# (Past the guard it is ieee::div_any that takes over now, not the division.)
 @pytest.mark.parametrize("n", [700, 5000, 65536])
 def test_rows_scaled_across_the_exponent_range_bitexact(cuda, n):
     """Rows scaled by random powers of two up to 2^+-500.  A power-of-two row

@@ -81,6 +81,8 @@ def bands(kind, rng, m, n):
 @pytest.mark.gpu
 # one row case short of / at / past: the short-system limit (320), the tile (512), its window with halos (544), two
 # and more passes; odd, and powers of two
+# (The short-system limit is 2048 rows since, so these batches run the one case for all rows; test_row_cases_gpu.py
+# runs the same kinds in the kernels that take a case per kind of row.)
 @pytest.mark.parametrize("n", [3, 33, 320, 321, 512, 513, 1023, 1024, 1090, 4096, 9001])
 @pytest.mark.parametrize("kind", ["tiny", "a0", "e0", "holes", "dyadic", "huge"])
 def test_row_cases_bitexact(cuda, n, kind):
