@@ -289,6 +289,19 @@ pcrp_status pcrp_measure_pipes(float* ms, pcrp_stream stream);
 pcrp_status pcrp_check_quotients(int32_t mode, uint64_t seed, int64_t samples, uint64_t* mismatches,
                                  uint64_t* markstein, pcrp_stream stream);
 
+/* Checks the integer-pipe products and quotients of the FP64 kernels one by
+ * one against IEEE arithmetic (__dmul_rn, __ddiv_rn) on `samples` seeded random
+ * operand triples of class `mode` (0: exponents of the row cases' window
+ * 2^-400 .. 2^112, 1: its two ends, mantissas near all ones or a power of two,
+ * 2: such mantissas, exponents within 2^+-8, 3: short mantissas whose products
+ * are exact or ties, 4: any exponent).  Synchronous.  counts[0]: results whose
+ * bits differ; compared were counts[1] products of two operands, counts[2]
+ * quotients of two window operands and their product with a third, counts[3]
+ * quotients by the routine for operands of any size.  A diagnostic; no
+ * counterpart in the reference. */
+pcrp_status pcrp_check_integer_arithmetic(int32_t mode, uint64_t seed, int64_t samples, uint64_t counts[4],
+                                          pcrp_stream stream);
+
 /* ------------------------------------------------------------------------ */
 /* Seeded input generators (host memory, threads over systems)              */
 /* ------------------------------------------------------------------------ */

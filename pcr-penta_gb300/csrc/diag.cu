@@ -163,6 +163,63 @@ quotient_check(int mode, uint64_t seed, int64_t per_thread, unsigned long long* 
     atomicAdd(fast, nf);
 }
 
+// An operand of the products' check from 64 random bits and a few more (`t`).
+// Mode 3: an odd integer of t's width, p or 54 - p or 55 - p bits for the two
+// factors of a pair, so that a product has 53 to 55 bits: exact or, with its
+// lowest bit set and 54 of them, half way between two doubles.
+__device__ __forceinline__ double factor_operand(uint64_t r, int mode, int bits)
+{
+    uint64_t mant = r & 0xFFFFFFFFFFFFFull;
+    int e = (int)((r >> 52) & 0x7FFu);
+    const bool ones = (r >> 13) & 1;
+    switch (mode) {
+    case 0: e = 623 + e % 512; break;
+    case 1: e = (e & 1) ? 623 + (e >> 1) % 3 : 1134 - (e >> 1) % 3; mant = ones ? mant | 0xFFFFFFFFFFF80ull : mant & 0x7Full; break;
+    case 2: e = 1023 + e % 16 - 8; mant = ones ? mant | 0xFFFFFFFFFFF80ull : mant & 0x7Full; break;
+    case 3: {
+        e = 1023 + e % 16 - 8;
+        const uint64_t unit = uint64_t(1) << (53 - bits);       // lowest bit of a significand of `bits` bits
+        mant = bits == 1 ? 0 : ((mant & ~(2 * unit - 1)) | unit);
+        break;
+    }
+    default: break;
+    }
+    return __longlong_as_double((long long)((r & 0x8000000000000000ull) | ((uint64_t)e << 52) | mant));
+}
+
+__global__ void __launch_bounds__(kProbeThreads)
+arithmetic_check(int mode, uint64_t seed, int64_t per_thread, unsigned long long* counts)
+{
+    const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
+    unsigned long long bad = 0, np = 0, nq = 0, na = 0;
+    auto differ = [](double x, double ref) {
+        return __double_as_longlong(x) != __double_as_longlong(ref) && !(x != x && ref != ref);
+    };
+    for (int64_t i = 0; i < per_thread; i++) {
+        const uint64_t r1 = mix64(seed ^ (t * 0x100000001B3ull + (uint64_t)i * 3)), r2 = mix64(r1 + 1), r3 = mix64(r1 + 2);
+        const int p = 2 + (int)((r2 >> 3) % 51);                // 2 .. 52 bits
+        const double a = factor_operand(r1, mode, p), b = factor_operand(r2, mode, 54 - p + (int)(r3 & 1));
+        const double z = factor_operand(r3, mode, p);
+        const int sum = (int)((hiw(a) >> 20) & 0x7FFu) + (int)((hiw(b) >> 20) & 0x7FFu);
+        const bool normal = expw(a) != 0u && expw(b) != 0u && expw(a) < 0x7FF00000u && expw(b) < 0x7FF00000u;
+        if (normal && sum >= 1024 && sum <= 3068) {
+            bad += differ(ieee::mul(ieee::factor(a), b), __dmul_rn(a, b));
+            np++;
+        }
+        if (ieee::fits(ieee::off(a) | ieee::off(b) | ieee::off(z))) {
+            const double q = ieee::div(a, b, ieee::recip(b));
+            bad += differ(q, __ddiv_rn(a, b)) || differ(ieee::mul(ieee::factor(q), z), __dmul_rn(q, z));
+            nq++;
+        }
+        double q;
+        if (ieee::div_any(a, b, q)) { bad += differ(q, __ddiv_rn(a, b)); na++; }
+    }
+    atomicAdd(counts, bad);
+    atomicAdd(counts + 1, np);
+    atomicAdd(counts + 2, nq);
+    atomicAdd(counts + 3, na);
+}
+
 }  // namespace
 }  // namespace pcrp
 
@@ -197,6 +254,36 @@ extern "C" pcrp_status pcrp_check_quotients(int32_t mode, uint64_t seed, int64_t
     if (e != cudaSuccess) return cuda_error(e, "pcrp_check_quotients");
     *mismatches = host[0];
     *markstein = host[1];
+    return PCRP_OK;
+}
+
+extern "C" pcrp_status pcrp_check_integer_arithmetic(int32_t mode, uint64_t seed, int64_t samples, uint64_t counts[4],
+                                                     pcrp_stream stream)
+{
+    const char* who = "pcrp_check_integer_arithmetic";
+    if (!counts || samples < 0 || mode < 0 || mode > 4) return set_error(PCRP_EINVAL, "%s: bad argument", who);
+    cudaStream_t s = (cudaStream_t)stream;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return cuda_error(e, who);
+    unsigned long long* cnt = nullptr;
+    e = cudaMallocAsync(reinterpret_cast<void**>(&cnt), 4 * sizeof(unsigned long long), s);
+    if (e != cudaSuccess) return cuda_error(e, who);
+    const unsigned grid = (unsigned)sms * 8;
+    const int64_t threads = (int64_t)grid * kProbeThreads;
+    unsigned long long host[4] = {0, 0, 0, 0};
+    e = cudaMemsetAsync(cnt, 0, sizeof host, s);
+    if (e == cudaSuccess) {
+        arithmetic_check<<<grid, kProbeThreads, 0, s>>>(mode, seed, (samples + threads - 1) / threads, cnt);
+        count_launch();
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(host, cnt, sizeof host, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    cudaFreeAsync(cnt, s);
+    if (e != cudaSuccess) return cuda_error(e, who);
+    for (int k = 0; k < 4; k++) counts[k] = host[k];
     return PCRP_OK;
 }
 

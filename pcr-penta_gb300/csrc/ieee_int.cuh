@@ -81,20 +81,22 @@ PCRP_FN Factor factor(double x)
     return {lo(x), mant_hi(h), (h & 0xFFF00000u) - (1024u << 20)};
 }
 
-// Guard of both factors: exponent field in [513, 1533], so the product's is
-// in [3, 2044].
+// Both exponent fields in [513, 1533]: the product's is in [3, 2044].  (`mul`
+// takes any two normal factors whose fields sum to between 1024 and 3068: the
+// product's field is in [1, 2046], or it overflows by rounding.)
 PCRP_FN bool mid(double x) { return (hi(x) << 1) - (513u << 21) < (1021u << 21); }
 
 // Guard of many operands at once: `off(x)` is below 2^30 iff x's exponent
 // field is in [623, 1134] (2^-400 <= |x| < 2^112), so `fits` of the or of
-// several tests them all.  Quotients of such operands (2^-513 .. 2^513), and
-// products of a quotient with one, are inside the guards of `div` and `mul`
-// and normal.  The window reaches further down than up because the couplings
+// several tests them all.  Quotients of such operands are normal, their
+// exponent field in [511, 1535] (2^-512 < |q| <= 2^512), and so are products of
+// a quotient with one, [111, 1647]: inside what `div` and `mul` take, though a
+// quotient at either end is outside `mid`.  The window reaches further down than up because the couplings
 // of diagonally dominant systems square with every stride.
 PCRP_FN uint32_t off(double x) { return hi(x) * 2u - (623u << 21); }
 PCRP_FN bool fits(uint32_t offs) { return offs < (1u << 30); }
 
-// x*y for x, y inside the guard.  The 105- or 106-bit product of the
+// x*y for normal x, y with a normal product (see `mid`).  The 105- or 106-bit product of the
 // mantissas is formed in 32-bit words w3:w2:w1:w0, shifted left by 12 or 11
 // so that its upper words hold the 53 result bits and the next one the rest,
 // and rounded to nearest even: up iff the rest, with "odd, or more below"

@@ -87,6 +87,7 @@ _SIGS = {
     "pcrp_measure_fp64": [_vp, _vp, _vp],
     "pcrp_measure_pipes": [_vp, _vp],
     "pcrp_check_quotients": [_i32, ctypes.c_uint64, _i64, _vp, _vp, _vp],
+    "pcrp_check_integer_arithmetic": [_i32, ctypes.c_uint64, _i64, _vp, _vp],
     "pcrp_generate": [_i32, ctypes.c_uint64, _i64, _i64, _i32] + [_vp] * 6 + [_i32],
     "pcrp_generate_device": [_i32, ctypes.c_uint64, _i64, _i64, _i32] + [_vp] * 6 + [_vp],
     "pcrp_ragged_sizes": [ctypes.c_uint64, _i64, _i64, _i64, _vp],
@@ -328,6 +329,16 @@ def check_quotients(mode: int, seed: int, samples: int, stream=None):
     _check(lib().pcrp_check_quotients(mode, seed, samples, ctypes.byref(bad), ctypes.byref(fast), _stream(stream)),
            "pcrp_check_quotients")
     return int(bad.value), int(fast.value)
+
+
+def check_integer_arithmetic(mode: int, seed: int, samples: int, stream=None):
+    """(mismatches, products, quotients with a product of each, quotients of any
+    size) of the FP64 kernels' integer-pipe arithmetic against IEEE results
+    (pcrp_check_integer_arithmetic); synchronous."""
+    counts = (ctypes.c_uint64 * 4)()
+    _check(lib().pcrp_check_integer_arithmetic(mode, seed, samples, counts, _stream(stream)),
+           "pcrp_check_integer_arithmetic")
+    return tuple(int(c) for c in counts)
 
 
 # ----------------------------------------------------------------------------

@@ -103,3 +103,73 @@ def test_last_strides_across_passes_bitexact(cuda, opts):
         arrs = bands("dyadic", rng, 40, n)
         x, _ = gpu_f64(arrs, 40, n, opts=pcrp.Opts(**opts))
         assert_bitexact(x, O.pcr(*arrs, 40, n), f"n={n} {opts}")
+
+
+COMPOSED = HOST.split("static double gen")[0] + r"""
+static double make(int e, uint64_t m) {
+    const uint64_t u = (rnd() & (1ull << 63)) | ((uint64_t)e << 52) | (m & 0xFFFFFFFFFFFFFull);
+    double d; memcpy(&d, &u, 8); return d;
+}
+static double end() {                               // the window's ends, mantissas near all ones or a power of two
+    const uint64_t r = rnd(), m = (r & 4) ? ~(rnd() % 16) : rnd() % 16;
+    return make((r & 1) ? 623 + (r >> 8) % 2 : 1134 - (r >> 8) % 2, (r & 8) ? m : rnd() >> 12);
+}
+static double odd(int bits) {                       // an odd integer of so many bits, scaled into [1, 2)
+    const uint64_t unit = 1ull << (53 - bits);
+    return make(1015 + rnd() % 16, bits == 1 ? 0 : ((rnd() >> 12) & ~(2 * unit - 1)) | unit);
+}
+static bool same(double x, const volatile double& y) { return memcmp(&x, (const void*)&y, 8) == 0; }
+int main() {
+    long bad = 0, outside = 0, ties = 0;
+    for (int i = 0; i < 4000000; i++) {
+        const double x = end(), y = end(), z = end();
+        const volatile double q = x / y, p = q * z;
+        const double g = ieee::div(x, y, ieee::recip(y));
+        bad += !same(g, q) || !same(ieee::mul(ieee::factor(g), z), p);
+        outside += !ieee::mid(g);
+        const int k = 2 + rnd() % 51;
+        const double a = odd(k), b = odd(54 - k + rnd() % 2);
+        const volatile double r = a * b;
+        bad += !same(ieee::mul(ieee::factor(a), b), r);
+        ties += __builtin_fma(a, b, -r) != 0.0;
+    }
+    printf("%ld %ld %ld\n", bad, outside, ties);
+}
+"""
+
+
+def test_products_of_quotients_and_ties_are_ieee(tmp_path):
+    """Products as the kernels form them: a quotient of two window operands,
+    whose exponent may lie outside `mid`, times a third; and products half way
+    between two doubles."""
+    src = tmp_path / "t.cpp"
+    src.write_text(COMPOSED)
+    subprocess.run(["g++", "-O2", "-ffp-contract=off", "-I", CSRC, str(src), "-o", str(tmp_path / "t")], check=True)
+    bad, outside, ties = map(int, subprocess.run([str(tmp_path / "t")], check=True, capture_output=True,
+                                                 text=True).stdout.split())
+    assert bad == 0
+    assert outside > 100000 and ties > 1000000
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [0, 1, 2, 3, 4])
+def test_integer_arithmetic_on_the_device_is_ieee(cuda, mode):
+    """The device code (its own carry chains) one operation at a time."""
+    samples = 1 << 27
+    bad, products, quotients, any_size = pcrp.check_integer_arithmetic(mode, 77 + mode, samples)
+    assert bad == 0
+    # shares: every triple but in mode 4, where exponents of the window are (512/2048)^3 of them and sums that
+    # leave the product normal about 3/4
+    assert products >= (samples // 2 if mode == 4 else samples)
+    assert quotients >= (samples // 128 if mode == 4 else samples)
+    assert any_size >= samples // 4
+
+
+def test_integer_arithmetic_check_refuses_bad_arguments(built_lib):
+    import ctypes
+    counts = (ctypes.c_uint64 * 4)()
+    f = pcrp.lib().pcrp_check_integer_arithmetic
+    assert f(-1, 0, 1, counts, None) == 1
+    assert f(5, 0, 1, counts, None) == 1
+    assert f(0, 0, -1, counts, None) == 1
+    assert f(0, 0, 1, None, None) == 1
