@@ -186,7 +186,7 @@ pcrp_status f64_solve(const double* a, const double* b, const double* c, const d
     p.src[A_] = a; p.src[B_] = b; p.src[C_] = c; p.src[D_] = d; p.src[E_] = e; p.src[Y_] = y;
     p.src_ss = ss; p.src_rs = rs;
     p.n = n; p.m = m; p.G = 1;
-    p.tri = !a && !e;
+    const bool tri = !a && !e;
 
     double* bufs[2][NSTATE] = {};
     if (s1 > 0) {
@@ -226,7 +226,7 @@ pcrp_status f64_solve(const double* a, const double* b, const double* c, const d
         for (int k = 0; k < NSTATE; k++) p.dst[k] = bufs[cur][k];
         p.dst_ss = n; p.dst_rs = 1;
         p.dst_sub = 1;                      // the next pass reads each subsystem in one run
-        cudaError_t ce = launch_pcr_pass(p, pl.threads, st);
+        cudaError_t ce = launch_pcr_pass(p, pl.threads, st, tri);
         if (ce != cudaSuccess) return cuda_error(ce, "pcr global pass launch");
         for (int k = 0; k < NSTATE; k++) p.src[k] = bufs[cur][k];
         p.src_ss = n; p.src_rs = 1; p.src_sub = 1;
@@ -250,7 +250,7 @@ pcrp_status f64_solve(const double* a, const double* b, const double* c, const d
     }
     p.x = y; p.dst_ss = ss; p.dst_rs = rs; p.dst_sub = 0;
     for (int k = 0; k < NSTATE; k++) p.dst[k] = nullptr;
-    cudaError_t ce = launch_pcr_pass(p, pl.threads, st);
+    cudaError_t ce = launch_pcr_pass(p, pl.threads, st, tri);
     if (ce != cudaSuccess) return cuda_error(ce, "pcr shared-memory pass launch");
     return PCRP_OK;
 }

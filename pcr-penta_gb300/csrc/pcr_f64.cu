@@ -77,7 +77,7 @@ cudaError_t launch_tiles(const PcrPassArgs& p, int threads, int64_t blocks, cuda
 }
 
 template <int CAP>
-cudaError_t launch_cap(const PcrPassArgs& p, int threads, int64_t blocks, cudaStream_t s)
+cudaError_t launch_cap(const PcrPassArgs& p, bool tridiagonal, int threads, int64_t blocks, cudaStream_t s)
 {
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -95,7 +95,7 @@ cudaError_t launch_cap(const PcrPassArgs& p, int threads, int64_t blocks, cudaSt
     // systems of 512 rows 71 us by one case for all, 41 by theirs).
     const bool few = blocks * (threads / 32) <= 8 * (int64_t)sms;
     const bool shorts = p.n <= kShortRows;
-    if (p.tri) return launch_tiles<CAP, false, true>(p, threads, blocks, s);
+    if (tridiagonal) return launch_tiles<CAP, false, true>(p, threads, blocks, s);
     if (few || shorts) return launch_tiles<CAP, true, false>(p, threads, blocks, s);
     // window passes of the tuned plans' tiles (512 rows) have a kernel without the finish
     constexpr bool tuned = CAP == 544;
@@ -107,7 +107,7 @@ cudaError_t launch_cap(const PcrPassArgs& p, int threads, int64_t blocks, cudaSt
 
 int pcr_max_smem_rows() { return 1920; }
 
-cudaError_t launch_pcr_pass(const PcrPassArgs& p, int threads, cudaStream_t s)
+cudaError_t launch_pcr_pass(const PcrPassArgs& p, int threads, cudaStream_t s, bool tridiagonal)
 {
     if (threads <= 0 || threads > kMaxThreads) threads = kMaxThreads;
     threads = (threads + 31) / 32 * 32;
@@ -121,14 +121,14 @@ cudaError_t launch_pcr_pass(const PcrPassArgs& p, int threads, cudaStream_t s)
     const int64_t blocks = p.m * p.G * p.nwin;
     if (blocks <= 0) return cudaSuccess;
     if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-    if (p.TRmax <= 32) return launch_cap<32>(p, threads, blocks, s);
-    if (p.TRmax <= 64) return launch_cap<64>(p, threads, blocks, s);
-    if (p.TRmax <= 128) return launch_cap<128>(p, threads, blocks, s);
-    if (p.TRmax <= 256) return launch_cap<256>(p, threads, blocks, s);
-    if (p.TRmax <= 384) return launch_cap<384>(p, threads, blocks, s);
-    if (p.TRmax <= 544) return launch_cap<544>(p, threads, blocks, s);
-    if (p.TRmax <= 1024) return launch_cap<1024>(p, threads, blocks, s);
-    return launch_cap<1920>(p, threads, blocks, s);
+    if (p.TRmax <= 32) return launch_cap<32>(p, tridiagonal, threads, blocks, s);
+    if (p.TRmax <= 64) return launch_cap<64>(p, tridiagonal, threads, blocks, s);
+    if (p.TRmax <= 128) return launch_cap<128>(p, tridiagonal, threads, blocks, s);
+    if (p.TRmax <= 256) return launch_cap<256>(p, tridiagonal, threads, blocks, s);
+    if (p.TRmax <= 384) return launch_cap<384>(p, tridiagonal, threads, blocks, s);
+    if (p.TRmax <= 544) return launch_cap<544>(p, tridiagonal, threads, blocks, s);
+    if (p.TRmax <= 1024) return launch_cap<1024>(p, tridiagonal, threads, blocks, s);
+    return launch_cap<1920>(p, tridiagonal, threads, blocks, s);
 }
 
 }  // namespace pcrp

@@ -66,13 +66,13 @@ struct PcrPassArgs {
     int TRmax;                   // shared-memory rows per CTA (>= L + 2H, or whole subsystem)
     int src_sub;                 // 1: src is subsystem-major at stride G (uniform batches)
     int dst_sub;                 // 1: dst is subsystem-major at stride G*2^K (uniform batches)
-    int tri;                     // 1: the batch entered without outer bands (a = e = null)
     int bulk;                    // 1: whole systems (G = 1, one tile) of even n in contiguous, 16-byte aligned
                                  // arrays: the tile is staged by bulk asynchronous copies (one per array)
 };
 
-// Host-side launchers (pcr_f64.cu).
-cudaError_t launch_pcr_pass(const PcrPassArgs& p, int threads, cudaStream_t s);
+// Host-side launchers (pcr_f64.cu).  tridiagonal: the batch entered without
+// outer bands (a = e = null).
+cudaError_t launch_pcr_pass(const PcrPassArgs& p, int threads, cudaStream_t s, bool tridiagonal);
 // dst[k] (cols x rows) = transpose of src[k] (rows x cols), both row-major,
 // for up to 6 arrays in one launch; pairs with a null pointer are skipped
 // (layout.cu): interleaved n x m <-> contiguous m x n batches

@@ -241,7 +241,6 @@ rg_persistent_kernel(RgArgs a)
             // finish writes x in their natural order
             p.src_sub = lvl > 0 ? 1 : 0;
             p.dst_sub = fin ? 0 : 1;
-            p.tri = kTri;
             p.bulk = 0;                               // (per-thread loads through L2: data of this launch)
             const uint32_t nwin = (uint32_t)lv.nwin, r = fin ? (uint32_t)i : (uint32_t)i / nwin;
             const uint32_t w = fin ? 0u : (uint32_t)i - r * nwin;
