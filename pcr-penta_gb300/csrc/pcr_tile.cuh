@@ -80,17 +80,18 @@ constexpr int kMaxRowsPerThread = 8;
 // a row that no case takes runs the general form after its tests.  Where such
 // rows lie among others away from the ends (scattered zeros, rows scaled far
 // apart, exact zero pivots), the general form for all rows of the warp is
-// cheaper than the cases and then that.  So the rows without a case wait for a
-// second loop, and a warp that met one away from the ends sends all its rows
-// there in the next kGeneralStrides strides of the phase, and then tries the
-// cases again (1: a third of the gain lost; for the rest of a pass: 2 % more
-// lost where outer coefficients underflow unevenly).  us, before and after:
-// 2 % zeros among a, b, d, e and y, m=300 n=2049 941 -> 515, m=256 n=4096 1420
-// -> 780, 512 ragged systems 8437 -> 4560; small integers with exact zero
-// pivots, m=256 n=4096 1188 -> 757; rows scaled by up to 2^+-400 1311 -> 958;
-// dense rows, where the second loop is mostly for those near the ends: m=300
-// n=2049 457 -> 440, m=64 n=2^20 33.9 -> 34.2 ms, 20000 ragged systems of 32
-// rows 1.43 -> 1.51 ms.
+// cheaper than the cases and then that.  So a warp that met one away from the
+// ends sends all its rows there in the next kGeneralStrides strides of the
+// phase, and then tries the cases again (1: a third of the gain lost; for the
+// rest of a pass: 2 % more lost where outer coefficients underflow unevenly).
+// In phase A the rows without a case wait for a loop of their own, so that
+// those of a thread's two rows run together (inline 1-2 % slower); in phase B
+// that loop cost weakly dominant batches 1-2 % (m=64 n=2^20 34.2 against 33.75
+// ms, m=256 n=65536 8.80 against 8.61).  us, without any of this and now:
+// 2 % zeros among a, b, d, e and y, m=300 n=2049 945 -> 493, m=256 n=4096 1408
+// -> 740; small integers with exact zero pivots, m=256 n=4096 1189 -> 753; rows
+// scaled by up to 2^+-400 1306 -> 959; dense rows m=300 n=2049 457 -> 437,
+// m=64 n=2^20 33.9 -> 33.75 ms, 20000 ragged systems of 8 to 64 rows 1.53 -> 1.21.
 constexpr int kGeneralStrides = 3;
 
 // ---------------------------------------------------------------------------
@@ -765,6 +766,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
         // ---- phase A: T(m) = a1*row(m-d) + row(m) + a2*row(m+d) ----------
         bool zero_pivot = false;
         const bool tame = kTri && s_odd == 0;
+        bool odd = false;                         // a row away from the ends without a case
         unsigned rest = 0u;                       // rows no case took: bit q for row tid + q*bd
 #pragma unroll 1
         for (int k = tid, q = 0; k < TR; k += bd, q++) {
@@ -794,7 +796,6 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
             else rest |= 1u << q;
         }
         if (!kFew && __any_sync(~0u, rest != 0u)) {
-            bool odd = false;                     // a row away from the ends without a case
 #pragma unroll 1
             for (; rest != 0u; rest &= rest - 1u) {
                 const int k = tid + (__ffs(rest) - 1) * bd;
@@ -827,6 +828,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
         // (in place: phase B reads no other row's state)
         apart = final_step;
         const bool keep = s == p.rem - 2;
+        odd = false;
 #pragma unroll 1
         for (int k = tid, q = 0; k < TR; k += bd, q++) {
             if (k < klo || k >= khi) continue;
@@ -864,16 +866,6 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
                 if (kTri && !finite4(T.b[k], T.c[k], T.d[k], T.y[k])) s_odd = 1;
                 if (keep) { kept1[q] = f1; kept2[q] = f2; }
             } else {
-                rest |= 1u << q;
-            }
-        }
-        if (!kFew && __any_sync(~0u, rest != 0u)) {
-            bool odd = false;
-#pragma unroll 1
-            for (; rest != 0u; rest &= rest - 1u) {
-                const int q = __ffs(rest) - 1, k = tid + q * bd;
-                const bool hasL = k - dl >= kfirst, hasR = k + dl <= klast;
-                const bool left = hasL && nz(T.b[k]), right = hasR && nz(T.d[k]);
                 double2 f;
                 if (!(tame && row_b_wide(T, k, dl, hasL, hasR, f.x, f.y)))
                     f = row_b_general(T, k, dl, hasL, hasR, pre1[q], pre2[q]);
@@ -882,8 +874,8 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
                 if (kTri && !finite4(T.b[k], T.c[k], T.d[k], T.y[k])) s_odd = 1;
                 if (keep) { kept1[q] = f.x; kept2[q] = f.y; }
             }
-            if (!kTri && __any_sync(~0u, odd) && s >= casesB) casesB = s + 1 + kGeneralStrides;
         }
+        if (!kFew && !kTri && __any_sync(~0u, odd) && s >= casesB) casesB = s + 1 + kGeneralStrides;
         if (__syncthreads_and(apart)) break;
     }
 
