@@ -277,7 +277,8 @@ __device__ __forceinline__ M2 diag_inverse(const PairRow& P, int64_t i0, int64_t
     const RowScale s0 = row_scale(P.c0), s1 = row_scale(P.c1);
     int top = 0;
     M2 D = {d2f_row(P.c0, s0, top), d2f_row(P.d0, s0, top), d2f_row(P.b1, s1, top), d2f_row(P.c1, s1, top)};
-    if (!(i0 + 1 < n && s0.ok && s1.ok && row_fits(top))) D = block_of(P, i0, n).D;
+    if (i0 + 1 >= n) D = {d2f_scaled(P.c0, d_exponent(P.c0)), 0.0f, 0.0f, 1.0f};   // (the last row of an odd system)
+    else if (!(s0.ok && s1.ok && row_fits(top))) D = block_of(P, i0, n).D;
     return minv(D);
 }
 
