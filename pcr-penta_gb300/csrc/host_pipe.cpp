@@ -7,9 +7,15 @@
 // its solve the copy engines serve the other.  Chunks grow: the first holds
 // ceil(m/32) systems, so little copying precedes the first solve, and each
 // next one three times as many, up to ceil(m/4), because a solve of few
-// systems fills the GPU less well than a large one (measured on GB300, m=256
-// n=65536, with FP64 kernels 2.5 times slower than the present ones: 0.102 ms
-// per system at m=8, 0.088 at 32, 0.084 at 64).  The caller's stream is joined
+// systems fills the GPU less well than a large one (GB300, n=65536, us per
+// system at m = 8, 32, 64, 256: FP64 40, 33, 31, 30; mixed 8.4, 3.6, 2.7, 2.1).
+// Other plans, with pinned arrays (us; mixed 128 x 32768, mixed 256 x 65536, FP64
+// 256 x 65536, FP64 64 x 2^20, mixed 1000 x 500): this one 1229, 4297, 8557,
+// 34220, 293; twice as many each time 1238, 4344, 8375, 33746, 299; from
+// ceil(m/64) 1239, 4290, 8424, 33980, 301; eight equal chunks 1256, 4338, 8770,
+// 34667, 340; shrinking again at the end 1294, 4246, 8606, 33645, 345.  The
+// copies in alone take 979, 3840, 3842, 15264 and 138, those out 186, 707, 707,
+// 2789 and 33.  The caller's stream is joined
 // at both ends with events, so the call is asynchronous like the device
 // entry points (the host arrays must stay valid until the stream reaches
 // that point; page-locked host memory lets the copies run asynchronously).
