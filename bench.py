@@ -49,11 +49,11 @@ BYTES_PER_UNKNOWN = 56          # 5 FP64 bands + FP64 rhs read once, FP64 x writ
 # config's own layout and the autotuned plan.  The capture commands and the
 # raw figures are kept with the ncu summaries in the repository's profiles.
 MEASURED_TRAFFIC = {
-    ("c1", "f64"): (290.4, "ncu capture m=48 n=65536, the 4 pcr_pass_kernel launches of one solve"),
-    ("c1", "mixed"): (93.6, "ncu capture m=48 n=65536, mp_first_kernel + mp_try_kernel of one solve"),
+    ("c1", "f64"): (290.6, "ncu capture m=48 n=65536, the 4 pcr_pass_kernel launches of one solve"),
+    ("c1", "mixed"): (93.7, "ncu capture m=48 n=65536, mp_first_kernel + mp_try_kernel of one solve"),
     ("c2", "mixed"): (95.1, "ncu capture m=1024 n=4096, the mp_small_kernel launch of one solve"),
-    ("c4", "f64"): (387.7, "ncu capture m=4 n=2^20, the 5 pcr_pass_kernel launches of one solve"),
-    ("c4", "mixed"): (98.2, "ncu capture m=4 n=2^20, mp_first_kernel + mp_try_kernel of one solve"),
+    ("c4", "f64"): (388.0, "ncu capture m=4 n=2^20, the 5 pcr_pass_kernel launches of one solve"),
+    ("c4", "mixed"): (98.3, "ncu capture m=4 n=2^20, mp_first_kernel + mp_try_kernel of one solve"),
 }
 
 

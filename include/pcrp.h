@@ -108,6 +108,13 @@ typedef struct pcrp_mixed_info {
  * (a tridiagonal batch) the rows run the kernels' zero-operand form, with
  * the bits of explicit +0.0 bands.  The same holds for the two paths below,
  * pcrp_solve_f64_noalloc and pcrp_solve_host.
+ * Speed depends on the scale of the inputs (the bits do not): rows whose
+ * coefficients, given or formed by a stride, lie in [2^-400, 2^112) run most of
+ * their work on the integer pipe, others on the FP64 pipe.  A batch all outside
+ * (every row times 1e40, say) takes 1.4-1.6 times as long, one whose rows are
+ * scaled far apart up to twice as long; row scales by powers of two bring
+ * rows inside and leave the solution's bits alone while nothing under- or
+ * overflows.
  * Replaces: main.cu:46-87 (time_* dispatch around pcr_penta and the splitting
  * kernels), kernel prototypes performanalysis.h:53-59. */
 pcrp_status pcrp_solve_f64(const double* a, const double* b, const double* c,

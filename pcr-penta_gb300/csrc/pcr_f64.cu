@@ -36,8 +36,8 @@
 // the FP64 pipe 67 % and the integer ALU 62 % busy (4 CTAs of 256 threads per
 // SM; what is left is the latency of the row's dependent chains between two
 // barriers).  Measured, before and after: m=64 n=2^20 weakly dominant 91.7 ->
-// 34.0 ms, m=256 n=65536 19.8 -> 7.9 ms, m=1024 n=512 interleaved 0.535 -> 0.265
-// ms; a dense two-stride pass at m=4 n=2^20 1.00 -> 0.38 ms.
+// 33.9 ms, m=256 n=65536 19.8 -> 7.8 ms, m=1024 n=512 interleaved 0.535 -> 0.264
+// ms; a dense two-stride pass at m=4 n=2^20 1.00 -> 0.37 ms.
 //
 // The reference's multiplier registers, which outlive a stride and are reused
 // when a pivot is exactly zero (kernel.cu:122,129), are formed again when that
