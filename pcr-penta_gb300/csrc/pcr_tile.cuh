@@ -289,23 +289,25 @@ __device__ __forceinline__ bool row_a_self(TileRows<CAP>& t, int k, int dl, bool
     return true;
 }
 
-// The same with zeros among b and d (the ends of the system), or a side
-// missing.
+// The same with zeros among b, c, d and y (the ends of the system, sparse
+// right-hand sides), or a side missing: a zero takes its sign from the products
+// added to it.  Zeros of c and y used to take row_a_none with its tests of both
+// neighbours (us, one nonzero right-hand side value per system, 777 systems of
+// 3001 rows 706 -> 634).
 template <int CAP>
 __device__ __forceinline__ bool row_a_tri(TileRows<CAP>& t, int k, int dl, bool hasL, bool has2L, bool hasR, bool has2R, double& cT)
 {
     const int l = hasL ? k - dl : k, r = hasR ? k + dl : k;
     const double b = t.b[k], c = t.c[k], d = t.d[k], y = t.y[k], bL = t.b[l], dR = t.d[r];
-    if (!(nz(c) && nz(y))) return false;
     const unsigned s1 = has2L && nz(bL) ? hiw(t.a[k]) ^ hiw(bL) ^ 0x80000000u : 0u;
     const unsigned s2 = has2R && nz(dR) ? hiw(t.e[k]) ^ hiw(dR) ^ 0x80000000u : 0u;
     // (a missing side adds -0)
     const unsigned zb = (hasL ? s1 ^ hiw(t.c[l]) : ~0u) & (hasR ? s2 ^ hiw(t.a[r]) : ~0u);
     const unsigned zd = (hasL ? s1 ^ hiw(t.e[l]) : ~0u) & (hasR ? s2 ^ hiw(t.c[r]) : ~0u);
-    cT = c;
-    t.Tc[k] = c;
-    t.Tr[k] = ieee::recip(c);
-    t.Ty[k] = y;
+    cT = nz(c) ? c : szero(hiw(c) & (hasL ? s1 ^ hiw(t.d[l]) : ~0u) & (hasR ? s2 ^ hiw(t.b[r]) : ~0u));
+    t.Tc[k] = cT;
+    t.Tr[k] = ieee::recip(cT);
+    t.Ty[k] = nz(y) ? y : szero(hiw(y) & (hasL ? s1 ^ hiw(t.y[l]) : ~0u) & (hasR ? s2 ^ hiw(t.y[r]) : ~0u));
     t.Tb[k] = hasL ? add_z(b, zb) : 0.0;
     t.Td[k] = hasR ? add_z(d, zd) : 0.0;
     t.Ta[k] = hasL ? szero(s1 ^ hiw(t.a[l])) : 0.0;
@@ -396,6 +398,33 @@ __device__ __forceinline__ bool row_b_none(TileRows<CAP>& t, int k, int dl, bool
     t.y[k] = add_z(sub_z(g1.y, yi), g2.y);
     t.a[k] = szero(g1.a);
     t.e[k] = szero(g2.e);
+    return true;
+}
+
+// The same for a tridiagonal row in a tile without infinities and nans: a and e
+// of the row and of T are zeros, and a zero pivot leaves its multiplier (f1, f2
+// on entry) in place, a zero too but in the last stride.  Batches of small
+// integers, whose rows decouple in a few strides while a tenth of the pivots are
+// exactly zero, took the general form in every warp (figures at row_b_wide).
+template <int CAP>
+__device__ __forceinline__ bool row_b_self(TileRows<CAP>& t, int k, int dl, bool hasL, bool hasR, double& f1, double& f2)
+{
+    const int l = hasL ? k - dl : k, r = hasR ? k + dl : k;
+    const double cL = hasL ? t.Tc[l] : 1.0, cR = hasR ? t.Tc[r] : 1.0;
+    if (!nz(cL) && nz(f1) || !nz(cR) && nz(f2)) return false;
+    const double g1 = nz(cL) ? szero(hiw(t.b[k]) ^ hiw(cL)) : f1, g2 = nz(cR) ? szero(hiw(t.d[k]) ^ hiw(cR)) : f2;
+    const unsigned s1 = hiw(g1), s2 = hiw(g2);
+    const double ci = t.c[k], yi = t.y[k];
+    // (a missing side's products are +0)
+    const unsigned zb = (hasL ? s1 ^ hiw(t.Tb[l]) : 0u) & ~hiw(t.a[k]) & (hasR ? s2 ^ hiw(t.Ta[r]) : 0u);
+    const unsigned zd = (hasL ? s1 ^ hiw(t.Te[l]) : 0u) & ~hiw(t.e[k]) & (hasR ? s2 ^ hiw(t.Td[r]) : 0u);
+    t.c[k] = add_z(sub_z(hasL ? s1 ^ hiw(t.Td[l]) : 0u, ci), hasR ? s2 ^ hiw(t.Tb[r]) : 0u);
+    t.y[k] = add_z(sub_z(hasL ? s1 ^ hiw(t.Ty[l]) : 0u, yi), hasR ? s2 ^ hiw(t.Ty[r]) : 0u);
+    t.b[k] = szero(zb);
+    t.d[k] = szero(zd);
+    t.a[k] = szero(hasL ? s1 ^ hiw(t.Ta[l]) : 0u);
+    t.e[k] = szero(hasR ? s2 ^ hiw(t.Te[r]) : 0u);
+    f1 = g1; f2 = g2;
     return true;
 }
 
@@ -493,8 +522,8 @@ __device__ __forceinline__ bool row_b_tri(TileRows<CAP>& t, int k, int dl, bool 
     const double bi = t.b[k], di = t.d[k], cL = hasL ? t.Tc[l] : 1.0, cR = hasR ? t.Tc[r] : 1.0;
     const double bL = hasL ? t.Tb[l] : 0.0, dL = hasL ? t.Td[l] : 0.0;
     const double bR = hasR ? t.Tb[r] : 0.0, dR = hasR ? t.Td[r] : 0.0;
-    if (!ieee::fits(off_or_zero(bi) | off_or_zero(di) | ieee::off(cL) | ieee::off(cR) | off_or_zero(bL) |
-                    off_or_zero(dL) | off_or_zero(bR) | off_or_zero(dR))) return false;
+    if (!all_fit(off_or_zero(bi) | off_or_zero(di) | ieee::off(cL) | ieee::off(cR) | off_or_zero(bL) |
+                 off_or_zero(dL) | off_or_zero(bR) | off_or_zero(dR))) return false;
     const Multiplier m1 = multiplier(bi, cL, t.Tr[l], hasL && nz(bi), hasL);
     const Multiplier m2 = multiplier(di, cR, t.Tr[r], hasR && nz(di), hasR);
     const unsigned s1 = hiw(m1.x), s2 = hiw(m2.x);
@@ -512,17 +541,22 @@ __device__ __forceinline__ bool row_b_tri(TileRows<CAP>& t, int k, int dl, bool 
 }
 
 // The same for operands outside the integer forms' window, with the products
-// on the FP64 pipe (10 FP64 operations instead of the general form's 18, and
-// no second try: rows scaled by up to 2^+-400, us, 4000 systems of 128 rows
-// 224 -> 153, 777 of 3001 1299 -> 880; every row scaled by 1e40 151 -> 107 and
-// 854 -> 620).
+// on the FP64 pipe (10 FP64 operations instead of the general form's 18, and no
+// second try), and for zero pivots: f1, f2 enter as the multipliers those leave
+// in place.  The lanes of a warp take row_b_tri or this form together.  us, the
+// general form / this one lane by lane / together: rows scaled by up to
+// 2^+-400, 4000 systems of 128 rows 215 / 152 / 105, 777 of 3001 1362 / 983 /
+// 852; every row scaled by 1e40 145 / 104 / 104 and 818 / 617 / 619.  Small
+// integers with exact zero pivots (also by row_b_self, row_a_tri and zero_left),
+// the general form against now: 253 -> 145 and 1612 -> 909.
 template <int CAP>
 __device__ __forceinline__ bool row_b_wide(TileRows<CAP>& t, int k, int dl, bool hasL, bool hasR, double& f1, double& f2)
 {
     const int l = hasL ? k - dl : k, r = hasR ? k + dl : k;
     const double cL = hasL ? t.Tc[l] : 1.0, cR = hasR ? t.Tc[r] : 1.0;
-    if (!(nz(cL) && nz(cR))) return false;
-    const double g1 = hasL ? quot(t.b[k], cL, t.Tr[l]) : 0.0, g2 = hasR ? quot(t.d[k], cR, t.Tr[r]) : 0.0;
+    double g1 = 0.0, g2 = 0.0;
+    if (hasL) g1 = nz(cL) ? quot(t.b[k], cL, t.Tr[l]) : f1;
+    if (hasR) g2 = nz(cR) ? quot(t.d[k], cR, t.Tr[r]) : f2;
     if (max(expw(g1), expw(g2)) >= 0x7FF00000u) return false;
     const unsigned s1 = hiw(g1), s2 = hiw(g2);
     const double ny = add(sub(hasL ? mul(g1, t.Ty[l]) : 0.0, t.y[k]), hasR ? mul(g2, t.Ty[r]) : 0.0);
@@ -598,6 +632,18 @@ template <int CAP>
 __device__ __noinline__ double multiplier_right(TileRows<CAP>& t, int m, int dl, int klast)
 {
     return m + 2 * dl <= klast && nz(t.d[m + dl]) ? quot(neg(t.e[m]), t.d[m + dl]) : 0.0;
+}
+// The same of a tridiagonal row in a tile without infinities and nans, where a
+// and e are zeros
+template <int CAP>
+__device__ __forceinline__ double zero_left(TileRows<CAP>& t, int m, int dl, int kfirst)
+{
+    return m - 2 * dl >= kfirst && nz(t.b[m - dl]) ? szero(~(hiw(t.a[m]) ^ hiw(t.b[m - dl]))) : 0.0;
+}
+template <int CAP>
+__device__ __forceinline__ double zero_right(TileRows<CAP>& t, int m, int dl, int klast)
+{
+    return m + 2 * dl <= klast && nz(t.d[m + dl]) ? szero(~(hiw(t.e[m]) ^ hiw(t.d[m + dl]))) : 0.0;
 }
 
 // Row k couples to no other row, and no product of its c and y with another
@@ -808,18 +854,31 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
             if (!kTri && __any_sync(~0u, odd) && s >= casesA) casesA = s + 1 + kGeneralStrides;
         }
         double pre1[kMaxRowsPerThread], pre2[kMaxRowsPerThread];
-        if (__syncthreads_or(zero_pivot)) {
+        const bool zeros_left = __syncthreads_or(zero_pivot);   // (read again by tridiagonal tiles)
+        if (zeros_left) {
             // some pivot cT of the tile is exactly zero: the multipliers the
             // reference then uses (kernel.cu:96-112), from the state before
-            // phase B changes it
+            // phase B changes it (where one case serves all rows and in
+            // tridiagonal tiles, only of the rows that divide by it: the test in
+            // the per-case kernel costs dense batches 0.5-0.8 %)
             for (int k = tid, q = 0; k < TR; k += bd, q++) {
                 const bool hasL = k - dl >= kfirst, hasR = k + dl <= klast;
                 const bool has2L = k - 2 * dl >= kfirst, has2R = k + 2 * dl <= klast;
                 if (k < klo || k >= khi) continue;
-                pre1[q] = hasR ? multiplier_left(T, k + dl, dl, kfirst)
-                               : has2L ? multiplier_left(T, k - dl, dl, kfirst) : kept1[q];
-                pre2[q] = has2R ? multiplier_right(T, k + dl, dl, klast)
-                                : hasL ? multiplier_right(T, k - dl, dl, klast) : kept2[q];
+                if (kFew || kTri) {
+                    const int ml = hasR ? k + dl : k - dl, mr = has2R ? k + dl : k - dl;
+                    if (hasL && !nz(T.Tc[k - dl]))
+                        pre1[q] = !hasR && !has2L ? kept1[q]
+                                  : tame ? zero_left(T, ml, dl, kfirst) : multiplier_left(T, ml, dl, kfirst);
+                    if (hasR && !nz(T.Tc[k + dl]))
+                        pre2[q] = !has2R && !hasL ? kept2[q]
+                                  : tame ? zero_right(T, mr, dl, klast) : multiplier_right(T, mr, dl, klast);
+                } else {
+                    pre1[q] = hasR ? multiplier_left(T, k + dl, dl, kfirst)
+                                   : has2L ? multiplier_left(T, k - dl, dl, kfirst) : kept1[q];
+                    pre2[q] = has2R ? multiplier_right(T, k + dl, dl, klast)
+                                    : hasL ? multiplier_right(T, k - dl, dl, klast) : kept2[q];
+                }
             }
             __syncthreads();
         }
@@ -844,7 +903,12 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
                     done = true;
                 }
             } else if (!left && !right) {
-                done = row_b_none(T, k, dl, hasL, hasR, f1, f2);
+                if (tame) {
+                    if (zeros_left) { f1 = pre1[q]; f2 = pre2[q]; }
+                    done = row_b_self(T, k, dl, hasL, hasR, f1, f2);
+                } else {
+                    done = row_b_none(T, k, dl, hasL, hasR, f1, f2);
+                }
             } else if (kTri) {
                 // the dense form of inner rows in a window, one form for all in
                 // a whole subsystem, where most rows are near an end
@@ -867,6 +931,7 @@ __device__ __forceinline__ void pcr_tile(const PcrPassArgs& p, int64_t j, uint32
                 if (keep) { kept1[q] = f1; kept2[q] = f2; }
             } else {
                 double2 f;
+                if (kTri) f = make_double2(pre1[q], pre2[q]);
                 if (!(tame && row_b_wide(T, k, dl, hasL, hasR, f.x, f.y)))
                     f = row_b_general(T, k, dl, hasL, hasR, pre1[q], pre2[q]);
                 if (!kTri) odd = odd || (k - 4 * dl >= kfirst && k + 4 * dl <= klast);

@@ -122,3 +122,36 @@ def test_tridiagonal_rows_scaled_apart_bitexact(cuda, n, spread):
     torch.cuda.synchronize()
     assert_bitexact(t[5].cpu().numpy(), ref, f"n={n} spread={spread}")
     assert_bitexact(r.cpu().numpy(), ref, f"ragged n={n} spread={spread}")
+
+
+@pytest.mark.parametrize("opts", [None, dict(smem_rows=5, fuse_strides=2), dict(smem_rows=33, fuse_strides=1, tile_rows=31),
+                                  dict(smem_rows=64, fuse_strides=3, threads=32)])
+@pytest.mark.parametrize("n", [1, 2, 3, 5, 33, 64, 90, 513, 3001])
+@pytest.mark.parametrize("kind", ["dyadic", "holes", "spike"])
+def test_tridiagonal_zeros_and_zero_pivots_bitexact(cuda, kind, n, opts):
+    """Null outer bands with zeros of both signs anywhere: exact zero pivots,
+    also in the last stride and across passes, and zero right-hand sides but
+    for one value per system; uniform and ragged."""
+    import torch
+    m = 40
+    rng = np.random.default_rng(n)
+    arrs = operands("holes" if kind == "spike" else kind, rng, m, n)
+    if kind == "spike":
+        arrs[5][:] = 0.0
+        arrs[5].reshape(m, n)[:, n // 2] = 1.0
+    arrs[0][:] = 0.0
+    arrs[4][:] = 0.0
+    for v in (arrs[1], arrs[2], arrs[3], arrs[5]):
+        z = (v == 0.0) & (rng.random(m * n) < 0.5)
+        v[z] = -0.0
+    ref = O.pcr(*arrs, m, n)
+    t = to_device(arrs, "cuda:0")
+    t[0] = t[4] = None
+    r = t[5].clone()
+    o = pcrp.Opts(**opts) if opts else None
+    pcrp.solve_f64(*t, m, n, opts=o)
+    assert_bitexact(t[5].cpu().numpy(), ref, f"{kind} n={n} {opts}")
+    if not opts:
+        offsets = torch.arange(m + 1, dtype=torch.int64, device="cuda:0") * n
+        pcrp.solve_ragged(*t[:5], r, offsets, m, n)
+        assert_bitexact(r.cpu().numpy(), ref, f"ragged {kind} n={n}")
