@@ -1497,7 +1497,20 @@ cudaError_t launch_mp_try(const MpPassArgs& p, cudaStream_t s)
                                          (int)mp_pass_smem(kMpMaxRows));
     if (e != cudaSuccess) return e;
     const int64_t blocks = std::min<int64_t>(items, mp_grid_cap((const void*)mp_try_kernel, kMpTryThreads, smem));
-    e = launch_dependent(mp_try_kernel, (unsigned)blocks, kMpTryThreads, smem, s, p);
+    // Uniform batches of at most two tiles per SM take the largest shared
+    // memory of the SM.  Without that the general passes of a graph's sweeps are
+    // up to a fifth slower in such batches (this kernel's 60 registers allow
+    // four tiles, whose shared memory leaves the SM a smaller one; at the 48
+    // registers of before it took the largest by itself), with it slower in
+    // larger ones.  Coupled systems, us, with / without: 8 of 30000 rows 246 /
+    // 279, 16 of 20000 262 / 296, 30 of 9000 235 / 269, 16 of 30000 (272 tiles)
+    // 292 / 329; 20 of 30000 (340) 370 / 352, 64 of 30000 740 / 707; classes of a
+    // ragged batch, several at once, 2203 / 2157.
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        sms = 0;
+    const bool spare = !p.rg && items <= 2 * (int64_t)sms;
+    e = launch_dependent_as(spare, mp_try_kernel, (unsigned)blocks, kMpTryThreads, smem, s, p);
     count_launch();
     return e;
 }

@@ -97,21 +97,32 @@ struct MpPassArgs {
 // (griddepcontrol.wait) for the predecessor to complete and its writes to be
 // visible before touching memory.  Hides the launch gap between the many
 // short dependent kernels of a solve.
+// full_carveout: the launch asks for the largest shared memory (and the
+// smallest L1) of its SMs.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
-                             Args&&... args)
+cudaError_t launch_dependent_as(bool full_carveout, void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
+                                cudaStream_t s, Args&&... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = full_carveout ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
+                             Args&&... args)
+{
+    return launch_dependent_as(false, kernel, grid, block, smem, s, static_cast<Args&&>(args)...);
 }
 
 // Window geometry of the windowed passes (level 0).
